@@ -167,6 +167,35 @@ struct DetView {
     const double* varpsf;
     const double* norm;  // SX x SY box counts (normImage)
 };
+
+// detect_fft.cu: line transforms of M points, `lines` of them a CTA, and a
+// detector's twiddles and library spectra.
+constexpr int DET_FFT_MIN_R = 14;  // see det_fft_wanted
+constexpr size_t DET_FFT_MAX_LIBRARY = (size_t)512 << 20;  // bytes of library spectra a detector may hold
+constexpr size_t DET_FFT_T_BYTES = (size_t)56 << 20;       // column transforms in flight (see frames_together)
+struct FftDim {
+    int M = 0, lines = 0;
+};
+struct DetFft {
+    FftDim x, y;
+    int pairs = 0;
+    double2* d_tab = nullptr;  // twiddles of x and y, then the spectra of the slice pairs
+    const double2* twx() const { return d_tab; }
+    const double2* twy() const { return d_tab + x.M; }
+    double2* K() const { return d_tab + x.M + y.M; }
+};
+// detect.cu: candidate lists of device frames, and the direct scores and offsets
+// of listed candidates.
+int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap, int rows, int want, double* d_out,
+                  int* d_counts, double* d_var, cudaStream_t st);
+int detect_refine(zola_detector* d, const double* d_frames, const double* d_var, double* d_cand, int cap, int n,
+                  const int* d_frame, const int* d_index, cudaStream_t st);
+bool det_fft_wanted(const DetView& v);
+void det_fft_build(zola_ctx* ctx, const DetView& v, DetFft& p);
+void det_fft_free(DetFft& p);
+size_t det_fft_scratch(const DetView& v, const DetFft& p, int nf);
+void det_fft_scores(zola_ctx* ctx, const DetView& v, const DetFft& p, const double* frames, int nf, const double* isv,
+                    char* scratch, double* score, cudaStream_t st);
 }  // namespace zola
 
 struct zola_detector {
@@ -174,6 +203,7 @@ struct zola_detector {
     zola::DetView v{};
     std::vector<double> range;
     double* d_lib = nullptr;    // psf0 | varpsf | norm
+    zola::DetFft fft;           // library spectra (empty: direct correlation)
     std::vector<double> h_psf;  // Z x R x R normalised library PSFs (pipeline initialisation)
     int cand_room = 0;          // longest candidate list the pipeline has met (its next starting room)
 };
