@@ -17,7 +17,7 @@
 // the mask, so the fits do not depend on the order.  Frames advance in waves:
 // each wave takes, per frame, the next K candidates that need a fit under the
 // current mask (one CTA per frame tests candidates in parallel chunks: border,
-// centre and patch masks, getAandB, SNR), fits all of them in one batched call
+// centre and patch masks, getAandB, SNR), completes their starts, fits all of them in one batched call
 // (FP64 or split), evaluates the model at every fitted position, and then one
 // CTA per frame replays the reference's sequential walk over the candidates
 // the wave covered: mask tests, acceptance, mask updates.  A candidate masked
@@ -73,119 +73,172 @@ __device__ inline bool pipe_inside(const PipeView& V, int ci, int cj) {
     return ci > h + 1 && cj > h + 1 && ci < V.SX - h - 1 && cj < V.SY - h - 1;
 }
 
+__device__ inline double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ inline double warp_max(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
 // getAandB with the library PSF of slice r, threshold 10% of its max, on the
-// patch minus the sCMOS term when there is one (:1119-1211); returns whether
-// the candidate is fitted (maxPatch / B > maxSNR and B > 0).
+// patch minus the sCMOS term when there is one (:1119-1211), by one warp; returns
+// whether the candidate is fitted (maxPatch / B > maxSNR and B > 0).
 __device__ bool pipe_a_and_b(const PipeView& V, const double* img, int r, int ci, int cj, double* A_, double* B_,
                              double* maxp_) {
     const double* vm = V.vmap;
-    const int R = V.R, h = R / 2, SY = V.SY;
-    const double* psf = V.libpsf + (size_t)r * R * R;
+    const int R = V.R, RR = R * R, SY = V.SY, lane = threadIdx.x & 31;
+    const size_t corner = (size_t)(ci - R / 2) * SY + (cj - R / 2);
+    const double* psf = V.libpsf + (size_t)r * RR;
     double maxp = -INFINITY, maxi = -INFINITY;
-    for (int a = 0; a < R; ++a)
-        for (int b = 0; b < R; ++b) {
-            const size_t px = (size_t)(ci - h + a) * SY + (cj - h + b);
-            maxi = fmax(maxi, psf[a * R + b]);
-            maxp = fmax(maxp, img[px] - (vm ? vm[px] : 0.0));
-        }
+#pragma unroll 4
+    for (int k = lane; k < RR; k += 32) {
+        const size_t px = corner + (size_t)(k / R) * SY + k % R;
+        maxi = fmax(maxi, psf[k]);
+        maxp = fmax(maxp, img[px] - (vm ? vm[px] : 0.0));
+    }
+    maxi = warp_max(maxi);
+    maxp = warp_max(maxp);
     const double thr = maxi * 0.1;
-    double B = 0, A = 0, cb = 0, ca = 0;
-    for (int a = 0; a < R; ++a)
-        for (int b = 0; b < R; ++b) {
-            const size_t px = (size_t)(ci - h + a) * SY + (cj - h + b);
-            const double v = img[px] - (vm ? vm[px] : 0.0);
-            if (psf[a * R + b] < thr) { B += v; cb += 1; } else { A += v; ca += 1; }
-        }
+    double B = 0, A = 0;
+    int cb = 0;
+#pragma unroll 4
+    for (int k = lane; k < RR; k += 32) {
+        const size_t px = corner + (size_t)(k / R) * SY + k % R;
+        const double v = img[px] - (vm ? vm[px] : 0.0);
+        const bool low = psf[k] < thr;
+        B += low ? v : 0.0;
+        A += low ? 0.0 : v;
+        cb += low;
+    }
+    B = warp_sum(B);
+    A = warp_sum(A);
+    cb = __reduce_add_sync(0xffffffffu, cb);
     B = cb != 0 ? B / cb : 0.0;
-    A -= ca * B;
+    A -= (double)(RR - cb) * B;
     *A_ = A;
     *B_ = B;
     *maxp_ = maxp;
     return maxp / B > V.max_snr && B > 0;
 }
 
-// One wave's selection for one frame (one CTA): walking the candidates from
-// the frame's pointer in chunks of blockDim, each thread tests one candidate
-// under the current mask; the first K that need a fit (in candidate order) get
-// slots and their ROI and start.  limit = just past the K-th (or the end).
-__global__ void __launch_bounds__(128) k_pipe_wave(PipeView V, int K) {
+// One wave's selection for one frame (one CTA): walking the candidates from the
+// frame's pointer, the first K (in candidate order) that need a fit under the
+// current mask get slots, their ROI and the A, B of their start (k_pipe_start adds
+// the position).  limit = just past the K-th (or the end).
+// 512 candidates at a time: a thread drops the ones outside the border or with a
+// masked centre, which late in a frame are nearly all; the rest are taken in order,
+// a warp each, until K are found.  (A thread a candidate for everything read its
+// 1,600 pixels one after the other: 2.8 ms a wave at R = 40.)
+constexpr int PW_THREADS = 512, PW_WARPS = PW_THREADS / 32;
+__global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
     const int f = blockIdx.x, SX = V.SX, SY = V.SY, R = V.R, h = R / 2, RR = R * R;
     if (V.done[f]) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double* img = V.fimg + (size_t)f * SX * SY;
     const unsigned char* mk = V.mask + (size_t)f * SX * SY;
     const double* cand = V.cand + (size_t)f * V.cap * 7;
+    int* code_of = V.cand_slot + (size_t)f * V.cap;
     const int n = min(V.counts[f], V.cap);
-    __shared__ unsigned char sel[128];
-    __shared__ int s_got, s_lim, s_base;
+    __shared__ int live[PW_THREADS], wcount[PW_WARPS], sel[PW_WARPS], s_base;
     int taken = 0, limit = n;
-    for (int c0 = V.pointer[f]; c0 < n && taken < K; c0 += blockDim.x) {
+    for (int c0 = V.pointer[f]; c0 < n && taken < K; c0 += PW_THREADS) {
         const int i = c0 + threadIdx.x;
-        int code = -4;
-        double A = 0, B = 0, maxp = 0;
+        bool look = false;
         if (i < n) {
-            const double* row = cand + (size_t)i * 7;
+            const int ci = (int)llrint(cand[(size_t)i * 7 + 2]), cj = (int)llrint(cand[(size_t)i * 7 + 3]);
+            const bool in = pipe_inside(V, ci, cj);
+            look = in && mk[(size_t)ci * SY + cj] == 0;
+            if (!look) code_of[i] = in ? -3 : -2;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, look);
+        if (lane == 0) wcount[warp] = __popc(bal);
+        __syncthreads();
+        int at = 0, nl = 0;
+        for (int w = 0; w < PW_WARPS; ++w) {
+            if (w < warp) at += wcount[w];
+            nl += wcount[w];
+        }
+        if (look) live[at + __popc(bal & ((1u << lane) - 1))] = i;
+        __syncthreads();
+        for (int l0 = 0; l0 < nl && taken < K; l0 += PW_WARPS) {
+            const bool mine = l0 + warp < nl;
+            const int k = live[min(l0 + warp, nl - 1)];
+            const double* row = cand + (size_t)k * 7;
             const int r = (int)llrint(row[1]), ci = (int)llrint(row[2]), cj = (int)llrint(row[3]);
-            if (!pipe_inside(V, ci, cj)) {
-                code = -2;
-            } else {
-                bool masked = mk[(size_t)ci * SY + cj] != 0;
-                for (int k = 0; k < RR && !masked; ++k) masked = mk[(size_t)(ci - h + k / R) * SY + (cj - h + k % R)] != 0;
-                code = masked ? -3 : (pipe_a_and_b(V, img, r, ci, cj, &A, &B, &maxp) ? 0 : -1);
-            }
-            V.cand_slot[(size_t)f * V.cap + i] = code;
-            V.cand_maxp[(size_t)f * V.cap + i] = maxp;
-        }
-        sel[threadIdx.x] = code == 0;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int got = 0, lim = -1;
-            for (int t = 0; t < (int)blockDim.x && c0 + t < n; ++t) {
-                if (!sel[t]) continue;
-                if (got == K - taken) { sel[t] = 0; continue; }
-                ++got;
-                if (got == K - taken) lim = c0 + t + 1;
-            }
-            if (lim >= 0)
-                for (int t = lim - c0; t < (int)blockDim.x; ++t) sel[t] = 0;
-            s_got = got;
-            s_lim = lim;
-            s_base = got ? atomicAdd(V.nslots, got) : 0;
-            int k = 0;
-            for (int t = 0; t < (int)blockDim.x && c0 + t < n; ++t)
-                if (sel[t]) {
-                    const int s = s_base + k++;
-                    V.cand_slot[(size_t)f * V.cap + c0 + t] = s < V.slot_cap ? s : -5;
+            const size_t corner = (size_t)(ci - h) * SY + (cj - h);
+            double A = 0, B = 0, maxp = 0;
+            int code = -3;
+            if (mine) {
+                bool masked = false;
+                for (int q0 = 0; q0 < RR && !masked; q0 += 256) {
+                    bool any = false;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int q = q0 + 32 * u + lane;
+                        any |= q < RR && mk[corner + (size_t)(q / R) * SY + q % R] != 0;
+                    }
+                    masked = __any_sync(0xffffffffu, any);
                 }
-        }
-        __syncthreads();
-        if (sel[threadIdx.x]) {
-            const int s = V.cand_slot[(size_t)f * V.cap + i];
-            if (s >= 0) {
-                const double* row = cand + (size_t)i * 7;
-                const int r = (int)llrint(row[1]), ci = (int)llrint(row[2]), cj = (int)llrint(row[3]);
-                float* roi = V.rois + (size_t)s * RR;
-                for (int a = 0; a < R; ++a)
-                    for (int b = 0; b < R; ++b) roi[a * R + b] = (float)img[(size_t)(ci - h + a) * SY + (cj - h + b)];
-                if (V.vmap) {
-                    float* sv = V.slot_v + (size_t)s * RR;
-                    for (int a = 0; a < R; ++a)
-                        for (int b = 0; b < R; ++b) sv[a * R + b] = (float)V.vmap[(size_t)(ci - h + a) * SY + (cj - h + b)];
+                if (!masked) code = pipe_a_and_b(V, img, r, ci, cj, &A, &B, &maxp) ? 0 : -1;
+                if (lane == 0) {
+                    code_of[k] = code;
+                    V.cand_maxp[(size_t)f * V.cap + k] = maxp;
                 }
-                double* in = V.init + (size_t)s * 5;  // loc.init(A, B, -dx, -dy, range[r] + dz)
-                in[0] = -row[5];
-                in[1] = -row[6];
-                in[2] = V.range[r] + row[4];
-                in[3] = A;
-                in[4] = B;
-                V.slot_frame[s] = f;
-                V.slot_cand[s] = i;
             }
+            if (lane == 0) sel[warp] = mine && code == 0;
+            __syncthreads();
+            int rank = 0, got = 0, last = -1;
+            for (int w = 0; w < PW_WARPS; ++w)
+                if (sel[w] && got < K - taken) {
+                    if (w < warp) ++rank;
+                    ++got;
+                    last = w;
+                }
+            if (threadIdx.x == 0) s_base = got ? atomicAdd(V.nslots, got) : 0;
+            __syncthreads();
+            if (mine && code == 0 && warp <= last) {
+                const int s = s_base + rank;
+                if (lane == 0) code_of[k] = s < V.slot_cap ? s : -5;
+                if (s < V.slot_cap) {
+                    float* roi = V.rois + (size_t)s * RR;
+                    float* sv = V.vmap ? V.slot_v + (size_t)s * RR : nullptr;
+#pragma unroll 4
+                    for (int q = lane; q < RR; q += 32) {
+                        const size_t px = corner + (size_t)(q / R) * SY + q % R;
+                        roi[q] = (float)img[px];
+                        if (sv) sv[q] = (float)V.vmap[px];
+                    }
+                    if (lane == 0) {
+                        V.init[(size_t)s * 5 + 3] = A;
+                        V.init[(size_t)s * 5 + 4] = B;
+                        V.slot_frame[s] = f;
+                        V.slot_cand[s] = k;
+                    }
+                }
+            }
+            taken += got;
+            if (taken == K) limit = live[l0 + last] + 1;
+            __syncthreads();  // sel, s_base and live are written again
         }
-        taken += s_got;
-        if (s_lim >= 0) limit = s_lim;
         __syncthreads();
     }
     if (threadIdx.x == 0) V.limit[f] = limit;
+}
+
+// Start positions of the wave's slots, from their candidates' refined offsets:
+// loc.init(A, B, -dx, -dy, range[r] + dz).
+__global__ void k_pipe_start(PipeView V, int n) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const double* row = V.cand + ((size_t)V.slot_frame[s] * V.cap + V.slot_cand[s]) * 7;
+    double* in = V.init + (size_t)s * 5;
+    in[0] = -row[5];
+    in[1] = -row[6];
+    in[2] = V.range[(int)llrint(row[1])] + row[4];
 }
 
 // The fitted slots that can be accepted whatever the mask: every test of the
@@ -211,17 +264,20 @@ __global__ void k_pipe_need(PipeView V, int n, const double* theta, const int* s
 
 // Model threshold of each listed slot: 0.2 max(0, max(model - B)), model =
 // psi A + B (+ sCMOS v) (maxModelThreshold, LocalizationPipeline.java:860-880).
-__global__ void k_pipe_mthr(int n, int RR, const double* theta, const double* psi, const float* slot_v, double* mthr,
-                            const int* list, const int* count) {
-    const int li = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp a slot.
+__global__ void __launch_bounds__(128) k_pipe_mthr(int n, int RR, const double* theta, const double* psi,
+                                                   const float* slot_v, double* mthr, const int* list, const int* count) {
+    const int li = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (li >= min(n, *count)) return;
     const int s = list[li];
     const double A = theta[5 * s + 3], B = theta[5 * s + 4];
     const double* ps = psi + (size_t)s * RR;
     const float* sv = slot_v ? slot_v + (size_t)s * RR : nullptr;
     double m = 0.0;
-    for (int k = 0; k < RR; ++k) m = fmax(m, ps[k] * A + B + (sv ? (double)sv[k] : 0.0) - B);
-    mthr[s] = m * 0.2;
+#pragma unroll 4
+    for (int k = lane; k < RR; k += 32) m = fmax(m, ps[k] * A + B + (sv ? (double)sv[k] : 0.0) - B);
+    m = warp_max(m);
+    if (lane == 0) mthr[s] = m * 0.2;
 }
 
 // The reference's sequential walk over one frame's candidates (one CTA per
@@ -235,10 +291,30 @@ __global__ void __launch_bounds__(256) k_pipe_replay(PipeView V, const double* t
     const double* img = V.fimg + (size_t)f * SX * SY;
     const double* cand = V.cand + (size_t)f * V.cap * 7;
     if (V.done[f]) return;
-    const int n = min(V.counts[f], V.cap), lim = V.limit[f];
-    for (int i = V.pointer[f]; i < lim; ++i) {
-        const int slot = V.cand_slot[(size_t)f * V.cap + i];
-        if (slot == -2 || slot == -3) continue;  // outside the border, or masked (masks only grow)
+    const int n = min(V.counts[f], V.cap), lim = V.limit[f], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // The candidates to walk, in order: 256 at a time, without those outside the border
+    // or already masked when the wave looked (masks only grow).
+    __shared__ int list[256], wcount[8];
+    int c0 = V.pointer[f] - 256, at = 0, nl = 0;
+    for (;;) {
+        if (at == nl) {
+            c0 += 256;
+            if (c0 >= lim) break;
+            __syncthreads();
+            const int k = c0 + threadIdx.x, code = k < lim ? V.cand_slot[(size_t)f * V.cap + k] : -2;
+            const unsigned bal = __ballot_sync(0xffffffffu, code != -2 && code != -3);
+            if (lane == 0) wcount[warp] = __popc(bal);
+            __syncthreads();
+            int o = at = nl = 0;
+            for (int w = 0; w < 8; ++w) {
+                if (w < warp) o += wcount[w];
+                nl += wcount[w];
+            }
+            if (code != -2 && code != -3) list[o + __popc(bal & ((1u << lane) - 1))] = k;
+            __syncthreads();
+            continue;
+        }
+        const int i = list[at++], slot = V.cand_slot[(size_t)f * V.cap + i];
         const int ci = (int)llrint(cand[(size_t)i * 7 + 2]), cj = (int)llrint(cand[(size_t)i * 7 + 3]);
         if (mk[(size_t)ci * SY + cj]) continue;  // uniform read of the (synchronised) mask
         bool mine = false;
@@ -297,11 +373,12 @@ __global__ void k_take_acc(int n, const int* acc_slot, const double* theta, doub
 }
 
 // chi2 and CRLB of the accepted localizations (psi, dpsi evaluated at their
-// fitted positions, in acceptance-list order).
-__global__ void k_pipe_rows(PipeView V, int n, const int* acc_slot, const int* acc_seq, const int* status,
-                            const double* theta,
-                            const double* psi, const double* dpsi, LocRow* rows) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// fitted positions, in acceptance-list order).  A warp a row; a thread a row read
+// its 4 R^2 model values one after the other (2.0 ms for 100 rows at R = 40).
+__global__ void __launch_bounds__(128) k_pipe_rows(PipeView V, int n, const int* acc_slot, const int* acc_seq,
+                                                   const int* status, const double* theta, const double* psi,
+                                                   const double* dpsi, LocRow* rows) {
+    const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (k >= n) return;
     const int s = acc_slot[k], R = V.R, RR = R * R;
     const int f = V.slot_frame[s], i = V.slot_cand[s];
@@ -312,22 +389,32 @@ __global__ void k_pipe_rows(PipeView V, int n, const int* acc_slot, const int* a
     const double* ps = psi + (size_t)k * RR;
     const float* roi = V.rois + (size_t)s * RR;
     const float* sv = V.vmap ? V.slot_v + (size_t)s * RR : nullptr;
-    double chi = 0;
-    for (int q = 0; q < RR; ++q) {  // scoreCompute against the model (with the sCMOS term)
-        const double mu = ps[q] * A + B + (sv ? (double)sv[q] : 0.0);
-        const double dd = roi[q] - mu;
+    double chi = 0, acc[15];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) acc[q] = 0;
+#pragma unroll 2
+    for (int p = lane; p < RR; p += 32) {
+        const double m = ps[p] * A + B, mu = m + (sv ? (double)sv[p] : 0.0);
+        const double dd = roi[p] - mu;  // scoreCompute against the model (with the sCMOS term)
         chi += dd * dd / mu;
-    }
-    chi /= RR;
-    double F[25];
-    for (int q = 0; q < 25; ++q) F[q] = 0;
-    for (int p = 0; p < RR; ++p) {
-        const double mu = ps[p] * A + B;
         const double d[5] = {A * dpsi[((size_t)k * 3 + 0) * RR + p], A * dpsi[((size_t)k * 3 + 1) * RR + p],
-                             A * dpsi[((size_t)k * 3 + 2) * RR + p], mu, 1.0};
+                             A * dpsi[((size_t)k * 3 + 2) * RR + p], m, 1.0};
+        int o = 0;
+#pragma unroll
         for (int q = 0; q < 5; ++q)
-            for (int r2 = 0; r2 < 5; ++r2) F[q * 5 + r2] += d[q] * d[r2] / mu;
+#pragma unroll
+            for (int r2 = 0; r2 <= q; ++r2) acc[o++] += d[q] * d[r2] / m;
     }
+    chi = warp_sum(chi) / RR;
+#pragma unroll
+    for (int q = 0; q < 15; ++q) acc[q] = warp_sum(acc[q]);
+    if (lane != 0) return;
+    double F[25];
+    int o = 0;
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int r2 = 0; r2 <= q; ++r2) F[q * 5 + r2] = F[r2 * 5 + q] = acc[o++];
     double cr[5];
     lm_crlb(F, cr);
     for (int q = 0; q < 3; ++q)
@@ -415,10 +502,10 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
     const int slot_cap = FB * K;
     Buf b_img, b_mask, b_cand, b_cnt, b_lib, b_rng, b_cslot, b_cmax, b_ptr, b_lim, b_done, b_ns, b_rois, b_init, b_sf,
         b_sc, b_out5, b_st, b_xyz, b_psi, b_mthr, b_acc, b_seq, b_nacc, b_dpsi, b_rows, b_fimg, b_adu, b_off, b_gain,
-        b_vg, b_sv, b_u16, b_list, b_nlist;
+        b_vg, b_sv, b_u16, b_list, b_nlist, b_var;
     cudaError_t e = cudaSuccess;
     auto A = [&](Buf& b, size_t bytes) { if (e == cudaSuccess) e = b.alloc(bytes); };
-    A(b_img, SS * FB * 8); A(b_mask, SS * FB); A(b_cand, (size_t)FB * cap * 7 * 8); A(b_cnt, (size_t)FB * 4);
+    A(b_img, SS * FB * 8); A(b_var, SS * FB * 8); A(b_mask, SS * FB); A(b_cand, (size_t)FB * cap * 7 * 8); A(b_cnt, (size_t)FB * 4);
     A(b_lib, lib.size() * 8); A(b_rng, range.size() * 8); A(b_cslot, (size_t)FB * cap * 4);
     A(b_cmax, (size_t)FB * cap * 8); A(b_ptr, (size_t)FB * 4); A(b_lim, (size_t)FB * 4); A(b_done, (size_t)FB * 4);
     A(b_ns, 64); A(b_nacc, 64);
@@ -481,7 +568,9 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
         if (e == cudaSuccess) e = cudaMemsetAsync(b_ptr.p, 0, (size_t)nf * 4, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(b_done.p, 0, (size_t)nf * 4, st);
         if (e != cudaSuccess) return fail(e);
-        int rc = zola_detect_dev(det, (double*)b_img.p, nf, cap, (double*)b_cand.p, (int*)b_cnt.p, st);
+        // positions and order of every candidate; the offsets of those that get a fit follow per wave
+        int rc = detect_frames(det, (double*)b_img.p, nf, cap, cap, 0, (double*)b_cand.p, (int*)b_cnt.p,
+                               (double*)b_var.p, st);
         if (rc) return rc;
         std::vector<int> counts(nf);
         e = cudaMemcpyAsync(counts.data(), b_cnt.p, (size_t)nf * 4, cudaMemcpyDeviceToHost, st);
@@ -525,7 +614,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 e = cudaMemcpyAsync((double*)g_img.p + k * SS, (double*)b_img.p + (size_t)cut[k] * SS, SS * 8,
                                     cudaMemcpyDeviceToDevice, st);
             if (e != cudaSuccess) return fail(e);
-            rc = zola_detect_dev(det, (double*)g_img.p, (int)nc, cap, (double*)g_out.p, (int*)g_cnt.p, st);
+            rc = detect_frames(det, (double*)g_img.p, (int)nc, cap, cap, 0, (double*)g_out.p, (int*)g_cnt.p, nullptr, st);
             if (rc) return rc;
             for (size_t k = 0; k < nc && e == cudaSuccess; ++k) {
                 e = cudaMemcpyAsync((double*)b_cand.p + (size_t)cut[k] * cap * 7, (double*)g_out.p + k * cap * 7,
@@ -539,13 +628,18 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
             e = cudaMemsetAsync(b_ns.p, 0, 4, st);
             if (e == cudaSuccess) e = cudaMemsetAsync(b_nacc.p, 0, 4, st);
             if (e != cudaSuccess) return fail(e);
-            k_pipe_wave<<<nf, 128, 0, st>>>(V, K);
+            k_pipe_wave<<<nf, PW_THREADS, 0, st>>>(V, K);
             ctx->launches++;
             int nslot = 0;
             e = cudaMemcpyAsync(&nslot, b_ns.p, 4, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) return fail(e);
             if (nslot > 0) {
+                rc = detect_refine(det, (double*)b_img.p, (double*)b_var.p, (double*)b_cand.p, cap, nslot,
+                                   (int*)b_sf.p, (int*)b_sc.p, st);
+                if (rc) return rc;
+                k_pipe_start<<<(nslot + 127) / 128, 128, 0, st>>>(V, nslot);
+                ctx->launches++;
                 rc = scmos ? zola_fit_batch_scmos_dev(ctx, fit_psf, R, (float*)b_rois.p, (float*)b_sv.p,
                                                       (double*)b_init.p, nslot, &fp, (double*)b_out5.p, nullptr,
                                                       nullptr, (int*)b_st.p, nullptr, st)
@@ -564,7 +658,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 rc = launch_model_f64(ctx, fit_psf, wt, (double*)b_xyz.p, nslot, (double*)b_psi.p, nullptr, st,
                                       (const int*)b_list.p, (const int*)b_nlist.p);
                 if (rc) return rc;
-                k_pipe_mthr<<<(nslot + 127) / 128, 128, 0, st>>>(nslot, (int)RR, (double*)b_out5.p,
+                k_pipe_mthr<<<(nslot + 3) / 4, 128, 0, st>>>(nslot, (int)RR, (double*)b_out5.p,
                                                                  (double*)b_psi.p, V.slot_v, (double*)b_mthr.p,
                                                                  (const int*)b_list.p, (const int*)b_nlist.p);
                 ctx->launches++;
@@ -587,7 +681,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 // the walk has used psi; its buffer now takes the accepted positions' models
                 rc = zola_psf_model_dev(fit_psf, R, (double*)b_xyz.p, nacc, (double*)b_psi.p, (double*)b_dpsi.p, st);
                 if (rc) return rc;
-                k_pipe_rows<<<(nacc + 127) / 128, 128, 0, st>>>(V, nacc, (int*)b_acc.p, (int*)b_seq.p, (int*)b_st.p,
+                k_pipe_rows<<<(nacc + 3) / 4, 128, 0, st>>>(V, nacc, (int*)b_acc.p, (int*)b_seq.p, (int*)b_st.p,
                                                                 (double*)b_out5.p, (double*)b_psi.p,
                                                                 (double*)b_dpsi.p, (LocRow*)b_rows.p);
                 ctx->launches++;
