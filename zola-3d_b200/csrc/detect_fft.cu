@@ -30,81 +30,10 @@
 #include <cmath>
 #include <vector>
 
+#include "fft_f64.h"
 #include "zola_internal.h"
 
 namespace zola {
-
-__device__ inline double2 c_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ inline double2 c_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ inline double2 c_mul(double2 a, double2 b) {
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-// a times exp(SIGN i pi / 2)
-template <int SIGN>
-__device__ inline double2 c_rot(double2 a) { return SIGN > 0 ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x); }
-
-template <int SIGN>
-__device__ inline void dft3(double2& a, double2& b, double2& c) {
-    const double h = 0.86602540378443864676;  // sin(2 pi / 3)
-    const double2 s = c_add(b, c), d = c_rot<SIGN>(make_double2(h * (b.x - c.x), h * (b.y - c.y)));
-    const double2 m = make_double2(fma(-0.5, s.x, a.x), fma(-0.5, s.y, a.y));
-    a = c_add(a, s);
-    b = c_add(m, d);
-    c = c_sub(m, d);
-}
-
-template <int SIGN>
-__device__ inline void dft4(double2& a, double2& b, double2& c, double2& d) {
-    const double2 s0 = c_add(a, c), s1 = c_sub(a, c), s2 = c_add(b, d), s3 = c_rot<SIGN>(c_sub(b, d));
-    a = c_add(s0, s2);
-    b = c_add(s1, s3);
-    c = c_sub(s0, s2);
-    d = c_sub(s1, s3);
-}
-
-template <int SIGN, int R>
-__device__ inline void dft(double2 (&x)[R]) {
-    if constexpr (R == 4) {
-        dft4<SIGN>(x[0], x[1], x[2], x[3]);
-    } else if constexpr (R == 5) {
-        const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;  // cos(2 pi k / 5)
-        const double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;   // sin(2 pi k / 5)
-        const double2 p = c_add(x[1], x[4]), q = c_add(x[2], x[3]), u = c_sub(x[1], x[4]), v = c_sub(x[2], x[3]);
-        const double2 e = make_double2(fma(c1, p.x, fma(c2, q.x, x[0].x)), fma(c1, p.y, fma(c2, q.y, x[0].y)));
-        const double2 f = make_double2(fma(c2, p.x, fma(c1, q.x, x[0].x)), fma(c2, p.y, fma(c1, q.y, x[0].y)));
-        const double2 g = c_rot<SIGN>(make_double2(fma(s1, u.x, s2 * v.x), fma(s1, u.y, s2 * v.y)));
-        const double2 h = c_rot<SIGN>(make_double2(fma(s2, u.x, -s1 * v.x), fma(s2, u.y, -s1 * v.y)));
-        x[0] = c_add(x[0], c_add(p, q));
-        x[1] = c_add(e, g);
-        x[4] = c_sub(e, g);
-        x[2] = c_add(f, h);
-        x[3] = c_sub(f, h);
-    } else if constexpr (R == 6) {  // 2 x 3, prime factors: inputs (3a + 2b) mod 6, outputs (3a + 4b) mod 6
-        double2 a[3] = {x[0], x[2], x[4]}, b[3] = {x[3], x[5], x[1]};
-        dft3<SIGN>(a[0], a[1], a[2]);
-        dft3<SIGN>(b[0], b[1], b[2]);
-        x[0] = c_add(a[0], b[0]);
-        x[3] = c_sub(a[0], b[0]);
-        x[4] = c_add(a[1], b[1]);
-        x[1] = c_sub(a[1], b[1]);
-        x[2] = c_add(a[2], b[2]);
-        x[5] = c_sub(a[2], b[2]);
-    } else if constexpr (R == 8) {
-        const double h = 0.70710678118654752440;
-        double2 a[4] = {x[0], x[2], x[4], x[6]}, b[4] = {x[1], x[3], x[5], x[7]};
-        dft4<SIGN>(a[0], a[1], a[2], a[3]);
-        dft4<SIGN>(b[0], b[1], b[2], b[3]);
-        const double2 r1 = c_rot<SIGN>(b[1]), r3 = c_rot<SIGN>(b[3]);
-        b[1] = make_double2(h * (b[1].x + r1.x), h * (b[1].y + r1.y));
-        b[2] = c_rot<SIGN>(b[2]);
-        b[3] = make_double2(h * (r3.x - b[3].x), h * (r3.y - b[3].y));
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            x[q] = c_add(a[q], b[q]);
-            x[q + 4] = c_sub(a[q], b[q]);
-        }
-    }
-}
 
 // A line length M = R0 R1 R2 [R3] and how a CTA runs it, all known at compile
 // time: radices behind a run-time switch put the operands in local memory and

@@ -1,7 +1,7 @@
 // Plain FP64 GPU form of the PSF model and of the per-ROI Poisson MLE fit.
 //
-// One CTA per ROI (persistent grid pulling ROIs from a device counter), all
-// arithmetic in FP64 on the CUDA cores, no tensor cores.  This is the 1x
+// One cluster of CTAs per ROI (persistent grid pulling ROIs from a device
+// counter), all arithmetic in FP64 on the CUDA cores, no tensor cores.  This is the 1x
 // reference the split-precision tcgen05 path is measured against, and the
 // FP64 device model that the parity tests compare with the CPU oracle.
 //
@@ -16,53 +16,112 @@
 // The forward field uses the reference's (cos q, sin r) pair (PSFPhase.java:565-569)
 // so evanescent tables built with resetKz are reproduced; derivatives assume
 // q == r, which holds for the fit tables (kz = 0 where evanescent).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
+#include "fft_f64.h"
 #include "lm.h"
 #include "zola_internal.h"
 
 namespace zola {
 
-constexpr int F64_THREADS = 512;
+// Pupil grids of 64 .. 1024 points (every power of two in use) run the partial
+// DFTs as FFTs (eval_maps_fft); smaller ones, which no camera pixel leads
+// to, as direct sums (eval_maps_direct).
+constexpr int F64_THREADS = 256;
 constexpr int F64_WARPS = F64_THREADS / 32;
 constexpr int F64_NRED = 1 + 5 + 15 + 15;  // nll, g, H (lower), F (lower)
+constexpr int F64_RED_BYTES = 4096;        // reduction areas at the start of shared memory
+constexpr size_t F64_G_SMEM = 56 * 1024;   // blur matrices up to this size are kept in shared memory
 
+// Work areas of a cluster in global memory (they stay in L2).  S holds (w, a) planes
+// of the FFT form and (a, w) planes of the direct form.
 struct F64Work {
-    double2* Q;  // D*D
+    double2* Q;  // D*D (direct form)
     double2* S;  // 3 * D*W
-    double* I;   // 4 * W*W
+    double* I;   // 4 * W*W (direct form)
     double* J;   // 4 * R*W
-    double* T;   // 4 * R*R
+    double* T;   // 4 * R*R: the CTA's rows of map m start at T + m * nt
+    int nt;      // pixels of the CTA's rows
 };
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+__host__ __device__ inline bool f64_fft(int N) { return N >= 64 && N <= 1024; }
 
-__host__ __device__ inline size_t f64_work_bytes(int D, int W, int R) {
+__host__ __device__ inline size_t f64_work_bytes(int N, int D, int W, int R) {
     size_t b = 0;
-    b += align_up((size_t)D * D * 16, 256);
+    if (!f64_fft(N)) b += align_up((size_t)D * D * 16, 256) + align_up((size_t)4 * W * W * 8, 256);
     b += align_up((size_t)3 * D * W * 16, 256);
-    b += align_up((size_t)4 * W * W * 8, 256);
     b += align_up((size_t)4 * R * W * 8, 256);
     b += align_up((size_t)4 * R * R * 8, 256);
     return b;
 }
 
-__device__ inline F64Work f64_carve(char* base, int D, int W, int R) {
-    F64Work w;
+__device__ inline F64Work f64_carve(char* base, int N, int D, int W, int R) {
+    F64Work w{};
     size_t o = 0;
-    w.Q = (double2*)(base + o); o += align_up((size_t)D * D * 16, 256);
+    if (!f64_fft(N)) {
+        w.Q = (double2*)(base + o); o += align_up((size_t)D * D * 16, 256);
+        w.I = (double*)(base + o);  o += align_up((size_t)4 * W * W * 8, 256);
+    }
     w.S = (double2*)(base + o); o += align_up((size_t)3 * D * W * 16, 256);
-    w.I = (double*)(base + o);  o += align_up((size_t)4 * W * W * 8, 256);
     w.J = (double*)(base + o);  o += align_up((size_t)4 * R * W * 8, 256);
     w.T = (double*)(base + o);
     return w;
 }
 
-// Block-wide sum of NV doubles per thread; result in red[0..NV) for all threads.
+// Shared memory of the FFT form: reduction area, transform buffer, one tile of the
+// pupil field (LINES rows of D | 1) or of an intensity map (W x LINES), and the
+// transposed blur matrix (W x R) when it is small enough.
+__host__ __device__ inline size_t f64_tile_bytes(int N, int D, int W) {
+    const size_t lines = 2048 / N, q = lines * (D | 1) * 16, x = (size_t)W * lines * 8;
+    return align_up(q > x ? q : x, 256);
+}
+__host__ __device__ inline size_t f64_smem(int N, int D, int W, int R) {
+    if (!f64_fft(N)) return F64_RED_BYTES;
+    const size_t g = (size_t)W * R * 8;
+    return F64_RED_BYTES + FL_SMEM + f64_tile_bytes(N, D, W) + (g <= F64_G_SMEM ? g : 0);
+}
+
+// The CTAs of a cluster share one ROI or model: each takes its part of the pupil
+// rows, of the window columns and of the pixel rows, and they meet at cluster
+// barriers.  An evaluation then takes a fraction of the time, which is what one ROI,
+// a few of them, or the last slow fits of a batch wait for.
+struct Cluster {
+    unsigned rank, size;
+    __device__ Cluster() {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    }
+    __device__ void sync() const {
+        if (size == 1) __syncthreads();
+        else asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    }
+    // p (in this CTA's shared memory) as CTA r of the cluster has it
+    template <class T>
+    __device__ T read(const T* p, unsigned r) const { return *cooperative_groups::this_cluster().map_shared_rank((T*)p, r); }
+    __device__ unsigned id() const { return blockIdx.x / size; }
+    __device__ unsigned count() const { return gridDim.x / size; }
+    // this CTA's part of the row pairs of an R x R map
+    __device__ int row0(int R) const { return (int)(R / 2 * rank / size) * 2; }
+    __device__ int row1(int R) const { return (int)(R / 2 * (rank + 1) / size) * 2; }
+};
+// CTAs a cluster, by the window's columns (LINES at a time); never by the number of
+// ROIs, so that a result does not depend on its batch.
+__host__ __device__ inline int f64_cluster(int N, int W) {
+    if (!f64_fft(N)) return 1;
+    const int t = W / (2048 / N);
+    return t >= 4 ? 4 : (t >= 2 ? 2 : 1);
+}
+
+// Sum of NV doubles per thread over the cluster; every thread gets it.  red: 9 NV
+// doubles, part: NV doubles of shared memory not used by the previous call.
 template <int NV>
-__device__ inline void block_sum(double (&v)[NV], double* red) {
+__device__ inline void cluster_sum(const Cluster& cl, double (&v)[NV], double* red, double* part) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -79,13 +138,21 @@ __device__ inline void block_sum(double (&v)[NV], double* red) {
     __syncthreads();
     if (threadIdx.x < NV) {
         double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w * NV + threadIdx.x];
+        for (int w = 0; w < F64_WARPS; ++w) s += red[w * NV + threadIdx.x];
+        part[threadIdx.x] = s;
+    }
+    cl.sync();
+    if (threadIdx.x < NV) {
+        double s = part[threadIdx.x];
+        if (cl.size > 1) {
+            s = 0.0;
+            for (unsigned r = 0; r < cl.size; ++r) s += cl.read(part + threadIdx.x, r);
+        }
         red[F64_WARPS * NV + threadIdx.x] = s;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] = red[F64_WARPS * NV + k];
-    __syncthreads();
 }
 
 __device__ inline double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
@@ -95,23 +162,161 @@ __device__ inline double2 cmadd(double2 acc, double2 a, double2 b) {
     return acc;
 }
 
+// Pupil field at (row a, column b): pupil (cos q, sin r).
+__device__ __forceinline__ double2 pupil_field(const PsfView& P, int a, int b, double x, double y, double zoil, double zwat) {
+    const int idx = a * P.D + b;
+    const double pup = P.pupil[idx];
+    if (pup == 0.0) return make_double2(0.0, 0.0);
+    const double pp = P.kx[a] * x + P.ky[b] * y + P.phase[idx];
+    const double q = pp + P.kz[idx] * zwat - P.kzoil[idx] * zoil;
+    const double r = pp + P.kz[idx] * zwat * P.isim[idx] - P.kzoil[idx] * zoil * P.isimoil[idx];
+    double s, c;
+    sincos(q, &s, &c);
+    if (r != q) s = sin(r);
+    return make_double2(pup * c, pup * s);
+}
+
+// The four blurred maps through N-point FFTs.  E[w] = sum_a C[w][a] Q[a] is, up to a
+// sign (-1)^(w - W/2) that |E|^2 and conj(E) E_t do not see, output (w - W/2) mod N of
+// the inverse N-point transform of Q at points a0 .. a0 + D - 1.  Per LINES pupil rows
+// a: Q in shared memory, transforms of Q, i ky Q and i kz Q along b into S (w, a);
+// per LINES window columns: transforms of S, i kx S, S_y, S_z along a, E in registers,
+// each intensity map straight from registers into a shared tile, blurred along its
+// first index there (2 x 2 outputs a thread, two 16-byte loads for four FMAs); then
+// the second blur (4 x 2 outputs a thread).
+// The direct sums took 8 D W (3 D + 4 W) flops, bound by loads from the work area;
+// this takes a sixth of that at N = 128, W = 64 and an eighth at W = 128.  It is bound by
+// latency (20% of the FP64 rate with two CTAs an SM: the barriers between passes and the
+// reads of S), which is why a cluster shares an evaluation.  200 models with derivatives
+// at 32 px (N = 128) 611 -> 124 us; 800 fits of 24 px 15.5 -> 3.8 ms, of which one CTA a
+// fit left 6.8; 26 fits of 42 px 8.4 -> 0.75 ms.
+template <class F>
+__device__ void eval_maps_fft(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w, char* smem,
+                              double x, double y, double zoil, double zwat, bool derivs) {
+    constexpr int N = F::N, L = F::LINES;
+    const int D = P.D, DP = D | 1, W = Wn.W, R = Wn.R, tid = threadIdx.x, a0 = P.a0;
+    double2* buf = (double2*)(smem + F64_RED_BYTES);
+    char* tile = smem + F64_RED_BYTES + FL_SMEM;
+    double2* Qt = (double2*)tile;  // [row][column]
+    double* X = (double*)tile;     // [window row][column]
+    const bool gs = (size_t)W * R * 8 <= F64_G_SMEM;
+    const double* GT = gs ? (const double*)(tile + f64_tile_bytes(N, D, W)) : Wn.GT;
+    const size_t plane = (size_t)W * D;
+    // a CTA takes whole tiles of rows, or, where there are fewer tiles than CTAs, fields
+    const int nf = derivs ? 3 : 1, tiles = (D + L - 1) / L;
+    const bool by_field = tiles < (int)cl.size;
+    for (int t = by_field ? 0 : cl.rank; t < tiles; t += by_field ? 1 : cl.size) {
+        const int r0 = t * L;
+        for (int k = tid; k < L * D; k += FL_THREADS) {
+            const int l = k / D, b = k - l * D;
+            Qt[l * DP + b] = r0 + l < D ? pupil_field(P, r0 + l, b, x, y, zoil, zwat) : make_double2(0, 0);
+        }
+        __syncthreads();
+        for (int f = by_field ? cl.rank : 0; f < nf; f += by_field ? cl.size : 1) {
+            double2* S = w.S + f * plane;
+            auto ld = [&](unsigned k, unsigned l) {
+                const int b = (int)k - a0;
+                if ((unsigned)b >= (unsigned)D) return make_double2(0, 0);
+                const double2 q = Qt[l * DP + b];
+                if (f == 0) return q;
+                const double s = f == 1 ? P.ky[b] : P.kz[min(r0 + (int)l, D - 1) * D + b];
+                return make_double2(-s * q.y, s * q.x);
+            };
+            auto st = [&](unsigned k, unsigned l, int, double2 v) {
+                const unsigned o = (k + W / 2) & (N - 1);
+                if (o < (unsigned)W && r0 + (int)l < D) S[(size_t)o * D + r0 + l] = v;
+            };
+            fl_transform<F, 1>(buf, P.tw, ld, st);
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+    cl.sync();
+    for (int c0 = cl.rank * L; c0 < W; c0 += cl.size * L) {
+        double2 e[FL_OUT];
+        for (int m = 0; m < (derivs ? 4 : 1); ++m) {
+            const double2* S = w.S + (m < 2 ? 0 : m - 1) * plane;
+            auto ld = [&](unsigned k, unsigned l) {
+                const int a = (int)k - a0;
+                if ((unsigned)a >= (unsigned)D || c0 + (int)l >= W) return make_double2(0, 0);
+                const double2 q = S[(size_t)(c0 + l) * D + a];
+                if (m != 1) return q;
+                const double s = P.kx[a];
+                return make_double2(-s * q.y, s * q.x);
+            };
+            auto st = [&](unsigned k, unsigned l, int slot, double2 v) {
+                const unsigned o = (k + W / 2) & (N - 1);
+                if (m == 0) e[slot] = v;
+                if (o < (unsigned)W)
+                    X[o * L + l] = m == 0 ? v.x * v.x + v.y * v.y : 2.0 * (e[slot].x * v.x + e[slot].y * v.y);
+            };
+            fl_transform<F, 1>(buf, P.tw, ld, st);
+            __syncthreads();
+            // J[m][i'][j] = sum_i G[i'][i] I[m][i][j]
+            double* J = w.J + (size_t)m * R * W;
+            for (int t = tid; t < (R / 2) * (L / 2); t += FL_THREADS) {
+                const int rp = t / (L / 2), c = t - rp * (L / 2);
+                const double* g = GT + 2 * rp;
+                const double* xi = X + 2 * c;
+                double s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+#pragma unroll 4
+                for (int i = 0; i < W; ++i) {
+                    const double2 gv = *(const double2*)(g + (size_t)i * R), xv = *(const double2*)(xi + i * L);
+                    s00 = fma(gv.x, xv.x, s00);
+                    s01 = fma(gv.x, xv.y, s01);
+                    s10 = fma(gv.y, xv.x, s10);
+                    s11 = fma(gv.y, xv.y, s11);
+                }
+                if (c0 + 2 * c < W) {
+                    *(double2*)(J + (size_t)(2 * rp) * W + c0 + 2 * c) = make_double2(s00, s01);
+                    *(double2*)(J + (size_t)(2 * rp + 1) * W + c0 + 2 * c) = make_double2(s10, s11);
+                }
+            }
+            __syncthreads();
+        }
+    }
+    cl.sync();
+    // T[m][i'][j'] = sum_j G[j'][j] J[m][i'][j] for the CTA's rows: two rows i', two maps and two j' a thread
+    const int nm = derivs ? 4 : 1, hp = R / 2, i0 = cl.row0(R), pairs = (cl.row1(R) - i0) / 2, mg = derivs ? 2 : 1;
+    for (int t = tid; t < pairs * mg * hp; t += FL_THREADS) {
+        const int u = t / hp, jp = t - u * hp, ip = u / mg, m0 = 2 * (u - ip * mg), m1 = min(m0 + 1, nm - 1);
+        const double* g = GT + 2 * jp;
+        const double* j0 = w.J + ((size_t)m0 * R + i0 + 2 * ip) * W;
+        const double* j1 = w.J + ((size_t)m1 * R + i0 + 2 * ip) * W;
+        double2 s[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = make_double2(0, 0);
+#pragma unroll 4
+        for (int j = 0; j < W; j += 2) {
+            const double2 ga = *(const double2*)(g + (size_t)j * R), gb = *(const double2*)(g + (size_t)(j + 1) * R);
+            const double2 v[4] = {*(const double2*)(j0 + j), *(const double2*)(j0 + W + j), *(const double2*)(j1 + j),
+                                  *(const double2*)(j1 + W + j)};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                s[q].x = fma(gb.x, v[q].y, fma(ga.x, v[q].x, s[q].x));
+                s[q].y = fma(gb.y, v[q].y, fma(ga.y, v[q].x, s[q].y));
+            }
+        }
+        double* o = w.T + 2 * ip * R + 2 * jp;
+        *(double2*)(o + (size_t)m0 * w.nt) = s[0];
+        *(double2*)(o + (size_t)m0 * w.nt + R) = s[1];
+        if (m1 != m0) {
+            *(double2*)(o + (size_t)m1 * w.nt) = s[2];
+            *(double2*)(o + (size_t)m1 * w.nt + R) = s[3];
+        }
+    }
+    __syncthreads();
+}
+
 // Computes the four blurred R x R maps T[0..3] = blurred I, I_x, I_y, I_z
-// (only T[0] when derivs is false).  All threads of the block participate.
-__device__ void eval_maps_f64(const PsfView& P, const WinView& Wn, const F64Work& w, double x, double y,
+// (only T[0] when derivs is false) by direct sums.
+__device__ void eval_maps_direct(const PsfView& P, const WinView& Wn, const F64Work& w, double x, double y,
                               double zoil, double zwat, bool derivs) {
     const int D = P.D, W = Wn.W, R = Wn.R, tid = threadIdx.x, nt = blockDim.x;
     // 1. pupil field on the disk square
     for (int idx = tid; idx < D * D; idx += nt) {
-        int a = idx / D, b = idx - a * D;
-        double pup = P.pupil[idx];
-        double2 q2 = make_double2(0.0, 0.0);
-        if (pup != 0.0) {
-            double pp = P.kx[a] * x + P.ky[b] * y + P.phase[idx];
-            double q = pp + P.kz[idx] * zwat - P.kzoil[idx] * zoil;
-            double r = pp + P.kz[idx] * zwat * P.isim[idx] - P.kzoil[idx] * zoil * P.isimoil[idx];
-            q2 = make_double2(pup * cos(q), pup * sin(r));
-        }
-        w.Q[idx] = q2;
+        const int a = idx / D;
+        w.Q[idx] = pupil_field(P, a, idx - a * D, x, y, zoil, zwat);
     }
     __syncthreads();
     // 2. first contraction over pupil columns b
@@ -229,81 +434,120 @@ __device__ void eval_maps_f64(const PsfView& P, const WinView& Wn, const F64Work
     __syncthreads();
 }
 
+// All threads of the block participate.  NFFT: P.N where it takes the FFT form, else 0.
+template <int NFFT>
+__device__ __forceinline__ void eval_maps_f64(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w,
+                                              char* smem, double x, double y, double zoil, double zwat, bool derivs) {
+    if constexpr (NFFT > 0) eval_maps_fft<FftLines<NFFT>>(cl, P, Wn, w, smem, x, y, zoil, zwat, derivs);
+    else eval_maps_direct(P, Wn, w, x, y, zoil, zwat, derivs);
+}
+
+// A CTA's set-up: the work areas of its cluster, T in the transform buffer (free
+// when the maps are used) where the CTA's rows fit, and the transposed blur matrix in
+// shared memory.
+template <int NFFT>
+__device__ __forceinline__ F64Work f64_begin(const Cluster& cl, const PsfView& P, const WinView& Wn, char* scratch,
+                                             size_t per_cluster, char* smem) {
+    F64Work w = f64_carve(scratch + cl.id() * per_cluster, P.N, P.D, Wn.W, Wn.R);
+    const int i0 = cl.row0(Wn.R);
+    w.nt = (cl.row1(Wn.R) - i0) * Wn.R;
+    if (NFFT > 0 && (size_t)4 * w.nt * 8 <= FL_SMEM) w.T = (double*)(smem + F64_RED_BYTES);
+    else w.T += (size_t)4 * i0 * Wn.R;
+    if constexpr (NFFT > 0) {
+        const int n = Wn.W * Wn.R;
+        if ((size_t)n * 8 <= F64_G_SMEM) {
+            double* g = (double*)(smem + F64_RED_BYTES + FL_SMEM + f64_tile_bytes(NFFT, P.D, Wn.W));
+            for (int k = threadIdx.x; k < n; k += FL_THREADS) g[k] = Wn.GT[k];
+        }
+    }
+    __syncthreads();
+    return w;
+}
+
+// Reduction areas: cluster_sum<36> and cluster_sum<4> have parts of their own.
+__device__ inline double* part_lik(double* red) { return red + (F64_WARPS + 1) * F64_NRED; }
+__device__ inline double* part_norm(double* red) { return part_lik(red) + F64_NRED; }
+
 // Normalisation sums: S = sum |T0|, Dt = sum sgn(T0) T_t.
-__device__ inline void norm_sums(const F64Work& w, int R, bool derivs, double* red, double (&s)[4]) {
+__device__ inline void norm_sums(const Cluster& cl, const F64Work& w, bool derivs, double* red, double (&s)[4]) {
     double v[4] = {0, 0, 0, 0};
     const double* T = w.T;
-    for (int k = threadIdx.x; k < R * R; k += blockDim.x) {
+    for (int k = threadIdx.x; k < w.nt; k += blockDim.x) {
         double t0 = T[k];
         double sg = t0 < 0 ? -1.0 : 1.0;
         v[0] += fabs(t0);
         if (derivs) {
-            v[1] += sg * T[R * R + k];
-            v[2] += sg * T[2 * R * R + k];
-            v[3] += sg * T[3 * R * R + k];
+            v[1] += sg * T[w.nt + k];
+            v[2] += sg * T[2 * w.nt + k];
+            v[3] += sg * T[3 * w.nt + k];
         }
     }
-    block_sum<4>(v, red);
+    cluster_sum<4>(cl, v, red, part_norm(red));
     for (int k = 0; k < 4; ++k) s[k] = v[k];
 }
 
-// Writes psi (and dpsi) of n models; one CTA per model.  With a list, only
+// Writes psi (and dpsi) of n models; one cluster per model.  With a list, only
 // the models list[0 .. *n_dev) are evaluated (position list[m] of xyz, written
 // at the same index of out).
-__global__ void __launch_bounds__(F64_THREADS) model_f64_kernel(PsfView P, WinView Wn, const double* xyz, int n,
-                                                                double* out, double* dout, char* gscratch,
-                                                                size_t per_cta, int use_smem, const int* list,
-                                                                const int* n_dev) {
+template <int NFFT>
+__global__ void __launch_bounds__(F64_THREADS, 2) model_f64_kernel(PsfView P, WinView Wn, const double* xyz, int n,
+                                                                   double* out, double* dout, char* gscratch,
+                                                                   size_t per_cluster, const int* list,
+                                                                   const int* n_dev) {
     extern __shared__ __align__(256) char smem_raw[];
     double* red = (double*)smem_raw;
-    char* base = use_smem ? smem_raw + 8192 : gscratch + (size_t)blockIdx.x * per_cta;
-    F64Work w = f64_carve(base, P.D, Wn.W, Wn.R);
-    const int R = Wn.R;
+    const Cluster cl;
+    const F64Work w = f64_begin<NFFT>(cl, P, Wn, gscratch, per_cluster, smem_raw);
+    const int R = Wn.R, nt = w.nt;
+    const size_t RR = (size_t)R * R, px0 = (size_t)cl.row0(R) * R;
     const bool derivs = dout != nullptr;
     const int nn = n_dev ? min(n, *n_dev) : n;
-    for (int mi = blockIdx.x; mi < nn; mi += gridDim.x) {
+    for (int mi = cl.id(); mi < nn; mi += cl.count()) {
         const int m = list ? list[mi] : mi;
-        eval_maps_f64(P, Wn, w, xyz[3 * m], xyz[3 * m + 1], P.zfocus, xyz[3 * m + 2], derivs);
+        eval_maps_f64<NFFT>(cl, P, Wn, w, smem_raw, xyz[3 * m], xyz[3 * m + 1], P.zfocus, xyz[3 * m + 2], derivs);
         double s[4];
-        norm_sums(w, R, derivs, red, s);
-        for (int k = threadIdx.x; k < R * R; k += blockDim.x) {
+        norm_sums(cl, w, derivs, red, s);
+        for (int k = threadIdx.x; k < nt; k += blockDim.x) {
             double t0 = w.T[k];
             double sg = t0 < 0 ? -1.0 : 1.0;
             double psi = fabs(t0) / s[0];
-            out[(size_t)m * R * R + k] = psi;
+            out[m * RR + px0 + k] = psi;
             if (derivs)
                 for (int d = 0; d < 3; ++d)
-                    dout[((size_t)m * 3 + d) * R * R + k] = (sg * w.T[(d + 1) * R * R + k] - psi * s[d + 1]) / s[0];
+                    dout[((size_t)m * 3 + d) * RR + px0 + k] = (sg * w.T[(d + 1) * nt + k] - psi * s[d + 1]) / s[0];
         }
         __syncthreads();
     }
+    cl.sync();  // no CTA leaves while another may read its shared memory
 }
 
 // Likelihood, gradient, Gauss-Newton Hessian and Fisher matrix at theta.
 // sv (nullable): the ROI's sCMOS term var/gain^2, added to the mean
 // (process/cpu/Localization.java:1132).
-__device__ void eval_lik_f64(const PsfView& P, const WinView& Wn, const F64Work& w, const float* d, const float* sv,
-                             const double* th, double* red, double& nll, double* g, double* H, double* F) {
-    const int R = Wn.R;
-    eval_maps_f64(P, Wn, w, th[0], th[1], P.zfocus, th[2], true);
+template <int NFFT>
+__device__ void eval_lik_f64(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w, char* smem,
+                             const float* d, const float* sv, const double* th, double* red, double& nll, double* g,
+                             double* H, double* F) {
+    const int px0 = cl.row0(Wn.R) * Wn.R, nt = w.nt;
+    eval_maps_f64<NFFT>(cl, P, Wn, w, smem, th[0], th[1], P.zfocus, th[2], true);
     double s[4];
-    norm_sums(w, R, true, red, s);
+    norm_sums(cl, w, true, red, s);
     double v[F64_NRED];
 #pragma unroll
     for (int k = 0; k < F64_NRED; ++k) v[k] = 0.0;
     const double A = th[3], B = th[4];
     bool bad = false;
-    for (int k = threadIdx.x; k < R * R; k += blockDim.x) {
+    for (int k = threadIdx.x; k < nt; k += blockDim.x) {
         double t0 = w.T[k];
         double sg = t0 < 0 ? -1.0 : 1.0;
         double psi = fabs(t0) / s[0];
         double j[5];
-        for (int q = 0; q < 3; ++q) j[q] = A * (sg * w.T[(q + 1) * R * R + k] - psi * s[q + 1]) / s[0];
+        for (int q = 0; q < 3; ++q) j[q] = A * (sg * w.T[(q + 1) * nt + k] - psi * s[q + 1]) / s[0];
         j[3] = psi;
         j[4] = 1.0;
-        double mu = A * psi + B + (sv ? (double)sv[k] : 0.0);
+        double mu = A * psi + B + (sv ? (double)sv[px0 + k] : 0.0);
         if (!(mu > 0.0)) { bad = true; continue; }
-        double dk = (double)d[k];
+        double dk = (double)d[px0 + k];
         v[0] += dk > 0 ? mu - dk - dk * log(mu / dk) : mu;
         double wg = 1.0 - dk / mu, wh = dk / (mu * mu), wf = 1.0 / mu;
         int o = 1;
@@ -320,7 +564,7 @@ __device__ void eval_lik_f64(const PsfView& P, const WinView& Wn, const F64Work&
             }
     }
     if (bad) v[0] = INFINITY;
-    block_sum<F64_NRED>(v, red);
+    cluster_sum<F64_NRED>(cl, v, red, part_lik(red));
     nll = v[0];
     for (int q = 0; q < 5; ++q) g[q] = v[1 + q];
     int o = 6;
@@ -332,84 +576,119 @@ __device__ void eval_lik_f64(const PsfView& P, const WinView& Wn, const F64Work&
         }
 }
 
-__global__ void __launch_bounds__(F64_THREADS) fit_f64_kernel(PsfView P, WinView Wn, const float* rois,
-                                                              const float* scmos, const double* init, int n,
-                                                              FitParamsDev prm,
-                                                              double* out5, double* crlb5, double* nll_out,
-                                                              int* st_out, int* it_out, char* gscratch,
-                                                              size_t per_cta, int use_smem, int* counter) {
+template <int NFFT>
+__global__ void __launch_bounds__(F64_THREADS, 2) fit_f64_kernel(PsfView P, WinView Wn, const float* rois,
+                                                                 const float* scmos, const double* init, int n,
+                                                                 FitParamsDev prm, double* out5, double* crlb5,
+                                                                 double* nll_out, int* st_out, int* it_out,
+                                                                 char* gscratch, size_t per_cluster, int* counter) {
     extern __shared__ __align__(256) char smem_raw[];
-    double* red = (double*)smem_raw;  // 8192-byte reduction area
-    __shared__ LMState st;
+    double* red = (double*)smem_raw;  // reduction area
+    __shared__ LMState st;            // every CTA of the cluster steps its own copy, from the same sums
     __shared__ int roi;
     __shared__ int go;
-    char* base = use_smem ? smem_raw + 8192 : gscratch + (size_t)blockIdx.x * per_cta;
-    F64Work w = f64_carve(base, P.D, Wn.W, Wn.R);
+    const Cluster cl;
+    const F64Work w = f64_begin<NFFT>(cl, P, Wn, gscratch, per_cluster, smem_raw);
     const int R = Wn.R;
     for (;;) {
-        if (threadIdx.x == 0) roi = atomicAdd(counter, 1);
-        __syncthreads();
-        const int r = roi;
+        if (cl.rank == 0 && threadIdx.x == 0) roi = atomicAdd(counter, 1);
+        cl.sync();
+        const int r = cl.size > 1 ? cl.read(&roi, 0) : roi;
         if (r >= n) break;
         const float* d = rois + (size_t)r * R * R;
         const float* sv = scmos ? scmos + (size_t)r * R * R : nullptr;
         if (threadIdx.x == 0) {
-            for (int q = 0; q < 5; ++q) st.th[q] = init[5 * r + q];
-            lm_clamp(st.th, prm);
+            for (int q = 0; q < 5; ++q) st.trial[q] = init[5 * r + q];
+            lm_clamp(st.trial, prm);
+            st.status = 0;  // nothing evaluated yet
         }
         __syncthreads();
         double th[5], nll, g[5], H[25], F[25];
-        for (int q = 0; q < 5; ++q) th[q] = st.th[q];
-        eval_lik_f64(P, Wn, w, d, sv, th, red, nll, g, H, F);
-        if (threadIdx.x == 0) {
-            lm_start(st, nll, g, H, F, prm);
-            go = lm_propose(st, prm) ? 1 : 0;
-        }
-        __syncthreads();
-        while (go) {
+        do {
             for (int q = 0; q < 5; ++q) th[q] = st.trial[q];
-            eval_lik_f64(P, Wn, w, d, sv, th, red, nll, g, H, F);
+            eval_lik_f64<NFFT>(cl, P, Wn, w, smem_raw, d, sv, th, red, nll, g, H, F);
             if (threadIdx.x == 0) {
-                lm_update(st, nll, g, H, F, prm);
+                if (st.status == 0) {
+                    for (int q = 0; q < 5; ++q) st.th[q] = th[q];
+                    lm_start(st, nll, g, H, F, prm);
+                } else {
+                    lm_update(st, nll, g, H, F, prm);
+                }
                 go = lm_propose(st, prm) ? 1 : 0;
             }
             __syncthreads();
-        }
-        if (threadIdx.x == 0) {
+        } while (go);
+        if (cl.rank == 0 && threadIdx.x == 0) {
             for (int q = 0; q < 5; ++q) out5[5 * r + q] = st.th[q];
             if (nll_out) nll_out[r] = st.nll;
             if (st_out) st_out[r] = st.status;
             if (it_out) it_out[r] = st.evals;
             if (crlb5) lm_crlb(st.F, crlb5 + 5 * r);
         }
-        __syncthreads();
+        cl.sync();  // roi is written again
+    }
+    cl.sync();  // no CTA leaves while another may read its shared memory
+}
+
+// fn(integral constant): NFFT of a pupil grid.
+template <class FN>
+static void with_fft(int N, const FN& fn) {
+    switch (N) {
+        case 64: fn(std::integral_constant<int, 64>()); break;
+        case 128: fn(std::integral_constant<int, 128>()); break;
+        case 256: fn(std::integral_constant<int, 256>()); break;
+        case 512: fn(std::integral_constant<int, 512>()); break;
+        case 1024: fn(std::integral_constant<int, 1024>()); break;
+        default: fn(std::integral_constant<int, 0>());
     }
 }
 
-static int f64_layout(zola_ctx* ctx, zola_psf* p, WindowTables* w, int nblocks, size_t& per_cta, int& use_smem,
-                      size_t& smem, std::string& err) {
-    per_cta = f64_work_bytes(p->D, w->W, w->R);
-    use_smem = per_cta + 8192 <= 200 * 1024;
-    smem = 8192 + (use_smem ? per_cta : 0);
-    if (!use_smem) {
-        if (ensure_scratch(ctx, per_cta * (size_t)nblocks, err)) return ZOLA_E_CUDA;
-    }
-    return 0;
+// Launch configuration for n ROIs or models: as many clusters as run at once (at
+// most `most`).  attr and cfg live as long as the launch.
+template <class K>
+static cudaError_t f64_config(K kernel, const zola_psf* p, const WindowTables* w, int n, long long most, cudaStream_t st,
+                              cudaLaunchAttribute* attr, cudaLaunchConfig_t* cfg, int* clusters) {
+    const int C = f64_cluster(p->N, w->W);
+    const size_t smem = f64_smem(p->N, p->D, w->W, w->R);
+    *cfg = cudaLaunchConfig_t();
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = C;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+    cfg->blockDim = dim3(F64_THREADS);
+    cfg->gridDim = dim3(C);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int at_once = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&at_once, kernel, cfg);
+    *clusters = (int)std::min<long long>(std::min(n, std::max(1, at_once)), most);
+    cfg->gridDim = dim3(C * *clusters);
+    return e;
 }
 
 int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n, double* d_out,
                      double* d_dout, cudaStream_t st, const int* d_list, const int* d_count) {
     if (n <= 0) return ZOLA_OK;
-    int nblocks = std::min(n, ctx->num_sms * 2);
-    size_t per_cta, smem;
-    int use_smem;
-    if (f64_layout(ctx, p, w, nblocks, per_cta, use_smem, smem, ctx->err)) return ZOLA_E_CUDA;
-    ZOLA_CUDA_CHECK(cudaFuncSetAttribute(model_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), ctx);
-    WinView wv{w->R, w->W, w->d_C, w->d_G};
-    prof_begin(ctx, 6, st);
-    model_f64_kernel<<<nblocks, F64_THREADS, smem, st>>>(p->view, wv, d_xyz, n, d_out, d_dout, (char*)ctx->scratch,
-                                                         per_cta, use_smem, d_list, d_count);
-    prof_end(ctx, st);
+    const size_t per_cluster = f64_work_bytes(p->N, p->D, w->W, w->R);
+    WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
+    int rc = ZOLA_OK;
+    with_fft(p->N, [&](auto nfft) {
+        auto kernel = model_f64_kernel<decltype(nfft)::value>;
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg;
+        int clusters = 0;
+        cudaError_t e = f64_config(kernel, p, w, n, n, st, &attr, &cfg, &clusters);
+        if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) { rc = ZOLA_E_CUDA; return; }
+        prof_begin(ctx, 6, st);
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, kernel, p->view, wv, d_xyz, n, d_out, d_dout, (char*)ctx->scratch, per_cluster,
+                                   d_list, d_count);
+        prof_end(ctx, st);
+        if (e != cudaSuccess) { ctx->err = std::string("model: ") + cudaGetErrorString(e); rc = ZOLA_E_CUDA; }
+    });
+    if (rc) return rc;
     ctx->launches++;
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
     return ZOLA_OK;
@@ -419,21 +698,26 @@ int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_r
                    const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
                    double* d_nll, int* d_status, int* d_iters, cudaStream_t st) {
     if (n <= 0) return ZOLA_OK;
-    int nblocks = std::min(n, ctx->num_sms * 2);
-    size_t per_cta, smem;
-    int use_smem;
-    if (f64_layout(ctx, p, w, nblocks, per_cta, use_smem, smem, ctx->err)) return ZOLA_E_CUDA;
-    if (use_smem && smem > 110 * 1024) nblocks = std::min(n, ctx->num_sms);
-    ZOLA_CUDA_CHECK(cudaFuncSetAttribute(fit_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), ctx);
+    const size_t per_cluster = f64_work_bytes(p->N, p->D, w->W, w->R);
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
-    WinView wv{w->R, w->W, w->d_C, w->d_G};
+    WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
     ZOLA_CUDA_CHECK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int), st), ctx);
-    prof_begin(ctx, 5, st);
-    fit_f64_kernel<<<nblocks, F64_THREADS, smem, st>>>(p->view, wv, d_rois, d_scmos, d_init, n, fp, d_out5, d_crlb5,
-                                                       d_nll,
-                                                       d_status, d_iters, (char*)ctx->scratch, per_cta, use_smem,
-                                                       ctx->d_counter);
-    prof_end(ctx, st);
+    int rc = ZOLA_OK;
+    with_fft(p->N, [&](auto nfft) {
+        auto kernel = fit_f64_kernel<decltype(nfft)::value>;
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg;
+        int clusters = 0;
+        cudaError_t e = f64_config(kernel, p, w, n, n, st, &attr, &cfg, &clusters);
+        if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) { rc = ZOLA_E_CUDA; return; }
+        prof_begin(ctx, 5, st);
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, kernel, p->view, wv, d_rois, d_scmos, d_init, n, fp, d_out5, d_crlb5, d_nll,
+                                   d_status, d_iters, (char*)ctx->scratch, per_cluster, ctx->d_counter);
+        prof_end(ctx, st);
+        if (e != cudaSuccess) { ctx->err = std::string("fit: ") + cudaGetErrorString(e); rc = ZOLA_E_CUDA; }
+    });
+    if (rc) return rc;
     ctx->launches++;
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
     return ZOLA_OK;
@@ -553,36 +837,34 @@ extern "C" int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois,
     }
     char* base = (char*)noalloc_scratch(ctx->device, ctx->err);
     if (!base) return ZOLA_E_CUDA;
-    const size_t per_cta = f64_work_bytes(psf->D, w->W, w->R);
-    const int use_smem = per_cta + 8192 <= 200 * 1024;
-    const size_t smem = 8192 + (use_smem ? per_cta : 0);
+    const size_t per_cluster = f64_work_bytes(psf->N, psf->D, w->W, w->R);
     int* counter = (int*)base;
     char* work = base + 256;
     const size_t room = NOALLOC_SCRATCH_BYTES - 256;
-    int nblocks = std::min(n, ctx->num_sms * 2);
-    if (use_smem && smem > 110 * 1024) nblocks = std::min(n, ctx->num_sms);
-    if (!use_smem) {
-        if (per_cta > room) {
-            ctx->err = "zola_fit_batch_noalloc: one block's work area (" + std::to_string(per_cta) +
-                       " bytes for this ROI size) exceeds the 64 MiB static scratch";
-            return ZOLA_E_ARG;
-        }
-        nblocks = std::min<long long>(nblocks, (long long)(room / per_cta));
+    // The windows that are refused: those whose field, transform and intensity planes
+    // would not fit the array together (the FFT form itself keeps fewer planes).
+    const size_t D = psf->D, W = w->W, planes = (D * D + 3 * D * W) * 16 + (4 * W * W + 4 * R * W + 4 * (size_t)R * R) * 8;
+    if (per_cluster > room || planes > room) {
+        ctx->err = "zola_fit_batch_noalloc: one block's work area (" + std::to_string(std::max(planes, per_cluster)) +
+                   " bytes for this ROI size) exceeds the 64 MiB static scratch";
+        return ZOLA_E_ARG;
     }
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    cudaError_t e = cudaFuncSetAttribute(fit_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaMemsetAsync(counter, 0, sizeof(int), st);
-    if (e != cudaSuccess) {
-        ctx->err = std::string("zola_fit_batch_noalloc: ") + cudaGetErrorString(e);
-        return ZOLA_E_CUDA;
-    }
+    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
-    WinView wv{w->R, w->W, w->d_C, w->d_G};
-    fit_f64_kernel<<<nblocks, F64_THREADS, smem, st>>>(psf->view, wv, d_rois, nullptr, d_init5, n, fp, d_out5,
-                                                       d_crlb5, d_nll,
-                                                       d_status, d_iters, work, per_cta, use_smem, counter);
-    ctx->launches++;
-    e = cudaGetLastError();
+    WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
+    if (e == cudaSuccess)
+        with_fft(psf->N, [&](auto nfft) {
+            auto kernel = fit_f64_kernel<decltype(nfft)::value>;
+            cudaLaunchAttribute attr;
+            cudaLaunchConfig_t cfg;
+            int clusters = 0;
+            e = f64_config(kernel, psf, w, n, (long long)(room / per_cluster), st, &attr, &cfg, &clusters);
+            if (e != cudaSuccess) return;
+            e = cudaLaunchKernelEx(&cfg, kernel, psf->view, wv, d_rois, (const float*)nullptr, d_init5, n, fp, d_out5,
+                                   d_crlb5, d_nll, d_status, d_iters, work, per_cluster, counter);
+            ctx->launches++;
+        });
     if (e != cudaSuccess) {
         ctx->err = std::string("zola_fit_batch_noalloc: ") + cudaGetErrorString(e);
         return ZOLA_E_CUDA;

@@ -118,19 +118,25 @@ int build_psf_tables(zola_psf* p, const zola_optics* o, const double* zern, int 
                 p->pupil[k] = 1.0 / std::sqrt((double)K);
             }
         }
-    // upload: 6 D*D arrays + 2 D arrays
-    size_t total = 6 * DD + 2 * (size_t)D;
+    // upload: 2 N twiddle components, 6 D*D arrays, 2 D arrays
+    size_t total = 2 * (size_t)N + 6 * DD + 2 * (size_t)D;
     std::vector<double> h(total);
     double* w = h.data();
     auto put = [&](const std::vector<double>& v) { std::memcpy(w, v.data(), v.size() * sizeof(double)); w += v.size(); };
-    put(p->pupil); put(p->phase); put(p->kz); put(p->kzoil); put(p->isim); put(p->isimoil); put(p->kx); put(p->ky);
+    std::vector<double> tw(2 * (size_t)N);
+    for (int k = 0; k < N; ++k) {
+        tw[2 * k] = std::cos(2 * M_PI * k / N);
+        tw[2 * k + 1] = -std::sin(2 * M_PI * k / N);
+    }
+    put(tw); put(p->pupil); put(p->phase); put(p->kz); put(p->kzoil); put(p->isim); put(p->isimoil); put(p->kx); put(p->ky);
     cudaError_t e = cudaMalloc(&p->d_tables, total * sizeof(double));
     if (e != cudaSuccess) { err = std::string("cudaMalloc: ") + cudaGetErrorString(e); return ZOLA_E_CUDA; }
     e = cudaMemcpy(p->d_tables, h.data(), total * sizeof(double), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { err = std::string("cudaMemcpy: ") + cudaGetErrorString(e); return ZOLA_E_CUDA; }
     PsfView& pv = p->view;
     pv.N = N; pv.D = D; pv.a0 = a0; pv.dx = dx; pv.zfocus = o->zfocus;
-    pv.pupil = p->d_tables; pv.phase = pv.pupil + DD; pv.kz = pv.phase + DD; pv.kzoil = pv.kz + DD;
+    pv.tw = (const double2*)p->d_tables;
+    pv.pupil = p->d_tables + 2 * (size_t)N; pv.phase = pv.pupil + DD; pv.kz = pv.phase + DD; pv.kzoil = pv.kz + DD;
     pv.isim = pv.kzoil + DD; pv.isimoil = pv.isim + DD; pv.kx = pv.isimoil + DD; pv.ky = pv.kx + D;
     return ZOLA_OK;
 }
@@ -205,8 +211,12 @@ WindowTables* get_window(zola_psf* p, int R, std::string& err) {
     blur_matrix(R, W, p->o.sigma, t.G, nullptr);
     cudaError_t e = cudaMalloc(&t.d_C, t.C.size() * sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpy(t.d_C, t.C.data(), t.C.size() * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&t.d_G, t.G.size() * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemcpy(t.d_G, t.G.data(), t.G.size() * sizeof(double), cudaMemcpyHostToDevice);
+    std::vector<double> g(2 * t.G.size());
+    for (int i = 0; i < R; ++i)
+        for (int k = 0; k < W; ++k) g[(size_t)i * W + k] = g[t.G.size() + (size_t)k * R + i] = t.G[(size_t)i * W + k];
+    if (e == cudaSuccess) e = cudaMalloc(&t.d_G, g.size() * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemcpy(t.d_G, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice);
+    t.d_GT = t.d_G + t.G.size();
     if (e != cudaSuccess) {
         err = std::string("window tables: ") + cudaGetErrorString(e);
         return nullptr;

@@ -29,6 +29,7 @@ struct PsfView {
     const double* isimoil;  // D*D
     const double* kx;       // D   (kx of row a)
     const double* ky;       // D   (ky of column b)
+    const double2* tw;      // N   exp(-2 pi i k / N)
 };
 
 // Per-ROI-size tables: the partial-DFT twiddles and the circular blur.
@@ -37,6 +38,7 @@ struct WinView {
     int W;          // intensity window, pow2(min(2R, N)) (PSFPhase.java:100-108)
     const double2* C;   // W x D: C[w][a] = exp(+2 pi i ((a0+a+N/2)(w-W/2) mod N) / N)
     const double* G;    // R x W: blur row i' <- window row i (circulant, see optics.cpp)
+    const double* GT;   // W x R: its transpose
 };
 
 struct FitParamsDev {
@@ -68,7 +70,8 @@ struct WindowTables {
     std::vector<double> C;     // W*D*2 interleaved
     std::vector<double> G;     // R*W
     double2* d_C = nullptr;
-    double* d_G = nullptr;
+    double* d_G = nullptr;   // R*W, then its transpose d_GT (W*R)
+    double* d_GT = nullptr;
     // split-precision operand packs (tcgen05 path), built lazily
     void* d_split = nullptr;
     size_t split_bytes = 0;
