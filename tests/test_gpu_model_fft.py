@@ -55,7 +55,7 @@ def reference(N, R, zern, xyz, kz_reset, na, sigma=0.9, dx=0.11, lam=0.66, n=1.5
 
 
 @pytest.mark.parametrize("N,R,na,kz_reset", [
-    (32, 8, 1.4, False), (32, 32, 1.4, False),                     # direct sums
+    (8, 4, 1.4, False), (16, 16, 1.4, False), (32, 8, 1.4, False), (32, 32, 1.4, False),  # one tile
     (64, 4, 1.4, False), (64, 16, 1.4, False), (64, 18, 1.4, True), (64, 64, 1.4, False),   # one CTA, two
     (128, 6, 1.4, False), (128, 16, 1.4, False), (128, 18, 1.2, False), (128, 50, 1.4, True),  # one, two, four
     (128, 30, 0.45, False), (128, 128, 1.4, False),                # fewer row tiles than CTAs; the whole grid

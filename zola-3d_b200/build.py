@@ -7,6 +7,7 @@ next to this file.  Objects go to _build/ (git-ignored).
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -30,7 +31,7 @@ def headers():
 def build(force=False, verbose=False, ptxas_v=False):
     os.makedirs(BUILD, exist_ok=True)
     hdr_t = max(os.path.getmtime(h) for h in headers())
-    objs = []
+    objs, todo = [], []
     for src in sources():
         obj = os.path.join(BUILD, os.path.basename(src) + ".o")
         objs.append(obj)
@@ -40,7 +41,9 @@ def build(force=False, verbose=False, ptxas_v=False):
                 cmd = [NVCC] + FLAGS + ["-x", "cu"] + ARCH + ["-c", src, "-o", obj]
             if verbose:
                 print(" ".join(cmd), flush=True)
-            subprocess.check_call(cmd)
+            todo.append(cmd)
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        list(pool.map(subprocess.check_call, todo))
     if force or not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(o) for o in objs):
         cmd = [NVCC] + ARCH + ["-shared", "-o", LIB] + objs + ["-lcudart", "-Xlinker", "-rpath",
                                                               "-Xlinker", "/usr/local/cuda/lib64"]

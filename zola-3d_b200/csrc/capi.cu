@@ -213,6 +213,7 @@ int zola_psf_load(zola_ctx* ctx, const zola_optics* optics, const double* zernik
     int rc = build_psf_tables(p, optics, zernike, nz, ctx->err);
     if (rc) {
         if (p->d_tables) cudaFree(p->d_tables);
+        if (p->d_calZ) cudaFree(p->d_calZ);
         delete p;
         return rc;
     }
@@ -230,6 +231,7 @@ int zola_psf_free(zola_psf* psf) {
         if (kv.second.d_split) free_split_plan(kv.second.d_split);
     }
     if (psf->d_tables) cudaFree(psf->d_tables);
+    if (psf->d_calZ) cudaFree(psf->d_calZ);
     delete psf;
     return ZOLA_OK;
 }

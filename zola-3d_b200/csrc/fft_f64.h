@@ -1,8 +1,11 @@
 // FP64 Fourier transforms inside a CTA: complex arithmetic, small DFTs, and the
-// transform of LINES lines of N = 64 .. 1024 points by 256 threads.
+// transform of LINES lines of N = 4 .. 1024 points by 256 threads; clusters.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 namespace zola {
 
@@ -88,8 +91,9 @@ constexpr int FL_THREADS = 256, FL_OUT = 8;
 template <int N_>
 struct FftLines {
     static constexpr int N = N_, LINES = 2048 / N_;
-    static constexpr int R0 = 8, R1 = N == 128 ? 4 : 8, R2 = N == 64 ? 1 : (N == 512 ? 8 : 4), R3 = N == 1024 ? 4 : 1;
-    static_assert(R0 * R1 * R2 * R3 == N, "64 .. 1024 points");
+    static constexpr int R0 = N == 4 || N == 16 ? 4 : 8, R1 = N <= 8 ? 1 : (N <= 32 || N == 128 ? 4 : 8),
+                         R2 = N <= 64 ? 1 : (N == 512 ? 8 : 4), R3 = N == 1024 ? 4 : 1;
+    static_assert(R0 * R1 * R2 * R3 == N, "4 .. 1024 points");
 };
 constexpr size_t FL_SMEM = 2048 * sizeof(double2);
 
@@ -135,9 +139,116 @@ __device__ __forceinline__ void fl_pass(double2* sm, const double2* tw, const LD
 template <class F, int SIGN, class LD, class ST>
 __device__ __forceinline__ void fl_transform(double2* sm, const double2* tw, const LD& ld, const ST& st) {
     fl_pass<F, SIGN, F::R0, 1>(sm, tw, ld, st);
-    fl_pass<F, SIGN, F::R1, F::R0>(sm, tw, ld, st);
+    if constexpr (F::R1 > 1) fl_pass<F, SIGN, F::R1, F::R0>(sm, tw, ld, st);
     if constexpr (F::R2 > 1) fl_pass<F, SIGN, F::R2, F::R0 * F::R1>(sm, tw, ld, st);
     if constexpr (F::R3 > 1) fl_pass<F, SIGN, F::R3, F::R0 * F::R1 * F::R2>(sm, tw, ld, st);
+}
+
+constexpr int FL_WARPS = FL_THREADS / 32;
+
+// The CTAs of a cluster share one ROI, model or bead slice: each takes its part of the pupil
+// rows, of the window columns and of the pixel rows, and they meet at cluster
+// barriers.  An evaluation then takes a fraction of the time, which is what one ROI,
+// a few of them, or the last slow fits of a batch wait for.
+struct Cluster {
+    unsigned rank, size;
+    __device__ Cluster() {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    }
+    __device__ void sync() const {
+        if (size == 1) __syncthreads();
+        else asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    }
+    // p (in this CTA's shared memory) as CTA r of the cluster has it
+    template <class T>
+    __device__ T read(const T* p, unsigned r) const { return *cooperative_groups::this_cluster().map_shared_rank((T*)p, r); }
+    __device__ unsigned id() const { return blockIdx.x / size; }
+    __device__ unsigned count() const { return gridDim.x / size; }
+    // this CTA's part of the row pairs of an R x R map
+    __device__ int row0(int R) const { return (int)(R / 2 * rank / size) * 2; }
+    __device__ int row1(int R) const { return (int)(R / 2 * (rank + 1) / size) * 2; }
+};
+// CTAs a cluster, by the window's columns (LINES at a time); never by the number of
+// ROIs, so that a result does not depend on its batch.
+__host__ __device__ inline int f64_cluster(int N, int W) {
+    const int t = W / (2048 / N);
+    return t >= 4 ? 4 : (t >= 2 ? 2 : 1);
+}
+
+// Sum of NV doubles per thread over the cluster; every thread gets it.  red: 9 NV
+// doubles, part: NV doubles of shared memory not used by the previous call.
+template <int NV>
+__device__ inline void cluster_sum(const Cluster& cl, double (&v)[NV], double* red, double* part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        double x = v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        v[k] = x;
+    }
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) red[warp * NV + k] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double s = 0.0;
+        for (int w = 0; w < FL_WARPS; ++w) s += red[w * NV + threadIdx.x];
+        part[threadIdx.x] = s;
+    }
+    cl.sync();
+    if (threadIdx.x < NV) {
+        double s = part[threadIdx.x];
+        if (cl.size > 1) {
+            s = 0.0;
+            for (unsigned r = 0; r < cl.size; ++r) s += cl.read(part + threadIdx.x, r);
+        }
+        red[FL_WARPS * NV + threadIdx.x] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = red[FL_WARPS * NV + k];
+}
+
+// J[i'][c0 + c] = sum_i G[i'][i] X[i][c] for a shared tile X (W x L, L the row stride)
+// of `cols` columns: two rows i' by two columns a thread, two 16-byte loads for four
+// FMAs.  GT = the transposed blur matrix (W x R).  J has W columns.
+__device__ __forceinline__ void blur_tile(const double* GT, const double* X, int R, int W, int L, int cols, double* J) {
+    const int hc = cols / 2;
+    for (int t = threadIdx.x; t < (R / 2) * hc; t += FL_THREADS) {
+        const int rp = t / hc, c = t - rp * hc;
+        const double *g = GT + 2 * rp, *xi = X + 2 * c;
+        double s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+#pragma unroll 4
+        for (int i = 0; i < W; ++i) {
+            const double2 gv = *(const double2*)(g + (size_t)i * R), xv = *(const double2*)(xi + i * L);
+            s00 = fma(gv.x, xv.x, s00);
+            s01 = fma(gv.x, xv.y, s01);
+            s10 = fma(gv.y, xv.x, s10);
+            s11 = fma(gv.y, xv.y, s11);
+        }
+        *(double2*)(J + (size_t)(2 * rp) * W + 2 * c) = make_double2(s00, s01);
+        *(double2*)(J + (size_t)(2 * rp + 1) * W + 2 * c) = make_double2(s10, s11);
+    }
+}
+
+// fn(integral constant N): the transforms of an N-point pupil grid.
+template <class FN>
+inline void with_fft(int N, const FN& fn) {
+    switch (N) {
+        case 4: fn(std::integral_constant<int, 4>()); break;
+        case 8: fn(std::integral_constant<int, 8>()); break;
+        case 16: fn(std::integral_constant<int, 16>()); break;
+        case 32: fn(std::integral_constant<int, 32>()); break;
+        case 64: fn(std::integral_constant<int, 64>()); break;
+        case 128: fn(std::integral_constant<int, 128>()); break;
+        case 256: fn(std::integral_constant<int, 256>()); break;
+        case 512: fn(std::integral_constant<int, 512>()); break;
+        case 1024: fn(std::integral_constant<int, 1024>()); break;
+    }
 }
 
 }  // namespace zola

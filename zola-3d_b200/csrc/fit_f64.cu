@@ -16,12 +16,10 @@
 // The forward field uses the reference's (cos q, sin r) pair (PSFPhase.java:565-569)
 // so evanescent tables built with resetKz are reproduced; derivatives assume
 // q == r, which holds for the fit tables (kz = 0 where evanescent).
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <mutex>
-#include <type_traits>
 
 #include "fft_f64.h"
 #include "lm.h"
@@ -29,52 +27,39 @@
 
 namespace zola {
 
-// Pupil grids of 64 .. 1024 points (every power of two in use) run the partial
-// DFTs as FFTs (eval_maps_fft); smaller ones, which no camera pixel leads
-// to, as direct sums (eval_maps_direct).
-constexpr int F64_THREADS = 256;
-constexpr int F64_WARPS = F64_THREADS / 32;
+constexpr int F64_THREADS = FL_THREADS;
 constexpr int F64_NRED = 1 + 5 + 15 + 15;  // nll, g, H (lower), F (lower)
 constexpr int F64_RED_BYTES = 4096;        // reduction areas at the start of shared memory
 constexpr size_t F64_G_SMEM = 56 * 1024;   // blur matrices up to this size are kept in shared memory
 
-// Work areas of a cluster in global memory (they stay in L2).  S holds (w, a) planes
-// of the FFT form and (a, w) planes of the direct form.
+// Work areas of a cluster in global memory (they stay in L2).
 struct F64Work {
-    double2* Q;  // D*D (direct form)
-    double2* S;  // 3 * D*W
-    double* I;   // 4 * W*W (direct form)
+    double2* S;  // 3 * (w, a) planes, W*D
     double* J;   // 4 * R*W
     double* T;   // 4 * R*R: the CTA's rows of map m start at T + m * nt
     int nt;      // pixels of the CTA's rows
 };
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-__host__ __device__ inline bool f64_fft(int N) { return N >= 64 && N <= 1024; }
 
-__host__ __device__ inline size_t f64_work_bytes(int N, int D, int W, int R) {
+__host__ __device__ inline size_t f64_work_bytes(int D, int W, int R) {
     size_t b = 0;
-    if (!f64_fft(N)) b += align_up((size_t)D * D * 16, 256) + align_up((size_t)4 * W * W * 8, 256);
     b += align_up((size_t)3 * D * W * 16, 256);
     b += align_up((size_t)4 * R * W * 8, 256);
     b += align_up((size_t)4 * R * R * 8, 256);
     return b;
 }
 
-__device__ inline F64Work f64_carve(char* base, int N, int D, int W, int R) {
+__device__ inline F64Work f64_carve(char* base, int D, int W, int R) {
     F64Work w{};
     size_t o = 0;
-    if (!f64_fft(N)) {
-        w.Q = (double2*)(base + o); o += align_up((size_t)D * D * 16, 256);
-        w.I = (double*)(base + o);  o += align_up((size_t)4 * W * W * 8, 256);
-    }
     w.S = (double2*)(base + o); o += align_up((size_t)3 * D * W * 16, 256);
     w.J = (double*)(base + o);  o += align_up((size_t)4 * R * W * 8, 256);
     w.T = (double*)(base + o);
     return w;
 }
 
-// Shared memory of the FFT form: reduction area, transform buffer, one tile of the
+// Shared memory: reduction areas, transform buffer, one tile of the
 // pupil field (LINES rows of D | 1) or of an intensity map (W x LINES), and the
 // transposed blur matrix (W x R) when it is small enough.
 __host__ __device__ inline size_t f64_tile_bytes(int N, int D, int W) {
@@ -82,85 +67,10 @@ __host__ __device__ inline size_t f64_tile_bytes(int N, int D, int W) {
     return align_up(q > x ? q : x, 256);
 }
 __host__ __device__ inline size_t f64_smem(int N, int D, int W, int R) {
-    if (!f64_fft(N)) return F64_RED_BYTES;
     const size_t g = (size_t)W * R * 8;
     return F64_RED_BYTES + FL_SMEM + f64_tile_bytes(N, D, W) + (g <= F64_G_SMEM ? g : 0);
 }
 
-// The CTAs of a cluster share one ROI or model: each takes its part of the pupil
-// rows, of the window columns and of the pixel rows, and they meet at cluster
-// barriers.  An evaluation then takes a fraction of the time, which is what one ROI,
-// a few of them, or the last slow fits of a batch wait for.
-struct Cluster {
-    unsigned rank, size;
-    __device__ Cluster() {
-        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-    }
-    __device__ void sync() const {
-        if (size == 1) __syncthreads();
-        else asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
-    }
-    // p (in this CTA's shared memory) as CTA r of the cluster has it
-    template <class T>
-    __device__ T read(const T* p, unsigned r) const { return *cooperative_groups::this_cluster().map_shared_rank((T*)p, r); }
-    __device__ unsigned id() const { return blockIdx.x / size; }
-    __device__ unsigned count() const { return gridDim.x / size; }
-    // this CTA's part of the row pairs of an R x R map
-    __device__ int row0(int R) const { return (int)(R / 2 * rank / size) * 2; }
-    __device__ int row1(int R) const { return (int)(R / 2 * (rank + 1) / size) * 2; }
-};
-// CTAs a cluster, by the window's columns (LINES at a time); never by the number of
-// ROIs, so that a result does not depend on its batch.
-__host__ __device__ inline int f64_cluster(int N, int W) {
-    if (!f64_fft(N)) return 1;
-    const int t = W / (2048 / N);
-    return t >= 4 ? 4 : (t >= 2 ? 2 : 1);
-}
-
-// Sum of NV doubles per thread over the cluster; every thread gets it.  red: 9 NV
-// doubles, part: NV doubles of shared memory not used by the previous call.
-template <int NV>
-__device__ inline void cluster_sum(const Cluster& cl, double (&v)[NV], double* red, double* part) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double x = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        v[k] = x;
-    }
-    __syncthreads();
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) red[warp * NV + k] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        double s = 0.0;
-        for (int w = 0; w < F64_WARPS; ++w) s += red[w * NV + threadIdx.x];
-        part[threadIdx.x] = s;
-    }
-    cl.sync();
-    if (threadIdx.x < NV) {
-        double s = part[threadIdx.x];
-        if (cl.size > 1) {
-            s = 0.0;
-            for (unsigned r = 0; r < cl.size; ++r) s += cl.read(part + threadIdx.x, r);
-        }
-        red[F64_WARPS * NV + threadIdx.x] = s;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = red[F64_WARPS * NV + k];
-}
-
-__device__ inline double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-__device__ inline double2 cmadd(double2 acc, double2 a, double2 b) {
-    acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
-    acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
-    return acc;
-}
 
 // Pupil field at (row a, column b): pupil (cos q, sin r).
 __device__ __forceinline__ double2 pupil_field(const PsfView& P, int a, int b, double x, double y, double zoil, double zwat) {
@@ -176,7 +86,8 @@ __device__ __forceinline__ double2 pupil_field(const PsfView& P, int a, int b, d
     return make_double2(pup * c, pup * s);
 }
 
-// The four blurred maps through N-point FFTs.  E[w] = sum_a C[w][a] Q[a] is, up to a
+// Computes the four blurred R x R maps T[0..3] = blurred I, I_x, I_y, I_z (only T[0]
+// when derivs is false) through N-point FFTs; all threads of the cluster take part.  E[w] = sum_a C[w][a] Q[a] is, up to a
 // sign (-1)^(w - W/2) that |E|^2 and conj(E) E_t do not see, output (w - W/2) mod N of
 // the inverse N-point transform of Q at points a0 .. a0 + D - 1.  Per LINES pupil rows
 // a: Q in shared memory, transforms of Q, i ky Q and i kz Q along b into S (w, a);
@@ -191,7 +102,7 @@ __device__ __forceinline__ double2 pupil_field(const PsfView& P, int a, int b, d
 // at 32 px (N = 128) 611 -> 124 us; 800 fits of 24 px 15.5 -> 3.8 ms, of which one CTA a
 // fit left 6.8; 26 fits of 42 px 8.4 -> 0.75 ms.
 template <class F>
-__device__ void eval_maps_fft(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w, char* smem,
+__device__ void eval_maps(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w, char* smem,
                               double x, double y, double zoil, double zwat, bool derivs) {
     constexpr int N = F::N, L = F::LINES;
     const int D = P.D, DP = D | 1, W = Wn.W, R = Wn.R, tid = threadIdx.x, a0 = P.a0;
@@ -253,25 +164,7 @@ __device__ void eval_maps_fft(const Cluster& cl, const PsfView& P, const WinView
             fl_transform<F, 1>(buf, P.tw, ld, st);
             __syncthreads();
             // J[m][i'][j] = sum_i G[i'][i] I[m][i][j]
-            double* J = w.J + (size_t)m * R * W;
-            for (int t = tid; t < (R / 2) * (L / 2); t += FL_THREADS) {
-                const int rp = t / (L / 2), c = t - rp * (L / 2);
-                const double* g = GT + 2 * rp;
-                const double* xi = X + 2 * c;
-                double s00 = 0, s01 = 0, s10 = 0, s11 = 0;
-#pragma unroll 4
-                for (int i = 0; i < W; ++i) {
-                    const double2 gv = *(const double2*)(g + (size_t)i * R), xv = *(const double2*)(xi + i * L);
-                    s00 = fma(gv.x, xv.x, s00);
-                    s01 = fma(gv.x, xv.y, s01);
-                    s10 = fma(gv.y, xv.x, s10);
-                    s11 = fma(gv.y, xv.y, s11);
-                }
-                if (c0 + 2 * c < W) {
-                    *(double2*)(J + (size_t)(2 * rp) * W + c0 + 2 * c) = make_double2(s00, s01);
-                    *(double2*)(J + (size_t)(2 * rp + 1) * W + c0 + 2 * c) = make_double2(s10, s11);
-                }
-            }
+            blur_tile(GT, X, R, W, L, min(L, W), w.J + (size_t)m * R * W + c0);
             __syncthreads();
         }
     }
@@ -308,164 +201,28 @@ __device__ void eval_maps_fft(const Cluster& cl, const PsfView& P, const WinView
     __syncthreads();
 }
 
-// Computes the four blurred R x R maps T[0..3] = blurred I, I_x, I_y, I_z
-// (only T[0] when derivs is false) by direct sums.
-__device__ void eval_maps_direct(const PsfView& P, const WinView& Wn, const F64Work& w, double x, double y,
-                              double zoil, double zwat, bool derivs) {
-    const int D = P.D, W = Wn.W, R = Wn.R, tid = threadIdx.x, nt = blockDim.x;
-    // 1. pupil field on the disk square
-    for (int idx = tid; idx < D * D; idx += nt) {
-        const int a = idx / D;
-        w.Q[idx] = pupil_field(P, a, idx - a * D, x, y, zoil, zwat);
-    }
-    __syncthreads();
-    // 2. first contraction over pupil columns b
-    double2* S = w.S;
-    double2* Sy = w.S + (size_t)D * W;
-    double2* Sz = w.S + (size_t)2 * D * W;
-    // a thread takes 4 rows a of one column j: each C value it loads serves 4 outputs
-    // (every output still sums its terms in the order b = 0, 1, ...)
-    constexpr int TA = 4;
-    const int DA = (D + TA - 1) / TA;
-    for (int idx = tid; idx < DA * W; idx += nt) {
-        const int a0 = (idx / W) * TA, j = idx - (idx / W) * W;
-        double2 s[TA], sy[TA], sz[TA];
-#pragma unroll
-        for (int t = 0; t < TA; ++t) { s[t] = make_double2(0, 0); sy[t] = make_double2(0, 0); sz[t] = make_double2(0, 0); }
-        const double2* crow = Wn.C + (size_t)j * D;
-        for (int b = 0; b < D; ++b) {
-            const double2 c = crow[b];
-            const double ky = P.ky[b];
-#pragma unroll
-            for (int t = 0; t < TA; ++t) {
-                if (a0 + t >= D) break;
-                const double2 q = w.Q[(size_t)(a0 + t) * D + b];
-                const double2 qc = cmul(q, c);
-                s[t].x += qc.x; s[t].y += qc.y;
-                if (derivs) {
-                    const double kz = P.kz[(a0 + t) * D + b];
-                    sy[t].x -= ky * qc.y; sy[t].y += ky * qc.x;   // (i ky) q c
-                    sz[t].x -= kz * qc.y; sz[t].y += kz * qc.x;   // (i kz) q c
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < TA; ++t) {
-            if (a0 + t >= D) break;
-            const size_t o = (size_t)(a0 + t) * W + j;
-            S[o] = s[t];
-            if (derivs) { Sy[o] = sy[t]; Sz[o] = sz[t]; }
-        }
-    }
-    __syncthreads();
-    // 3. second contraction over pupil rows a, then intensities
-    double* I0 = w.I;
-    double* I1 = w.I + (size_t)W * W;
-    double* I2 = w.I + (size_t)2 * W * W;
-    double* I3 = w.I + (size_t)3 * W * W;
-    // a thread takes 4 rows i of one column j: each S, S_y, S_z value it loads serves 4
-    // outputs (every output still sums its terms in the order a = 0, 1, ...)
-    constexpr int TI = 4;
-    for (int idx = tid; idx < (W / TI) * W; idx += nt) {
-        const int i0 = (idx / W) * TI, j = idx - (idx / W) * W;
-        double2 e[TI], ex[TI], ey[TI], ez[TI];
-#pragma unroll
-        for (int t = 0; t < TI; ++t) {
-            e[t] = make_double2(0, 0); ex[t] = make_double2(0, 0); ey[t] = make_double2(0, 0); ez[t] = make_double2(0, 0);
-        }
-        for (int a = 0; a < D; ++a) {
-            const double2 s = S[(size_t)a * W + j];
-            double2 sy, sz;
-            double kx = 0;
-            if (derivs) { sy = Sy[(size_t)a * W + j]; sz = Sz[(size_t)a * W + j]; kx = P.kx[a]; }
-#pragma unroll
-            for (int t = 0; t < TI; ++t) {
-                const double2 c = Wn.C[(size_t)(i0 + t) * D + a];
-                const double2 cs = cmul(c, s);
-                e[t].x += cs.x; e[t].y += cs.y;
-                if (derivs) {
-                    ex[t].x -= kx * cs.y; ex[t].y += kx * cs.x;
-                    ey[t] = cmadd(ey[t], c, sy);
-                    ez[t] = cmadd(ez[t], c, sz);
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < TI; ++t) {
-            const size_t o = (size_t)(i0 + t) * W + j;
-            I0[o] = e[t].x * e[t].x + e[t].y * e[t].y;
-            if (derivs) {
-                I1[o] = 2.0 * (e[t].x * ex[t].x + e[t].y * ex[t].y);
-                I2[o] = 2.0 * (e[t].x * ey[t].x + e[t].y * ey[t].y);
-                I3[o] = 2.0 * (e[t].x * ez[t].x + e[t].y * ez[t].y);
-            }
-        }
-    }
-    __syncthreads();
-    // 4. blur along the first index: J[m][i'][j] = sum_i G[i'][i] I[m][i][j]
-    const int nm = derivs ? 4 : 1;
-    // a thread takes 4 rows i' of one column j (each I value loaded serves 4 outputs)
-    constexpr int TR = 4;
-    const int RB = (R + TR - 1) / TR;
-    for (int idx = tid; idx < nm * RB * W; idx += nt) {
-        const int m = idx / (RB * W), rem = idx - m * RB * W, ip0 = (rem / W) * TR, j = rem - (rem / W) * W;
-        const double* Im = w.I + (size_t)m * W * W;
-        double acc[TR] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = 0; i < W; ++i) {
-            const double v = Im[(size_t)i * W + j];
-#pragma unroll
-            for (int t = 0; t < TR; ++t)
-                if (ip0 + t < R) acc[t] = fma(Wn.G[(size_t)(ip0 + t) * W + i], v, acc[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < TR; ++t)
-            if (ip0 + t < R) w.J[((size_t)m * R + ip0 + t) * W + j] = acc[t];
-    }
-    __syncthreads();
-    // 5. blur along the second index: T[m][i'][j'] = sum_j G[j'][j] J[m][i'][j]
-    for (int idx = tid; idx < nm * R * R; idx += nt) {
-        int m = idx / (R * R), rem = idx - m * R * R, ip = rem / R, jp = rem - ip * R;
-        const double* g = Wn.G + (size_t)jp * W;
-        const double* Jm = w.J + (size_t)m * R * W + (size_t)ip * W;
-        double acc = 0.0;
-        for (int j = 0; j < W; ++j) acc = fma(g[j], Jm[j], acc);
-        w.T[idx] = acc;
-    }
-    __syncthreads();
-}
-
-// All threads of the block participate.  NFFT: P.N where it takes the FFT form, else 0.
-template <int NFFT>
-__device__ __forceinline__ void eval_maps_f64(const Cluster& cl, const PsfView& P, const WinView& Wn, const F64Work& w,
-                                              char* smem, double x, double y, double zoil, double zwat, bool derivs) {
-    if constexpr (NFFT > 0) eval_maps_fft<FftLines<NFFT>>(cl, P, Wn, w, smem, x, y, zoil, zwat, derivs);
-    else eval_maps_direct(P, Wn, w, x, y, zoil, zwat, derivs);
-}
-
 // A CTA's set-up: the work areas of its cluster, T in the transform buffer (free
 // when the maps are used) where the CTA's rows fit, and the transposed blur matrix in
 // shared memory.
 template <int NFFT>
 __device__ __forceinline__ F64Work f64_begin(const Cluster& cl, const PsfView& P, const WinView& Wn, char* scratch,
                                              size_t per_cluster, char* smem) {
-    F64Work w = f64_carve(scratch + cl.id() * per_cluster, P.N, P.D, Wn.W, Wn.R);
+    F64Work w = f64_carve(scratch + cl.id() * per_cluster, P.D, Wn.W, Wn.R);
     const int i0 = cl.row0(Wn.R);
     w.nt = (cl.row1(Wn.R) - i0) * Wn.R;
-    if (NFFT > 0 && (size_t)4 * w.nt * 8 <= FL_SMEM) w.T = (double*)(smem + F64_RED_BYTES);
+    if ((size_t)4 * w.nt * 8 <= FL_SMEM) w.T = (double*)(smem + F64_RED_BYTES);
     else w.T += (size_t)4 * i0 * Wn.R;
-    if constexpr (NFFT > 0) {
-        const int n = Wn.W * Wn.R;
-        if ((size_t)n * 8 <= F64_G_SMEM) {
-            double* g = (double*)(smem + F64_RED_BYTES + FL_SMEM + f64_tile_bytes(NFFT, P.D, Wn.W));
-            for (int k = threadIdx.x; k < n; k += FL_THREADS) g[k] = Wn.GT[k];
-        }
+    const int n = Wn.W * Wn.R;
+    if ((size_t)n * 8 <= F64_G_SMEM) {
+        double* g = (double*)(smem + F64_RED_BYTES + FL_SMEM + f64_tile_bytes(NFFT, P.D, Wn.W));
+        for (int k = threadIdx.x; k < n; k += FL_THREADS) g[k] = Wn.GT[k];
     }
     __syncthreads();
     return w;
 }
 
 // Reduction areas: cluster_sum<36> and cluster_sum<4> have parts of their own.
-__device__ inline double* part_lik(double* red) { return red + (F64_WARPS + 1) * F64_NRED; }
+__device__ inline double* part_lik(double* red) { return red + (FL_WARPS + 1) * F64_NRED; }
 __device__ inline double* part_norm(double* red) { return part_lik(red) + F64_NRED; }
 
 // Normalisation sums: S = sum |T0|, Dt = sum sgn(T0) T_t.
@@ -504,7 +261,7 @@ __global__ void __launch_bounds__(F64_THREADS, 2) model_f64_kernel(PsfView P, Wi
     const int nn = n_dev ? min(n, *n_dev) : n;
     for (int mi = cl.id(); mi < nn; mi += cl.count()) {
         const int m = list ? list[mi] : mi;
-        eval_maps_f64<NFFT>(cl, P, Wn, w, smem_raw, xyz[3 * m], xyz[3 * m + 1], P.zfocus, xyz[3 * m + 2], derivs);
+        eval_maps<FftLines<NFFT>>(cl, P, Wn, w, smem_raw, xyz[3 * m], xyz[3 * m + 1], P.zfocus, xyz[3 * m + 2], derivs);
         double s[4];
         norm_sums(cl, w, derivs, red, s);
         for (int k = threadIdx.x; k < nt; k += blockDim.x) {
@@ -529,7 +286,7 @@ __device__ void eval_lik_f64(const Cluster& cl, const PsfView& P, const WinView&
                              const float* d, const float* sv, const double* th, double* red, double& nll, double* g,
                              double* H, double* F) {
     const int px0 = cl.row0(Wn.R) * Wn.R, nt = w.nt;
-    eval_maps_f64<NFFT>(cl, P, Wn, w, smem, th[0], th[1], P.zfocus, th[2], true);
+    eval_maps<FftLines<NFFT>>(cl, P, Wn, w, smem, th[0], th[1], P.zfocus, th[2], true);
     double s[4];
     norm_sums(cl, w, true, red, s);
     double v[F64_NRED];
@@ -630,19 +387,6 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fit_f64_kernel(PsfView P, WinV
     cl.sync();  // no CTA leaves while another may read its shared memory
 }
 
-// fn(integral constant): NFFT of a pupil grid.
-template <class FN>
-static void with_fft(int N, const FN& fn) {
-    switch (N) {
-        case 64: fn(std::integral_constant<int, 64>()); break;
-        case 128: fn(std::integral_constant<int, 128>()); break;
-        case 256: fn(std::integral_constant<int, 256>()); break;
-        case 512: fn(std::integral_constant<int, 512>()); break;
-        case 1024: fn(std::integral_constant<int, 1024>()); break;
-        default: fn(std::integral_constant<int, 0>());
-    }
-}
-
 // Launch configuration for n ROIs or models: as many clusters as run at once (at
 // most `most`).  attr and cfg live as long as the launch.
 template <class K>
@@ -671,7 +415,7 @@ static cudaError_t f64_config(K kernel, const zola_psf* p, const WindowTables* w
 int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n, double* d_out,
                      double* d_dout, cudaStream_t st, const int* d_list, const int* d_count) {
     if (n <= 0) return ZOLA_OK;
-    const size_t per_cluster = f64_work_bytes(p->N, p->D, w->W, w->R);
+    const size_t per_cluster = f64_work_bytes(p->D, w->W, w->R);
     WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
     int rc = ZOLA_OK;
     with_fft(p->N, [&](auto nfft) {
@@ -698,7 +442,7 @@ int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_r
                    const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
                    double* d_nll, int* d_status, int* d_iters, cudaStream_t st) {
     if (n <= 0) return ZOLA_OK;
-    const size_t per_cluster = f64_work_bytes(p->N, p->D, w->W, w->R);
+    const size_t per_cluster = f64_work_bytes(p->D, w->W, w->R);
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
     WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
     ZOLA_CUDA_CHECK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int), st), ctx);
@@ -837,7 +581,7 @@ extern "C" int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois,
     }
     char* base = (char*)noalloc_scratch(ctx->device, ctx->err);
     if (!base) return ZOLA_E_CUDA;
-    const size_t per_cluster = f64_work_bytes(psf->N, psf->D, w->W, w->R);
+    const size_t per_cluster = f64_work_bytes(psf->D, w->W, w->R);
     int* counter = (int*)base;
     char* work = base + 256;
     const size_t room = NOALLOC_SCRATCH_BYTES - 256;

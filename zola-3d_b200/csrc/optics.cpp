@@ -163,15 +163,19 @@ int build_psf_tables(zola_psf* p, const zola_optics* o, const double* zern, int 
 void blur_matrix(int R, int W, double sigma, std::vector<double>& G, std::vector<double>* dG) {
     std::vector<double> h(W), dh(W);
     const double s = W / (2 * M_PI * sigma);
+    std::vector<double> g(W), dg(W), cs(W);
+    for (int f = 0; f < W; ++f) {
+        const int fs = f < W / 2 ? f : f - W;
+        g[f] = std::exp(-0.5 * (double)fs * fs / (s * s));
+        dg[f] = -g[f] * (double)fs * fs / (s * s * sigma);
+        cs[f] = std::cos(2 * M_PI * (double)f / W);
+    }
     for (int d = 0; d < W; ++d) {
         double acc = 0.0, dacc = 0.0;
         for (int f = 0; f < W; ++f) {
-            int fs = f < W / 2 ? f : f - W;
-            double g = std::exp(-0.5 * (double)fs * fs / (s * s));
-            long long m = ((long long)f * d) % W;
-            const double cs = std::cos(2 * M_PI * (double)m / W);
-            acc += g * cs;
-            dacc += -g * (double)fs * fs / (s * s * sigma) * cs;
+            const double c = cs[(size_t)f * d % W];
+            acc += g[f] * c;
+            dacc += dg[f] * c;
         }
         h[d] = acc / W;
         dh[d] = dacc / W;

@@ -228,6 +228,8 @@ struct zola_psf {
     double* d_tables = nullptr;  // one allocation holding the arrays below
     zola::PsfView view{};
     std::map<int, zola::WindowTables> win;
+    double* d_calZ = nullptr;  // calibration: Zernike basis of cal_nz modes
+    int cal_nz = 0;
 };
 
 namespace zola {
