@@ -13,10 +13,13 @@
 // mean CRLB (:540-640).  The per-localization drift is the SplineFit of the
 // bin drifts at its frame (:660-700).
 //
-// GPU: histograms by atomic adds, batched 3-D C2C FFTs (the hand-written
-// radix-2 transform below, single precision like the reference's float
-// transforms), pair products, inverse FFTs and the centring crop in chunks of
-// pairs, and one CTA per pair for the peak centroid.  The circular shift the reference applies before the forward
+// GPU: histograms by atomic adds, 3-D C2C FFTs (radix-2 decimation in time, single
+// precision like the reference's float transforms), pair products, inverse FFTs and
+// the centring crop in chunks of pairs, and one CTA per pair for the peak centroid.
+// A plane of constant z fits in shared memory (k_drift_fwd_xy, k_drift_inv_xy), so its
+// x and y transforms and the pair product are one pass over memory, and the lines that
+// the padding leaves empty or the crop drops are not transformed; planes that do not fit
+// (P1 P2 > 24,000) go axis by axis (k_fft_lines).  The circular shift the reference applies before the forward
 // FFT multiplies every spectrum by the same sign pattern, which cancels in
 // F_t conj(F_s), so it is left out.  The least squares and the spline run on
 // the host.
@@ -37,32 +40,232 @@ struct DriftDev {
     double px;               // voxel size, nm
     double minX, minY, minZ;
     int minF, maxF;
-    double g0[3], g1[3];     // window bounds x, y, z (nm from the minima)
+};
+// Window bounds x, y, z (nm from the minima).
+struct DriftWin {
+    double g0[3], g1[3];
 };
 
-__global__ void k_drift_hist(DriftDev D, const double* xyz, const int* frame, int n, float2* cubes) {
+// Histogram counts of windows win[blockIdx.y] into [window][bin][S0][S1][S2], or, where
+// cubes is not null, into the centre of the padded cubes (one window).
+__global__ void k_drift_hist(DriftDev D, const DriftWin* win, const double* xyz, const int* frame, int n, float* hist,
+                             float2* cubes) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    const DriftWin w = win[blockIdx.y];
     const double x = xyz[3 * k] - D.minX, y = xyz[3 * k + 1] - D.minY, z = xyz[3 * k + 2] - D.minZ;
-    if (!(x >= D.g0[0] && x < D.g1[0] && y >= D.g0[1] && y < D.g1[1] && z >= D.g0[2] && z < D.g1[2])) return;
+    if (!(x >= w.g0[0] && x < w.g1[0] && y >= w.g0[1] && y < w.g1[1] && z >= w.g0[2] && z < w.g1[2])) return;
     const int b = D.bins * (frame[k] - D.minF) / (1 + D.maxF - D.minF);
-    const int xi = D.S2 / 2 + min(max((int)(fmod(x, D.S2 * D.px) / D.px), 0), D.S2 - 1);
-    const int yi = D.S1 / 2 + min(max((int)(fmod(y, D.S1 * D.px) / D.px), 0), D.S1 - 1);
-    const int zi = D.S0 / 2 + min(max((int)(fmod(z, D.S0 * D.px) / D.px), 0), D.S0 - 1);
-    const size_t PV = (size_t)D.P0 * D.P1 * D.P2;
-    atomicAdd(&cubes[(size_t)b * PV + ((size_t)zi * D.P1 + yi) * D.P2 + xi].x, 1.0f);
+    const int xi = min(max((int)(fmod(x, D.S2 * D.px) / D.px), 0), D.S2 - 1);
+    const int yi = min(max((int)(fmod(y, D.S1 * D.px) / D.px), 0), D.S1 - 1);
+    const int zi = min(max((int)(fmod(z, D.S0 * D.px) / D.px), 0), D.S0 - 1);
+    if (cubes) {
+        const size_t PV = (size_t)D.P0 * D.P1 * D.P2;
+        atomicAdd(&cubes[(size_t)b * PV + ((size_t)(D.S0 / 2 + zi) * D.P1 + D.S1 / 2 + yi) * D.P2 + D.S2 / 2 + xi].x, 1.0f);
+    } else {
+        atomicAdd(&hist[((((size_t)blockIdx.y * D.bins + b) * D.S0 + zi) * D.S1 + yi) * D.S2 + xi], 1.0f);
+    }
 }
 
-// Spectra times the float-rounded Fourier Gaussian (frequency index q -> q or q - P).
-__global__ void k_drift_gauss(DriftDev D, float2* spec, double sf0, double sf1, double sf2) {
+// The float-rounded Fourier Gaussian (frequency index q -> q or q - P), once a call.
+__global__ void k_drift_gauss(DriftDev D, double sf0, double sf1, double sf2, float* gauss) {
     const size_t PV = (size_t)D.P0 * D.P1 * D.P2;
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < PV * D.bins; k += (size_t)gridDim.x * blockDim.x) {
-        const size_t v = k % PV;
+    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < PV; v += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(v % D.P2), b = (int)((v / D.P2) % D.P1), a = (int)(v / ((size_t)D.P2 * D.P1));
         const double dz = a < D.P0 / 2 ? a : a - D.P0, dy = b < D.P1 / 2 ? b : b - D.P1, dx = c < D.P2 / 2 ? c : c - D.P2;
-        const float g = (float)exp(-.5 * (dx * dx / sf2 + dy * dy / sf1 + dz * dz / sf0));
+        gauss[v] = (float)exp(-.5 * (dx * dx / sf2 + dy * dy / sf1 + dz * dz / sf0));
+    }
+}
+
+__global__ void k_drift_mul(DriftDev D, float2* spec, const float* gauss) {
+    const size_t PV = (size_t)D.P0 * D.P1 * D.P2;
+    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < PV * D.bins; k += (size_t)gridDim.x * blockDim.x) {
+        const float g = gauss[k % PV];
         spec[k].x *= g;
         spec[k].y *= g;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Radix-2 decimation-in-time transforms of lines held in shared memory, with up to four
+// stages in registers between two visits (LG = log2 of the length, at most 8): the same
+// butterflies in the same order as k_fft_lines, so the same result bit for bit.  Lines
+// l < n; element k of line l is at(l, k).  Lanes run over the lines.  tw: k_fft_lines.
+constexpr int FFT_LMAX = 256, FFT_THREADS = 256;
+
+// w c as k_fft_lines rounds it (one product, one fused multiply-add a part), whatever
+// the compiler knows about the sign.
+__device__ __forceinline__ float2 cmul_f(float2 w, float2 c) {
+    return make_float2(__fmaf_rn(w.x, c.x, -__fmul_rn(w.y, c.y)), __fmaf_rn(w.y, c.x, __fmul_rn(w.x, c.y)));
+}
+
+template <int S0, int NS, class V>
+__device__ __forceinline__ void dit_stages(V (&x)[1 << NS], int lo, const float2* tw, float sign) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const int ts = (FFT_LMAX / 2) >> (S0 + s);
+#pragma unroll
+        for (int i = 0; i < (1 << NS); ++i) {
+            if (i >> s & 1) continue;
+            float2 w = __ldg(tw + (((i & ((1 << s) - 1)) << S0) + lo) * ts);
+            w.y *= -sign;
+            const float2 a = x[i], c = x[i | 1 << s], t = cmul_f(w, c);
+            x[i] = make_float2(a.x + t.x, a.y + t.y);
+            x[i | 1 << s] = make_float2(a.x - t.x, a.y - t.y);
+        }
+    }
+}
+
+template <int LG, class AT>
+__device__ __forceinline__ void dit_lines(float2* buf, int n, const AT& at, const float2* tw, float sign) {
+    constexpr int A = LG <= 4 ? LG : (LG + 1) / 2, B = LG - A;  // stages of the first and second visit
+    {
+        constexpr int G = 1 << (LG - A), LB = FFT_THREADS / G;
+        for (int l0 = 0; l0 < n; l0 += LB) {
+            const int l = l0 + (int)threadIdx.x % LB, g = threadIdx.x / LB;
+            float2 x[1 << A];
+            if (l < n) {
+#pragma unroll
+                for (int i = 0; i < (1 << A); ++i) x[i] = buf[at(l, (int)(__brev((unsigned)(g << A | i)) >> (32 - LG)))];
+                dit_stages<0, A>(x, 0, tw, sign);
+            }
+            __syncthreads();  // the line is in registers
+            if (l < n)
+#pragma unroll
+                for (int i = 0; i < (1 << A); ++i) buf[at(l, g << A | i)] = x[i];
+        }
+        __syncthreads();
+    }
+    if constexpr (B > 0) {
+        constexpr int G = 1 << A, LB = FFT_THREADS / G;
+        for (int l0 = 0; l0 < n; l0 += LB) {
+            const int l = l0 + (int)threadIdx.x % LB, lo = threadIdx.x / LB;
+            if (l >= n) continue;
+            float2 x[1 << B];
+#pragma unroll
+            for (int i = 0; i < (1 << B); ++i) x[i] = buf[at(l, i << A | lo)];
+            dit_stages<A, B>(x, lo, tw, sign);
+#pragma unroll
+            for (int i = 0; i < (1 << B); ++i) buf[at(l, i << A | lo)] = x[i];
+        }
+        __syncthreads();
+    }
+}
+
+template <class AT>
+__device__ void dit(float2* buf, int lg, int n, const AT& at, const float2* tw, float sign) {
+    switch (lg) {
+        case 1: dit_lines<1>(buf, n, at, tw, sign); break;
+        case 2: dit_lines<2>(buf, n, at, tw, sign); break;
+        case 3: dit_lines<3>(buf, n, at, tw, sign); break;
+        case 4: dit_lines<4>(buf, n, at, tw, sign); break;
+        case 5: dit_lines<5>(buf, n, at, tw, sign); break;
+        case 6: dit_lines<6>(buf, n, at, tw, sign); break;
+        case 7: dit_lines<7>(buf, n, at, tw, sign); break;
+        case 8: dit_lines<8>(buf, n, at, tw, sign); break;
+    }
+}
+
+__device__ inline int lg_of(int P) { return 31 - __clz(P); }
+// Window index c of an axis (size S, padded P = 2 S) in the centred correlation.
+__device__ inline int crop_of(int c, int S, int P) { return (c + S / 2 + P / 2) & (P - 1); }
+
+// Planes are kept as [y][x] with an odd row stride.
+constexpr int PLANE_MAX = 24000;  // elements of P1 x P2 that go through shared memory
+__host__ __device__ inline size_t plane_smem(int P1, int P2) { return (size_t)P1 * (P2 + 1) * sizeof(float2); }
+
+// x and y transforms of histogram plane blockIdx.x (z = S0 / 2 + blockIdx.x; the others
+// are empty) of bin blockIdx.y of the batch (windows x bins): xy[bin][plane][y][x].
+__global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_xy(DriftDev D, const float* hist, const float2* tw, float2* xy) {
+    extern __shared__ float2 plane[];
+    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1;
+    const size_t item = (size_t)blockIdx.y * D.S0 + blockIdx.x;
+    const float* h = hist + item * S1 * S2;
+    for (int e = threadIdx.x; e < P1 * P2; e += FFT_THREADS) {
+        const int y = e / P2, x = e - y * P2, yc = y - S1 / 2, xc = x - S2 / 2;
+        const bool in = yc >= 0 && yc < S1 && xc >= 0 && xc < S2;
+        plane[y * RS + x] = make_float2(in ? h[yc * S2 + xc] : 0.f, 0.f);
+    }
+    __syncthreads();
+    dit(plane, lg_of(P2), S1, [&](int l, int k) { return (S1 / 2 + l) * RS + k; }, tw, -1.f);
+    dit(plane, lg_of(P1), P2, [&](int l, int k) { return k * RS + l; }, tw, -1.f);
+    float2* out = xy + item * P1 * P2;
+    for (int e = threadIdx.x; e < P1 * P2; e += FFT_THREADS) out[e] = plane[e / P2 * RS + e % P2];
+}
+
+// z transforms, 32 lines a CTA, times the Gaussian: spec[bin][z][y][x].
+constexpr int ZL = 32;
+__global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_z(DriftDev D, const float2* xy, const float2* tw,
+                                                             const float* gauss, float2* spec) {
+    extern __shared__ float2 lines[];
+    const int P0 = D.P0, S0 = D.S0, PP = D.P1 * D.P2, q0 = blockIdx.x * ZL, nl = min(ZL, PP - q0);
+    const float2* in = xy + (size_t)blockIdx.y * S0 * PP;
+    float2* out = spec + (size_t)blockIdx.y * P0 * PP;
+    for (int e = threadIdx.x; e < P0 * ZL; e += FFT_THREADS) {
+        const int z = e / ZL, l = e % ZL, zc = z - S0 / 2;
+        lines[e] = zc >= 0 && zc < S0 && l < nl ? in[(size_t)zc * PP + q0 + l] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    dit(lines, lg_of(P0), ZL, [&](int l, int k) { return k * ZL + l; }, tw, -1.f);
+    for (int e = threadIdx.x; e < P0 * ZL; e += FFT_THREADS) {
+        const int z = e / ZL, l = e % ZL;
+        if (l >= nl) continue;
+        const size_t o = (size_t)z * PP + q0 + l;
+        float2 v = lines[e];
+        const float g = gauss[o];
+        v.x *= g;
+        v.y *= g;
+        out[o] = v;
+    }
+}
+
+// Plane z = blockIdx.x of F_p1 conj(F_p2) for pair first + blockIdx.y of window blockIdx.z
+// of the batch, its inverse x transforms, its inverse y transforms for the x that the crop
+// keeps, and the cropped plane: xy[window][pair][z][S1][S2].  66 pairs of 64^3 take 77 us
+// and their z pass 33, bound by L2 (64 KB of spectra a plane) and shared memory; product,
+// three axes and crop as five passes over whole cubes took 760.
+__global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_xy(DriftDev D, const float2* spec, const int* p1, const int* p2,
+                                                              int first, const float2* tw, float2* xy) {
+    extern __shared__ float2 plane[];
+    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1, PP = P1 * P2;
+    const size_t PV = (size_t)D.P0 * PP;
+    spec += (size_t)blockIdx.z * D.bins * PV + (size_t)blockIdx.x * PP;
+    const float2* f1 = spec + p1[first + blockIdx.y] * PV;
+    const float2* f2 = spec + p2[first + blockIdx.y] * PV;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < PP; e += FFT_THREADS) {
+        const float2 a = f1[e], b = f2[e];
+        plane[e / P2 * RS + e % P2] = make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)),
+                                                  __fmaf_rn(a.y, b.x, -__fmul_rn(a.x, b.y)));
+    }
+    __syncthreads();
+    dit(plane, lg_of(P2), P1, [&](int l, int k) { return l * RS + k; }, tw, 1.f);
+    dit(plane, lg_of(P1), S2, [&](int l, int k) { return k * RS + crop_of(l, S2, P2); }, tw, 1.f);
+    float2* out = xy + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * D.P0 + blockIdx.x) * S1 * S2;
+    for (int e = threadIdx.x; e < S1 * S2; e += FFT_THREADS) {
+        const int b = e / S2, c = e - b * S2;
+        out[e] = plane[crop_of(b, S1, P1) * RS + crop_of(c, S2, P2)];
+    }
+}
+
+// Inverse z transforms of the cropped planes, 32 lines a CTA; result[pair] += the real
+// part at the z that the crop keeps, window after window of the batch.
+__global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_z(DriftDev D, const float2* xy, int first, int nwin,
+                                                             const float2* tw, float* result) {
+    extern __shared__ float2 lines[];
+    const int P0 = D.P0, S0 = D.S0, SS = D.S1 * D.S2, q0 = blockIdx.x * ZL, nl = min(ZL, SS - q0);
+    float* res = result + (size_t)(first + blockIdx.y) * S0 * SS;
+    for (int w = 0; w < nwin; ++w) {
+        const float2* in = xy + ((size_t)w * gridDim.y + blockIdx.y) * P0 * SS;
+        for (int e = threadIdx.x; e < P0 * ZL; e += FFT_THREADS)
+            lines[e] = e % ZL < nl ? in[(size_t)(e / ZL) * SS + q0 + e % ZL] : make_float2(0.f, 0.f);
+        __syncthreads();
+        dit(lines, lg_of(P0), ZL, [&](int l, int k) { return k * ZL + l; }, tw, 1.f);
+        for (int e = threadIdx.x; e < S0 * ZL; e += FFT_THREADS) {
+            const int a = e / ZL, l = e % ZL;
+            if (l < nl) res[(size_t)a * SS + q0 + l] += lines[crop_of(a, S0, P0) * ZL + l].x;
+        }
+        __syncthreads();
     }
 }
 
@@ -75,8 +278,6 @@ __global__ void k_drift_gauss(DriftDev D, float2* spec, double sf0, double sf1, 
 // (inner > 1), whichever is contiguous in memory.  Unnormalised; sign -1 is
 // exp(-2 pi i j k / L) (forward), +1 the inverse.  tw[m] = exp(-2 pi i m / 256),
 // m < 128, rounded from double; length L uses every (256 / L)-th entry.
-constexpr int FFT_LMAX = 256, FFT_THREADS = 256;
-
 __global__ void __launch_bounds__(FFT_THREADS) k_fft_lines(float2* data, int L, int lg, long long inner,
                                                            long long lines, int TL, const float2* tw, float sign) {
     extern __shared__ float2 sbuf[];
@@ -184,15 +385,19 @@ __global__ void __launch_bounds__(LM_THREADS) k_drift_peak(DriftDev D, const flo
     bv[threadIdx.x] = best;
     bi[threadIdx.x] = bidx;
     __syncthreads();
-    if (threadIdx.x == 0) {  // strict > in scan order = the first index among equal maxima
-        float m = 0.0f;
-        long long idx = -1;
-        for (int t = 0; t < LM_THREADS; ++t) {
-            if (bi[t] < 0) continue;
-            if (idx < 0 || bv[t] > m || (bv[t] == m && bi[t] < idx)) { m = bv[t]; idx = bi[t]; }
+    // strict > in scan order = the first index among equal maxima
+    for (int o = LM_THREADS / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            const float v = bv[threadIdx.x + o];
+            const long long k = bi[threadIdx.x + o], mine = bi[threadIdx.x];
+            if (k >= 0 && (mine < 0 || v > bv[threadIdx.x] || (v == bv[threadIdx.x] && k < mine))) {
+                bv[threadIdx.x] = v;
+                bi[threadIdx.x] = k;
+            }
         }
-        bi[0] = idx < 0 ? 0 : idx;
+        __syncthreads();
     }
+    if (threadIdx.x == 0 && bi[0] < 0) bi[0] = 0;
     __syncthreads();
     const long long mi = bi[0];
     const int a0 = (int)(mi / ((long long)W1 * W2)), b0 = (int)((mi / W2) % W1), c0 = (int)(mi % W2);
@@ -203,18 +408,14 @@ __global__ void __launch_bounds__(LM_THREADS) k_drift_peak(DriftDev D, const flo
     // a one-voxel axis (flat data; the reference throws there) keeps its single voxel
     s0 = max(s0, 1); s1 = max(s1, 1); s2 = max(s2, 1);
     const int np = s0 * s1 * s2;
-    // gather in scan order (inside-the-volume entries), pad with +inf for the sort
-    __shared__ int number;
-    if (threadIdx.x == 0) {
-        int cnt = 0;
-        for (int q = 0; q < np; ++q) {
-            const int i = q / (s1 * s2), ii = (q / s2) % s1, iii = q % s2;
-            const int A = i + a0 - s0 / 2, B = ii + b0 - s1 / 2, C = iii + c0 - s2 / 2;
-            if (A >= 0 && B >= 0 && C >= 0 && A < W0 && B < W1 && C < W2) vals[cnt++] = im[((size_t)A * W1 + B) * W2 + C];
-        }
-        number = cnt;
+    // the entries inside the volume are a box: their values, padded with +inf for the sort
+    const int A0 = max(a0 - s0 / 2, 0), A1 = min(a0 - s0 / 2 + s0, W0), B0 = max(b0 - s1 / 2, 0),
+              B1 = min(b0 - s1 / 2 + s1, W1), C0 = max(c0 - s2 / 2, 0), C1 = min(c0 - s2 / 2 + s2, W2);
+    const int number = (A1 - A0) * (B1 - B0) * (C1 - C0);
+    for (int q = threadIdx.x; q < number; q += LM_THREADS) {
+        const int c = q % (C1 - C0), r = q / (C1 - C0), b = r % (B1 - B0), a = r / (B1 - B0);
+        vals[q] = im[((size_t)(A0 + a) * W1 + B0 + b) * W2 + C0 + c];
     }
-    __syncthreads();
     for (int q = number + threadIdx.x; q < 2048; q += LM_THREADS) vals[q] = INFINITY;
     __syncthreads();
     for (int k = 2; k <= 2048; k <<= 1)  // bitonic sort, ascending
@@ -404,71 +605,114 @@ extern "C" int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crl
     for (int t = 0; t < bin - 1; ++t)
         for (int s = t + 1; s < bin; ++s) { p1.push_back(t); p2.push_back(s); }
     const int tot = (int)p1.size();
-    // device buffers
-    const size_t chunk_budget = (size_t)4 << 30;
-    const int CH = tot > 0 ? (int)std::max<size_t>(1, std::min<size_t>(tot, chunk_budget / (PV * sizeof(float2)))) : 1;
-    DevBuf<double> d_xyz, d_drift;
-    DevBuf<int> d_frame, d_p1, d_p2;
-    DevBuf<float2> d_spec, d_corr;
-    DevBuf<float> d_res;
-    ZOLA_CUDA_CHECK(d_xyz.alloc((size_t)3 * n), ctx);
-    ZOLA_CUDA_CHECK(d_frame.alloc((size_t)n), ctx);
-    ZOLA_CUDA_CHECK(d_spec.alloc(PV * bin), ctx);
-    if (tot > 0) {
-        ZOLA_CUDA_CHECK(d_p1.alloc((size_t)tot), ctx);
-        ZOLA_CUDA_CHECK(d_p2.alloc((size_t)tot), ctx);
-        ZOLA_CUDA_CHECK(d_corr.alloc(PV * CH), ctx);
-        ZOLA_CUDA_CHECK(d_res.alloc(RV * tot), ctx);
-        ZOLA_CUDA_CHECK(d_drift.alloc((size_t)3 * tot), ctx);
-    }
-    cudaStream_t st = ctx->stream;
-    ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_xyz.p, xyz_nm, (size_t)24 * n, cudaMemcpyHostToDevice, st), ctx);
-    ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_frame.p, frame, (size_t)4 * n, cudaMemcpyHostToDevice, st), ctx);
-    if (tot > 0) {
-        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_p1.p, p1.data(), (size_t)4 * tot, cudaMemcpyHostToDevice, st), ctx);
-        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_p2.p, p2.data(), (size_t)4 * tot, cudaMemcpyHostToDevice, st), ctx);
-        ZOLA_CUDA_CHECK(cudaMemsetAsync(d_res.p, 0, RV * tot * sizeof(float), st), ctx);
-    }
-    // twiddles exp(-2 pi i m / 256), m < 128, for every transform length
-    DevBuf<float2> d_tw;
-    {
-        std::vector<float2> tw(FFT_LMAX / 2);
-        for (int m = 0; m < FFT_LMAX / 2; ++m)
-            tw[m] = make_float2((float)std::cos(2 * M_PI * m / FFT_LMAX), (float)-std::sin(2 * M_PI * m / FFT_LMAX));
-        ZOLA_CUDA_CHECK(d_tw.alloc(tw.size()), ctx);
-        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st),
-                        ctx);
-        ZOLA_CUDA_CHECK(cudaStreamSynchronize(st), ctx);  // tw is a host temporary
-    }
-    const int grid = ctx->num_sms * 8;
+    // device buffers, carved from the context's scratch: localizations, pairs, twiddles, the
+    // Gaussian, spectra, what the pairs of a chunk need at once, the summed correlations
+    const bool planes = (size_t)D.P1 * D.P2 <= PLANE_MAX;
+    const size_t per_pair = planes ? (size_t)D.P0 * D.S1 * D.S2 : PV;
+    // (planes: about half of the 126 MB L2, so that the z pass reads its input from there)
+    const size_t chunk_budget = planes ? (size_t)56 << 20 : (size_t)4 << 30;
+    const int CH = tot > 0 ? (int)std::min<size_t>(std::max<size_t>(1, std::min<size_t>(tot, chunk_budget / (per_pair * sizeof(float2)))), 65535) : 1;
+    // Small windows go through the kernels in batches (their launches would bound the call).
+    std::vector<DriftWin> wins;
     for (int u = 0; u < nbw[0]; ++u)
         for (int uu = 0; uu < nbw[1]; ++uu)
             for (int uuu = 0; uuu < nbw[2]; ++uuu) {
                 const int uv[3] = {u, uu, uuu};
+                DriftWin w;
                 for (int d = 0; d < 3; ++d) {
-                    D.g0[d] = (uv[d] / 2) * sF[d] * pixel + (uv[d] % 2) * (sF[d] / 2) * pixel;
-                    D.g1[d] = (uv[d] / 2 + 1) * sF[d] * pixel + (uv[d] % 2) * (sF[d] / 2) * pixel;
+                    w.g0[d] = (uv[d] / 2) * sF[d] * pixel + (uv[d] % 2) * (sF[d] / 2) * pixel;
+                    w.g1[d] = (uv[d] / 2 + 1) * sF[d] * pixel + (uv[d] % 2) * (sF[d] / 2) * pixel;
                 }
-                ZOLA_CUDA_CHECK(cudaMemsetAsync(d_spec.p, 0, PV * bin * sizeof(float2), st), ctx);
-                k_drift_hist<<<(n + 255) / 256, 256, 0, st>>>(D, d_xyz.p, d_frame.p, n, d_spec.p);
-                fft3d(ctx, d_spec.p, bin, D.P0, D.P1, D.P2, -1.f, d_tw.p, st);
-                k_drift_gauss<<<grid, 256, 0, st>>>(D, d_spec.p, sfp[2], sfp[1], sfp[0]);
-                ctx->launches += 2;
-                for (int first = 0; first < tot; first += CH) {
-                    const int np = std::min(CH, tot - first);
-                    k_drift_pairs<<<grid, 256, 0, st>>>(D, d_spec.p, d_p1.p, d_p2.p, first, np, d_corr.p);
-                    fft3d(ctx, d_corr.p, np, D.P0, D.P1, D.P2, 1.f, d_tw.p, st);
-                    k_drift_crop<<<grid, 256, 0, st>>>(D, d_corr.p, first, np, d_res.p);
-                    ctx->launches += 2;
-                }
-                ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
+                wins.push_back(w);
             }
+    const int nwin = (int)wins.size();
+    const size_t per_win = (per_pair * tot + PV * bin) * sizeof(float2);
+    const int WB = planes && CH == std::max(tot, 1)
+                       ? (int)std::min<size_t>(std::max<size_t>(chunk_budget / per_win, 1),
+                                                 std::min({nwin, 256, std::max(1, 65535 / bin)})) : 1;
+    size_t need = 0;
+    auto want = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) / 256 * 256; return o; };
+    const size_t o_xyz = want((size_t)24 * n), o_frame = want((size_t)4 * n), o_p1 = want((size_t)4 * tot),
+                 o_p2 = want((size_t)4 * tot), o_tw = want(FFT_LMAX / 2 * sizeof(float2)), o_gauss = want(PV * 4),
+                 o_drift = want((size_t)24 * tot), o_win = want(nwin * sizeof(DriftWin)), o_hist = want(RV * bin * 4 * WB),
+                 o_fxy = want(planes ? (size_t)D.S0 * D.P1 * D.P2 * bin * WB * sizeof(float2) : 0),
+                 o_spec = want(PV * bin * WB * sizeof(float2)), o_corr = want(tot > 0 ? per_pair * CH * WB * sizeof(float2) : 0),
+                 o_res = want(RV * tot * sizeof(float));
+    if (ensure_scratch(ctx, need, ctx->err)) return ZOLA_E_CUDA;
+    char* base = (char*)ctx->scratch;
+    double *d_xyz = (double*)(base + o_xyz), *d_drift = (double*)(base + o_drift);
+    int *d_frame = (int*)(base + o_frame), *d_p1 = (int*)(base + o_p1), *d_p2 = (int*)(base + o_p2);
+    float2 *d_tw = (float2*)(base + o_tw), *d_fxy = (float2*)(base + o_fxy), *d_spec = (float2*)(base + o_spec),
+           *d_corr = (float2*)(base + o_corr);
+    DriftWin* d_win = (DriftWin*)(base + o_win);
+    float *d_gauss = (float*)(base + o_gauss), *d_hist = (float*)(base + o_hist), *d_res = (float*)(base + o_res);
+    cudaStream_t st = ctx->stream;
+    ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_xyz, xyz_nm, (size_t)24 * n, cudaMemcpyHostToDevice, st), ctx);
+    ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_win, wins.data(), nwin * sizeof(DriftWin), cudaMemcpyHostToDevice, st), ctx);
+    ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_frame, frame, (size_t)4 * n, cudaMemcpyHostToDevice, st), ctx);
+    if (tot > 0) {
+        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_p1, p1.data(), (size_t)4 * tot, cudaMemcpyHostToDevice, st), ctx);
+        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_p2, p2.data(), (size_t)4 * tot, cudaMemcpyHostToDevice, st), ctx);
+        ZOLA_CUDA_CHECK(cudaMemsetAsync(d_res, 0, RV * tot * sizeof(float), st), ctx);
+    }
+    // twiddles exp(-2 pi i m / 256), m < 128, for every transform length
+    {
+        std::vector<float2> tw(FFT_LMAX / 2);
+        for (int m = 0; m < FFT_LMAX / 2; ++m)
+            tw[m] = make_float2((float)std::cos(2 * M_PI * m / FFT_LMAX), (float)-std::sin(2 * M_PI * m / FFT_LMAX));
+        ZOLA_CUDA_CHECK(cudaMemcpyAsync(d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st),
+                        ctx);
+        ZOLA_CUDA_CHECK(cudaStreamSynchronize(st), ctx);  // tw is a host temporary
+    }
+    const int grid = ctx->num_sms * 8;
+    k_drift_gauss<<<grid, 256, 0, st>>>(D, sfp[2], sfp[1], sfp[0], d_gauss);
+    ctx->launches++;
+    const size_t psm = plane_smem(D.P1, D.P2), zsm = (size_t)D.P0 * ZL * sizeof(float2);
+    if (planes) {
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_fwd_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm), ctx);
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_inv_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm), ctx);
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_fwd_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_inv_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
+    }
+    for (int w0 = 0; w0 < nwin; w0 += WB) {
+        const int nw = std::min(WB, nwin - w0);
+        const dim3 hgrid((n + 255) / 256, nw);
+        if (planes) {
+            ZOLA_CUDA_CHECK(cudaMemsetAsync(d_hist, 0, RV * bin * 4 * nw, st), ctx);
+            k_drift_hist<<<hgrid, 256, 0, st>>>(D, d_win + w0, d_xyz, d_frame, n, d_hist, nullptr);
+            k_drift_fwd_xy<<<dim3(D.S0, bin * nw), FFT_THREADS, psm, st>>>(D, d_hist, d_tw, d_fxy);
+            k_drift_fwd_z<<<dim3((D.P1 * D.P2 + ZL - 1) / ZL, bin * nw), FFT_THREADS, zsm, st>>>(D, d_fxy, d_tw, d_gauss,
+                                                                                               d_spec);
+            ctx->launches += 3;
+            for (int first = 0; first < tot; first += CH) {
+                const int np = std::min(CH, tot - first);
+                k_drift_inv_xy<<<dim3(D.P0, np, nw), FFT_THREADS, psm, st>>>(D, d_spec, d_p1, d_p2, first, d_tw, d_corr);
+                k_drift_inv_z<<<dim3((D.S1 * D.S2 + ZL - 1) / ZL, np), FFT_THREADS, zsm, st>>>(D, d_corr, first, nw, d_tw,
+                                                                                             d_res);
+                ctx->launches += 2;
+            }
+        } else {
+            ZOLA_CUDA_CHECK(cudaMemsetAsync(d_spec, 0, PV * bin * sizeof(float2), st), ctx);
+            k_drift_hist<<<hgrid, 256, 0, st>>>(D, d_win + w0, d_xyz, d_frame, n, nullptr, d_spec);
+            fft3d(ctx, d_spec, bin, D.P0, D.P1, D.P2, -1.f, d_tw, st);
+            k_drift_mul<<<grid, 256, 0, st>>>(D, d_spec, d_gauss);
+            ctx->launches += 2;
+            for (int first = 0; first < tot; first += CH) {
+                const int np = std::min(CH, tot - first);
+                k_drift_pairs<<<grid, 256, 0, st>>>(D, d_spec, d_p1, d_p2, first, np, d_corr);
+                fft3d(ctx, d_corr, np, D.P0, D.P1, D.P2, 1.f, d_tw, st);
+                k_drift_crop<<<grid, 256, 0, st>>>(D, d_corr, first, np, d_res);
+                ctx->launches += 2;
+            }
+        }
+        ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
+    }
     std::vector<double> pd((size_t)3 * tot);
     if (tot > 0) {
-        k_drift_peak<<<tot, LM_THREADS, 0, st>>>(D, d_res.p, d_drift.p);
+        k_drift_peak<<<tot, LM_THREADS, 0, st>>>(D, d_res, d_drift);
         ctx->launches++;
         ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
-        ZOLA_CUDA_CHECK(cudaMemcpyAsync(pd.data(), d_drift.p, pd.size() * 8, cudaMemcpyDeviceToHost, st), ctx);
+        ZOLA_CUDA_CHECK(cudaMemcpyAsync(pd.data(), d_drift, pd.size() * 8, cudaMemcpyDeviceToHost, st), ctx);
     }
     ZOLA_CUDA_CHECK(cudaStreamSynchronize(st), ctx);
     // bin drifts: pairs with bin 0, then least squares over all pairs (:480-640)
