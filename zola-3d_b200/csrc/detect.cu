@@ -853,10 +853,8 @@ int zola_detector_create(zola_psf* psf, int SX, int SY, int R, double minZ, doub
     double z = minZ;
     for (int i = 0; i < number; ++i) { d->range.push_back(z); z += step; }
     // library PSFs with the FP64 model: x = y = 0, zoil = Zfocus, zwat = range[i]
-    std::vector<double> xyz(3 * (size_t)number);
-    for (int i = 0; i < number; ++i) { xyz[3 * i] = 0; xyz[3 * i + 1] = 0; xyz[3 * i + 2] = d->range[i]; }
     d->h_psf.resize((size_t)number * R * R);
-    int rc = zola_psf_model(psf, R, xyz.data(), number, d->h_psf.data(), nullptr);
+    int rc = library_psfs(psf, R, d->range.data(), number, d->h_psf.data());
     if (rc) { delete d; return rc; }
     std::vector<double> psf0((size_t)number * R * R), varpsf(number), norm((size_t)SX * SY);
     for (int i = 0; i < number; ++i) {  // Predetection.java:178-204

@@ -84,11 +84,10 @@ __device__ inline double warp_max(double v) {
     return v;
 }
 
-// getAandB with the library PSF of slice r, threshold 10% of its max, on the
-// patch minus the sCMOS term when there is one (:1119-1211), by one warp; returns
-// whether the candidate is fitted (maxPatch / B > maxSNR and B > 0).
-__device__ bool pipe_a_and_b(const PipeView& V, const double* img, int r, int ci, int cj, double* A_, double* B_,
-                             double* maxp_) {
+// Whether a candidate is fitted (maxPatch / B > maxSNR and B > 0), by one warp, with B
+// of getAandB: the mean of the pixels whose library PSF of slice r is under 10% of its
+// maximum, of the patch minus the sCMOS term when there is one (:1119-1211).
+__device__ bool pipe_fitted(const PipeView& V, const double* img, int r, int ci, int cj, double* maxp_) {
     const double* vm = V.vmap;
     const int R = V.R, RR = R * R, SY = V.SY, lane = threadIdx.x & 31;
     const size_t corner = (size_t)(ci - R / 2) * SY + (cj - R / 2);
@@ -103,32 +102,26 @@ __device__ bool pipe_a_and_b(const PipeView& V, const double* img, int r, int ci
     maxi = warp_max(maxi);
     maxp = warp_max(maxp);
     const double thr = maxi * 0.1;
-    double B = 0, A = 0;
+    double B = 0;
     int cb = 0;
 #pragma unroll 4
     for (int k = lane; k < RR; k += 32) {
         const size_t px = corner + (size_t)(k / R) * SY + k % R;
-        const double v = img[px] - (vm ? vm[px] : 0.0);
         const bool low = psf[k] < thr;
-        B += low ? v : 0.0;
-        A += low ? 0.0 : v;
+        B += low ? img[px] - (vm ? vm[px] : 0.0) : 0.0;
         cb += low;
     }
     B = warp_sum(B);
-    A = warp_sum(A);
     cb = __reduce_add_sync(0xffffffffu, cb);
     B = cb != 0 ? B / cb : 0.0;
-    A -= (double)(RR - cb) * B;
-    *A_ = A;
-    *B_ = B;
     *maxp_ = maxp;
     return maxp / B > V.max_snr && B > 0;
 }
 
 // One wave's selection for one frame (one CTA): walking the candidates from the
 // frame's pointer, the first K (in candidate order) that need a fit under the
-// current mask get slots, their ROI and the A, B of their start (k_pipe_start adds
-// the position).  limit = just past the K-th (or the end).
+// current mask get slots and their ROI (k_pipe_start adds the start).  limit = just
+// past the K-th (or the end).
 // 512 candidates at a time: a thread drops the ones outside the border or with a
 // masked centre, which late in a frame are nearly all; the rest are taken in order,
 // a warp each, until K are found.  (A thread a candidate for everything read its
@@ -170,7 +163,7 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
             const double* row = cand + (size_t)k * 7;
             const int r = (int)llrint(row[1]), ci = (int)llrint(row[2]), cj = (int)llrint(row[3]);
             const size_t corner = (size_t)(ci - h) * SY + (cj - h);
-            double A = 0, B = 0, maxp = 0;
+            double maxp = 0;
             int code = -3;
             if (mine) {
                 bool masked = false;
@@ -183,7 +176,7 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
                     }
                     masked = __any_sync(0xffffffffu, any);
                 }
-                if (!masked) code = pipe_a_and_b(V, img, r, ci, cj, &A, &B, &maxp) ? 0 : -1;
+                if (!masked) code = pipe_fitted(V, img, r, ci, cj, &maxp) ? 0 : -1;
                 if (lane == 0) {
                     code_of[k] = code;
                     V.cand_maxp[(size_t)f * V.cap + k] = maxp;
@@ -213,8 +206,6 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
                         if (sv) sv[q] = (float)V.vmap[px];
                     }
                     if (lane == 0) {
-                        V.init[(size_t)s * 5 + 3] = A;
-                        V.init[(size_t)s * 5 + 4] = B;
                         V.slot_frame[s] = f;
                         V.slot_cand[s] = k;
                     }
@@ -229,16 +220,57 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
     if (threadIdx.x == 0) V.limit[f] = limit;
 }
 
-// Start positions of the wave's slots, from their candidates' refined offsets:
-// loc.init(A, B, -dx, -dy, range[r] + dz).
-__global__ void k_pipe_start(PipeView V, int n) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// Starts of the wave's slots: the candidates' refined offsets, loc.init(A, B, -dx, -dy,
+// range[r] + dz), and getAandB's A and B (pipe_fitted's B).  A warp a slot; the even lanes
+// add up B and the odd ones A, pixel after pixel: a split fit's path depends on the last
+// bit of its start, so the sums keep the order of getAandB's loop.  (40 px: 1,600 adds,
+// one after the other, about 30 us for a wave of 768 slots.)
+__global__ void __launch_bounds__(128) k_pipe_start(PipeView V, int n) {
+    const int s = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= n) return;
     const double* row = V.cand + ((size_t)V.slot_frame[s] * V.cap + V.slot_cand[s]) * 7;
+    const double* vm = V.vmap;
+    const int R = V.R, RR = R * R, SY = V.SY;
+    const int r = (int)llrint(row[1]), ci = (int)llrint(row[2]), cj = (int)llrint(row[3]);
+    const double* img = V.fimg + (size_t)V.slot_frame[s] * V.SX * SY;
+    const size_t corner = (size_t)(ci - R / 2) * SY + (cj - R / 2);
+    const double* psf = V.libpsf + (size_t)r * RR;
+    double maxi = -INFINITY;
+#pragma unroll 4
+    for (int k = lane; k < RR; k += 32) maxi = fmax(maxi, psf[k]);
+    const double thr = warp_max(maxi) * 0.1;
+    auto pixel = [&](int k, bool& low) {
+        if (k >= RR) return 0.0;
+        const size_t px = corner + (size_t)(k / R) * SY + k % R;
+        low = psf[k] < thr;
+        return img[px] - (vm ? vm[px] : 0.0);
+    };
+    bool low = false;
+    double v = pixel(lane, low), sum = 0;
+    int cb = 0;
+    for (int k0 = 0; k0 < RR; k0 += 32) {
+        const unsigned lows = __ballot_sync(0xffffffffu, low);
+        const double cur = v;
+        low = false;
+        v = pixel(k0 + 32 + lane, low);  // on its way while this one is added up
+        const unsigned mine = (lane & 1) ? ~lows : lows;
+        cb += __popc(lows);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            const double x = __shfl_sync(0xffffffffu, cur, q);
+            sum += (mine >> q & 1u) ? x : 0.0;
+        }
+    }
+    double B = __shfl_sync(0xffffffffu, sum, 0), A = __shfl_sync(0xffffffffu, sum, 1);
+    if (lane != 0) return;
+    B = cb != 0 ? B / cb : 0.0;
+    A -= (double)(RR - cb) * B;
     double* in = V.init + (size_t)s * 5;
     in[0] = -row[5];
     in[1] = -row[6];
-    in[2] = V.range[(int)llrint(row[1])] + row[4];
+    in[2] = V.range[r] + row[4];
+    in[3] = A;
+    in[4] = B;
 }
 
 // The fitted slots that can be accepted whatever the mask: every test of the
@@ -638,7 +670,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 rc = detect_refine(det, (double*)b_img.p, (double*)b_var.p, (double*)b_cand.p, cap, nslot,
                                    (int*)b_sf.p, (int*)b_sc.p, st);
                 if (rc) return rc;
-                k_pipe_start<<<(nslot + 127) / 128, 128, 0, st>>>(V, nslot);
+                k_pipe_start<<<(nslot + 3) / 4, 128, 0, st>>>(V, nslot);
                 ctx->launches++;
                 rc = scmos ? zola_fit_batch_scmos_dev(ctx, fit_psf, R, (float*)b_rois.p, (float*)b_sv.p,
                                                       (double*)b_init.p, nslot, &fp, (double*)b_out5.p, nullptr,

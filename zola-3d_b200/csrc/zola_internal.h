@@ -249,6 +249,9 @@ int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_r
                    const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
                    double* d_nll, int* d_status, int* d_iters, cudaStream_t st);
 
+// library.cu: normalised R x R images at x = y = 0 and depths zwat[0 .. n), to the host
+int library_psfs(zola_psf* psf, int R, const double* zwat, int n, double* out);
+
 // fit_split.cu
 int launch_model_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n, double* d_out,
                        double* d_dout, cudaStream_t st);
