@@ -204,7 +204,8 @@ class Context:
         self.check(lib().zola_ctx_set_flow(self.h, int(units), arr), "zola_ctx_set_flow")
 
     def set_round_graphs(self, enable=True):
-        """Replay the round-based split kernels' 4-round blocks as CUDA graphs (default) or launch them one by one."""
+        """Replay a mixed batch's 4-round blocks of the round-based split kernels as CUDA graphs (default) or
+        launch them one by one, as a fit of one class always does."""
         self.check(lib().zola_ctx_set_round_graphs(self.h, int(bool(enable))), "zola_ctx_set_round_graphs")
 
     def set_tuning(self, enable=True, cache_path=None):

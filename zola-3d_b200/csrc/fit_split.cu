@@ -486,18 +486,58 @@ __device__ __forceinline__ int take_roi(const SplitDev& P, int n) {
 }
 
 // ----------------------------------------------- persistent-kernel helpers ----
-// True in every thread when any of the tiles blockIdx.x, + gridDim.x, ... (of g
-// slots each) holds a ROI.  A CTA without one leaves before it allocates TMEM
-// or loads constants (a draining pool's last rounds).
-__device__ __forceinline__ bool cta_has_live_tile(const SplitDev& P, int ntiles, int g) {
-    __shared__ int s_any;
-    if (threadIdx.x == 0) {
-        int any = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !any; tile += gridDim.x) any = tile_live(P, tile * g, g);
-        s_any = any;
-    }
+// Programmatic dependent launch (rounds of one class, launch_dependent): a kernel
+// may start while the one before it runs.  Nothing that kernel writes is read
+// before grid_wait, which returns once it has completed; grid_release then lets the
+// next kernel start, so it is launched, and has its constants on the way to shared
+// memory, by the time this one ends.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The units blockIdx.x, + gridDim.x, ... of this CTA that hold a ROI, found by all
+// threads at once and listed in shared memory.  (Every role walking the units by itself
+// waited for one load after the other.  With it and the launches ahead, a full round of
+// 16384 slots of 16 px went from 187 to 157 us, of 24 px from 386 to 330.)
+constexpr int MAX_CTA_UNITS = 256;
+struct LiveUnits {
+    short list[MAX_CTA_UNITS];
+    unsigned word[MAX_CTA_UNITS / 32];
+    int n;
+};
+
+// Fills L and returns the number of live units; a barrier for the whole CTA (at least
+// 256 threads).  Volatile loads: the answer may be taken before grid_wait, and must not
+// leave old lines in L1.
+__device__ __forceinline__ int find_live_units(const SplitDev& P, LiveUnits& L) {
+    const int UG = P.G1 > P.G2 ? P.G1 : P.G2, U = P.P / UG, t = threadIdx.x, u = blockIdx.x + t * gridDim.x;
+    bool live = false;
+    if (t < MAX_CTA_UNITS && u < U)
+        for (int k = 0; k < UG; ++k) live |= *(volatile const int*)(P.slot_roi + u * UG + k) >= 0;
+    const unsigned b = __ballot_sync(0xffffffffu, live);
+    __syncthreads();  // L is free again
+    if (t < MAX_CTA_UNITS && (t & 31) == 0) L.word[t >> 5] = b;
     __syncthreads();
-    return s_any != 0;
+    int before = 0, n = 0;
+    for (int w = 0; w < MAX_CTA_UNITS / 32; ++w) {
+        if (w < (t >> 5)) before += __popc(L.word[w]);
+        n += __popc(L.word[w]);
+    }
+    if (live) L.list[before + __popc(b & ((1u << (t & 31)) - 1))] = (short)u;
+    if (t == 0) L.n = n;
+    __syncthreads();
+    return n;
+}
+
+// Whether this CTA of a stage kernel has work.  A CTA without any leaves before it
+// allocates TMEM or loads constants (a draining pool's last rounds).  Only the LM
+// step and k_refill change what a slot holds, and the LM step empties slots or keeps
+// them occupied, so a CTA that sees work here goes on to its set-up at once; one
+// that sees none looks again when the kernel before it has completed.
+__device__ __forceinline__ bool stage_has_work(const SplitDev& P, LiveUnits& L) {
+    if (find_live_units(P, L)) return true;
+    grid_wait();
+    grid_release();
+    return find_live_units(P, L) != 0;
 }
 
 // Named barrier 1 over the first N threads of the CTA (the epilogue warps).
@@ -624,17 +664,20 @@ __device__ int unit_after_lm(const SplitDev& P, const FitIO& F, int u, int tag) 
 
 struct StaticUnits {
     static constexpr bool flow = false;
-    int u = -1;
+    LiveUnits* L;
+    int i = -1;
+    // Before the first unit, by every thread of the CTA: waits for the kernel before
+    // this one, and lists the units that still hold a ROI.
+    __device__ void begin(const SplitDev& P) {
+        grid_wait();
+        grid_release();
+        find_live_units(P, *L);
+    }
     // The next unit with a live slot, or -1.  Every calling thread walks the
     // same sequence.
-    __device__ int next(const SplitDev& P, int& tag, bool = false) {
-        const int UG = unit_slots(P.G1, P.G2), U = P.P / UG;
-        for (u = u < 0 ? (int)blockIdx.x : u + (int)gridDim.x; u < U; u += gridDim.x)
-            if (tile_live(P, u * UG, UG)) {
-                tag = 0;
-                return u;
-            }
-        return -1;
+    __device__ int next(const SplitDev&, int& tag, bool = false) {
+        tag = 0;
+        return ++i < L->n ? L->list[i] : -1;
     }
     __device__ void fence_writes() {}
     __device__ void release(const SplitDev&, int, int) {}
@@ -649,6 +692,7 @@ struct UnitRing {
 
 struct FlowUnits {
     static constexpr bool flow = true;
+    __device__ void begin(const SplitDev&) {}
     UnitRing* r;
     int stage, first, stride;  // this CTA serves units first, first + stride, ... at stage `stage`
     int q;
@@ -815,6 +859,7 @@ __device__ __forceinline__ void stage1_body(const SplitDev& P, const FitIO& F, U
         for (int s = 0; s < NS; ++s)
             umma::bulk_g2s(CS + s * SLAB, (const char*)P.bcs + (size_t)s * SLAB, SLAB, &cfull);
     }
+    units.begin(P);
 
     if (warp == SPLIT_THREADS / 32) {  // ---------------- MMA issuer (lane 0), scheduler (lane 1)
         if constexpr (UNITS::flow)
@@ -1105,8 +1150,9 @@ __device__ __forceinline__ void stage1_body(const SplitDev& P, const FitIO& F, U
 
 template <int W>
 __global__ void __launch_bounds__(S1_THREADS, 1) k_stage1p(SplitDev P, FitIO F) {
-    if (!cta_has_live_tile(P, P.P / unit_slots(P.G1, P.G2), unit_slots(P.G1, P.G2))) return;
-    stage1_body<W>(P, F, StaticUnits{});
+    __shared__ LiveUnits live;
+    if (!stage_has_work(P, live)) return;
+    stage1_body<W>(P, F, StaticUnits{&live});
 }
 
 
@@ -1150,6 +1196,12 @@ __device__ __forceinline__ void stage2_body(const SplitDev& P, const FitIO& F, U
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = tmem_base;
+    if (t == SPLIT_THREADS) {
+        umma::mbar_expect_tx(&cfull, (uint32_t)(NS * SLAB));
+        for (int s = 0; s < NS; ++s)
+            umma::bulk_g2s(CS + s * SLAB, (const char*)P.bcs + (size_t)s * SLAB, SLAB, &cfull);
+    }
+    units.begin(P);
 
     if (t >= SPLIT_THREADS) {  // ---------------- producer (lane 0), scheduler (lane 1)
         if constexpr (UNITS::flow)
@@ -1158,9 +1210,6 @@ __device__ __forceinline__ void stage2_body(const SplitDev& P, const FitIO& F, U
                 return;
             }
         if (t != SPLIT_THREADS) return;
-        umma::mbar_expect_tx(&cfull, (uint32_t)(NS * SLAB));
-        for (int s = 0; s < NS; ++s)
-            umma::bulk_g2s(CS + s * SLAB, (const char*)P.bcs + (size_t)s * SLAB, SLAB, &cfull);
         int q = 0;
         for (int tag = 0;;) {
             const int unit = units.next(P, tag, true);
@@ -1343,8 +1392,9 @@ __device__ __forceinline__ void stage2_body(const SplitDev& P, const FitIO& F, U
 
 template <int W>
 __global__ void __launch_bounds__(S2_THREADS, 1) k_stage2p(SplitDev P, FitIO F) {
-    if (!cta_has_live_tile(P, P.P / unit_slots(P.G1, P.G2), unit_slots(P.G1, P.G2))) return;
-    stage2_body<W>(P, F, StaticUnits{});
+    __shared__ LiveUnits live;
+    if (!stage_has_work(P, live)) return;
+    stage2_body<W>(P, F, StaticUnits{&live});
 }
 
 
@@ -1389,6 +1439,12 @@ __device__ __forceinline__ void stage3_body(const SplitDev& P, const FitIO& F, U
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = tmem_base;
+    if (t == SPLIT_THREADS) {
+        umma::mbar_expect_tx(&gfull, (uint32_t)(2 * gbytes));
+        umma::bulk_g2s(GT, P.gt_hi, (uint32_t)gbytes, &gfull);
+        umma::bulk_g2s(GT + gbytes, P.gt_lo, (uint32_t)gbytes, &gfull);
+    }
+    units.begin(P);
 
     if (warp == SPLIT_THREADS / 32) {  // ------- MMAs (lane 0), scheduler (lane 1) or A3 loader (lane 1, two buffers)
         if constexpr (UNITS::flow)
@@ -1423,9 +1479,6 @@ __device__ __forceinline__ void stage3_body(const SplitDev& P, const FitIO& F, U
             return;
         }
         if (lane != 0) return;
-        umma::mbar_expect_tx(&gfull, (uint32_t)(2 * gbytes));
-        umma::bulk_g2s(GT, P.gt_hi, (uint32_t)gbytes, &gfull);
-        umma::bulk_g2s(GT + gbytes, P.gt_lo, (uint32_t)gbytes, &gfull);
         bool ok = umma::mbar_wait(&gfull, 0, P.err);
         const uint32_t sbo = (W / 8) * 128;
         const uint32_t id = umma::idesc_f16(128, RP, false, false);
@@ -1516,8 +1569,9 @@ __device__ __forceinline__ void stage3_body(const SplitDev& P, const FitIO& F, U
 }
 
 __global__ void __launch_bounds__(S3_THREADS, 1) k_stage3(SplitDev P, FitIO F) {
-    if (!cta_has_live_tile(P, P.P / unit_slots(P.G1, P.G2), unit_slots(P.G1, P.G2))) return;
-    stage3_body(P, F, StaticUnits{});
+    __shared__ LiveUnits live;
+    if (!stage_has_work(P, live)) return;
+    stage3_body(P, F, StaticUnits{&live});
 }
 
 
@@ -1677,13 +1731,141 @@ __device__ __noinline__ void lm_slot(const SplitDev& P, const FitIO& io, int slo
     }
 }
 
-// The round-based fit's LM step: every occupied slot of the pool, one thread each.
-__global__ void k_lm(SplitDev P, FitIO F) {
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = slot < P.P && P.slot_roi[slot] >= 0;
-    const unsigned m = __ballot_sync(0xffffffffu, live);  // model evaluations: one atomic per warp
-    if (P.evals && (threadIdx.x & 31) == 0 && m) atomicAdd(P.evals, (unsigned long long)__popc(m));
-    if (live) lm_slot(P, F, slot);
+// The round-based fit's LM step: every occupied slot of the pool, eight lanes each.
+// The step is lm_slot's, with its serial solves side by side: lane 0 takes the
+// undamped one (the convergence test), lane 1 the damped one (the next trial point),
+// and lanes 0 - 4 a column each of the retiring ROI's CRLB.  A thread a slot, with the
+// state copied to local memory, took 11 to 17 us a round from a few slots to 16384;
+// this takes 9 to 14.
+constexpr int LM_SLOTS = 16;  // a CTA
+__global__ void __launch_bounds__(8 * LM_SLOTS) k_lm(SplitDev P, FitIO F) {
+    grid_wait();
+    grid_release();
+    const FitParamsDev& prm = F.prm;
+    const int l8 = threadIdx.x & 7, lead = threadIdx.x & 24, slot = blockIdx.x * LM_SLOTS + (threadIdx.x >> 3);
+    const int roi = slot < P.P ? P.slot_roi[slot] : -1;
+    const bool live = roi >= 0;
+    const unsigned all = 0xffffffffu, m = __ballot_sync(all, live && l8 == 0);
+    if (m == 0) return;  // the whole warp
+    if (P.evals && (threadIdx.x & 31) == 0) atomicAdd(P.evals, (unsigned long long)__popc(m));
+    LMState& S = P.lm[live ? slot : 0];
+    const double* tot = P.sums + (size_t)(live ? slot : 0) * NSUM;
+    const bool start = live && P.slot_phase[slot] == 0;
+    const double nll = tot[NRED] != 0.0 ? INFINITY : tot[0];
+    // accept or reject (lm_start, lm_update)
+    double th[5], lambda, f = nll;
+    int status = 2, evals = 1;
+    bool accept = true;
+    if (start) {
+        lambda = 1e-3;
+        status = isfinite(nll) ? 2 : -1;
+    } else {
+        evals = S.evals + 1;
+        const double old = S.nll;
+        accept = nll <= old || (S.pred <= prm.accept_nll && nll <= old + prm.accept_nll);
+        lambda = S.lambda;
+        if (accept) {
+            lambda = fmax(lambda * 0.1, 1e-7);
+        } else {
+            f = old;
+            lambda *= 10.0;
+            if (lambda > 1e7) status = 3;
+        }
+    }
+    double g[5], H[25];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        th[q] = accept ? S.trial[q] : S.th[q];
+        g[q] = accept ? tot[1 + q] : S.g[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+#pragma unroll
+        for (int r = 0; r <= q; ++r) H[q * 5 + r] = H[r * 5 + q] = accept ? tot[6 + q * (q + 1) / 2 + r] : S.H[q * 5 + r];
+    double d[5] = {0, 0, 0, 0, 0};
+    bool solved = false;
+    if (live && status == 2 && (l8 == 1 || (l8 == 0 && accept))) solved = lm_solve(H, g, l8 == 0 ? 0.0 : lambda, d);
+    const bool opt = solved && l8 == 0 && fmax(fabs(d[0]), fmax(fabs(d[1]), fabs(d[2]))) < prm.tol_xyz &&
+                     fabs(d[3]) < 1e-4 * th[3] && fabs(d[4]) < 1e-4 * fmax(th[4], 1.0);
+    if (__shfl_sync(all, opt, lead)) status = 1;
+    __syncwarp();  // every lane has read the old state
+    // the next trial point (lm_propose), by lane 1
+    bool more = false;
+    if (live && l8 == 1) {
+        while (status == 2 && evals < prm.max_iter) {
+            if (!solved) {
+                lambda *= 10.0;
+                if (lambda > 1e7) status = 3;
+                else solved = lm_solve(H, g, lambda, d);
+                continue;
+            }
+            const double sxy = fmax(fabs(d[0]), fabs(d[1]));
+            double scale = 1.0;
+            if (sxy > prm.step_xy) scale = prm.step_xy / sxy;
+            if (fabs(d[2]) * scale > prm.step_z) scale = prm.step_z / fabs(d[2]);
+            double t[5], dl[5], hd = 0, gd = 0;
+            for (int q = 0; q < 5; ++q) t[q] = th[q] + scale * d[q];
+            lm_clamp(t, prm);
+            for (int q = 0; q < 5; ++q) dl[q] = t[q] - th[q];
+            for (int q = 0; q < 5; ++q) {
+                gd += g[q] * dl[q];
+                for (int r = 0; r < 5; ++r) hd += dl[q] * H[q * 5 + r] * dl[r];
+            }
+            for (int q = 0; q < 5; ++q) S.trial[q] = t[q];
+            S.step = fmax(fabs(dl[0]), fmax(fabs(dl[1]), fabs(dl[2])));
+            S.pred = -(gd + 0.5 * hd);
+            more = true;
+            break;
+        }
+        S.nll = f;
+        S.lambda = lambda;
+        S.evals = evals;
+        S.status = status;
+        if (start) P.slot_phase[slot] = 1;
+    }
+    more = __shfl_sync(all, more, lead + 1);
+    if (!live) return;
+    if (more) {
+        if (accept) {  // the accepted point, its gradient, Hessian and Fisher matrix
+            if (l8 == 1)
+                for (int q = 0; q < 5; ++q) S.th[q] = th[q];
+            if (l8 < 5) S.g[l8] = tot[1 + l8];
+            for (int e = l8; e < 25; e += 8) {
+                const int q = max(e / 5, e % 5), r = min(e / 5, e % 5), o = 6 + q * (q + 1) / 2 + r;
+                S.H[e] = tot[o];
+                S.F[e] = tot[o + 15];
+            }
+        }
+        return;
+    }
+    // retire
+    if (F.crlb5 && l8 < 5) {  // column l8 of F^-1 (lm_crlb)
+        double A[25], rhs[5], col[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+            for (int r = 0; r <= q; ++r) A[q * 5 + r] = A[r * 5 + q] = accept ? tot[21 + q * (q + 1) / 2 + r] : S.F[q * 5 + r];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) rhs[q] = q == l8 ? -1.0 : 0.0;
+        const bool ok = lm_solve(A, rhs, 0.0, col);
+        double v = col[0];
+#pragma unroll
+        for (int q = 1; q < 5; ++q) v = q == l8 ? col[q] : v;
+        F.crlb5[5 * (size_t)roi + l8] = ok ? sqrt(v) : NAN;
+    }
+    if (l8 == 1) {
+        for (int q = 0; q < 5; ++q) F.out5[5 * (size_t)roi + q] = th[q];
+        if (F.nll) F.nll[roi] = f;
+        if (F.status) F.status[roi] = status;
+        if (F.iters) F.iters[roi] = evals;
+        const int next = take_roi(P, F.n);  // refill from the queue
+        if (next >= 0) {
+            slot_take(P, F, slot, next);
+        } else {
+            P.slot_roi[slot] = -1;
+            atomicSub(P.active, 1);
+        }
+    }
 }
 
 // ------------------------------------------------- LM stage (dataflow) -----
@@ -1845,6 +2027,12 @@ __device__ __forceinline__ void stage45_body(const SplitDev& P, const FitIO& F, 
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = tmem_base;
+    if (t == E45_THREADS) {
+        umma::mbar_expect_tx(&gfull, 2 * garr);
+        umma::bulk_g2s(G, P.g128_hi, garr, &gfull);
+        umma::bulk_g2s(G + garr, P.g128_lo, garr, &gfull);
+    }
+    units.begin(P);
 
     if (warp == E45_THREADS / 32) {  // ---------------- producer (lane 0), scheduler (lane 1)
         if constexpr (UNITS::flow)
@@ -1853,9 +2041,6 @@ __device__ __forceinline__ void stage45_body(const SplitDev& P, const FitIO& F, 
                 return;
             }
         if (lane != 0) return;
-        umma::mbar_expect_tx(&gfull, 2 * garr);
-        umma::bulk_g2s(G, P.g128_hi, garr, &gfull);
-        umma::bulk_g2s(G + garr, P.g128_lo, garr, &gfull);
         int q = 0, n = 0;
         bool ok = true;
         for (int tag = 0; ok;) {
@@ -2086,8 +2271,9 @@ __device__ __forceinline__ void stage45_body(const SplitDev& P, const FitIO& F, 
 }
 
 __global__ void __launch_bounds__(S45_THREADS, 1) k_stage45p(SplitDev P, FitIO F) {
-    if (!cta_has_live_tile(P, P.P / unit_slots(P.G1, P.G2), unit_slots(P.G1, P.G2))) return;
-    stage45_body(P, F, StaticUnits{});
+    __shared__ LiveUnits live;
+    if (!stage_has_work(P, live)) return;
+    stage45_body(P, F, StaticUnits{&live});
 }
 
 // Likelihood sums of a unit's live slots from their maps in shared memory (slot
@@ -2318,6 +2504,12 @@ __device__ __forceinline__ void stage45s_body(const SplitDev& P, const FitIO& F,
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = tmem_base;
+    if (t == SPLIT_THREADS) {
+        umma::mbar_expect_tx(&gfull, 2 * garr);
+        umma::bulk_g2s(G, P.g128_hi, garr, &gfull);
+        umma::bulk_g2s(G + garr, P.g128_lo, garr, &gfull);
+    }
+    units.begin(P);
 
     if (warp == SPLIT_THREADS / 32) {  // ---------------- loads + MMAs (lane 0), scheduler (lane 1)
         if constexpr (UNITS::flow)
@@ -2326,9 +2518,6 @@ __device__ __forceinline__ void stage45s_body(const SplitDev& P, const FitIO& F,
                 return;
             }
         if (lane != 0) return;
-        umma::mbar_expect_tx(&gfull, 2 * garr);
-        umma::bulk_g2s(G, P.g128_hi, garr, &gfull);
-        umma::bulk_g2s(G + garr, P.g128_lo, garr, &gfull);
         bool ok = umma::mbar_wait(&gfull, 0, P.err);
         const uint32_t id = umma::idesc_f16(128, NT, false, true);
         const uint32_t ghi = umma::smem_u32(G), glo = ghi + garr;
@@ -2376,8 +2565,9 @@ __device__ __forceinline__ void stage45s_body(const SplitDev& P, const FitIO& F,
 }
 
 __global__ void __launch_bounds__(S45S_THREADS, 1) k_stage45s(SplitDev P, FitIO F) {
-    if (!cta_has_live_tile(P, P.P / unit_slots(P.G1, P.G2), unit_slots(P.G1, P.G2))) return;
-    stage45s_body(P, F, StaticUnits{});
+    __shared__ LiveUnits live;
+    if (!stage_has_work(P, live)) return;
+    stage45s_body(P, F, StaticUnits{&live});
 }
 
 
@@ -2725,16 +2915,17 @@ __global__ void k_init_slots(SplitDev P, const double* init, int n, int navail, 
     if (slot >= P.P) return;
     if (avail) navail = *(volatile const int*)avail;
     const int m = n < navail ? n : navail;
-    if (slot < m) {
-        P.slot_roi[slot] = slot;
+    // ROI r starts in unit r mod U: a few ROIs get a unit each (see setup_pool)
+    const int UG = unit_slots(P.G1, P.G2), U = P.P / UG, u = slot / UG, r = (slot - u * UG) * U + u;
+    if (r < m) {
+        P.slot_roi[slot] = r;
         P.slot_phase[slot] = 0;
-        for (int q = 0; q < 5; ++q) P.lm[slot].trial[q] = init[5 * slot + q];
+        for (int q = 0; q < 5; ++q) P.lm[slot].trial[q] = init[5 * r + q];
         lm_clamp(P.lm[slot].trial, prm);
     } else {
         P.slot_roi[slot] = -1;
     }
-    const int UG = unit_slots(P.G1, P.G2);
-    if (slot % UG == 0) P.ustate[slot / UG] = slot < m || navail < n ? 0 : UNIT_DEAD;
+    if (slot == u * UG) P.ustate[u] = r < m || navail < n ? 0 : UNIT_DEAD;
     if (slot == 0) {
         *P.queue = P.P < m ? P.P : m;
         *P.active = P.P < m ? P.P : m;
@@ -2911,24 +3102,34 @@ static cudaError_t smem_attrs(int W, const SplitPool& sp) {
 
 static int unit_grid(zola_ctx* ctx, const SplitPool& sp) { return std::min(sp.U, ctx->num_sms); }
 
-static void launch_stage1(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st) {
-    const int grid = unit_grid(ctx, sp);
-    if (sp.D.W == 32)
-        k_stage1p<32><<<grid, S1_THREADS, sp.s1, st>>>(sp.D, F);
-    else if (sp.D.W == 64)
-        k_stage1p<64><<<grid, S1_THREADS, sp.s1, st>>>(sp.D, F);
-    else
-        k_stage1p<128><<<grid, S1_THREADS, sp.s1, st>>>(sp.D, F);
+// Launch a kernel of a round; dep: it may start while the one before it runs (see
+// grid_wait).  Used where one class has the GPU to itself: a mixed batch's classes
+// would hold SMs that another class could use.
+static void launch_dependent(bool dep, void (*kernel)(SplitDev, FitIO), int grid, int threads, size_t smem,
+                             const SplitDev& D, const FitIO& F, cudaStream_t st) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dep ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, D, F);
 }
 
-static void launch_stage2(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st) {
+static void launch_stage1(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st, bool dep = false) {
     const int grid = unit_grid(ctx, sp);
-    if (sp.D.W == 32)
-        k_stage2p<32><<<grid, S2_THREADS, sp.s2, st>>>(sp.D, F);
-    else if (sp.D.W == 64)
-        k_stage2p<64><<<grid, S2_THREADS, sp.s2, st>>>(sp.D, F);
-    else
-        k_stage2p<128><<<grid, S2_THREADS, sp.s2, st>>>(sp.D, F);
+    auto kernel = sp.D.W == 32 ? k_stage1p<32> : sp.D.W == 64 ? k_stage1p<64> : k_stage1p<128>;
+    launch_dependent(dep, kernel, grid, S1_THREADS, sp.s1, sp.D, F, st);
+}
+
+static void launch_stage2(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st, bool dep = false) {
+    const int grid = unit_grid(ctx, sp);
+    auto kernel = sp.D.W == 32 ? k_stage2p<32> : sp.D.W == 64 ? k_stage2p<64> : k_stage2p<128>;
+    launch_dependent(dep, kernel, grid, S2_THREADS, sp.s2, sp.D, F, st);
 }
 
 // Pool of slots for n ROIs: at most pmax slots (0: state up to 8 GB, at most
@@ -2973,8 +3174,13 @@ static int setup_pool(zola_ctx* ctx, zola_psf* p, WindowTables* w, int n, int pm
     int Pmax = (int)std::min<size_t>(32768, ((size_t)8 << 30) / per_slot);  // at most 8 GB of pool state
     if (pmax_override > 0) Pmax = std::min(Pmax, pmax_override);
     if (max_units > 0) Pmax = std::min(Pmax, max_units * UG);
+    Pmax = std::min(Pmax, MAX_CTA_UNITS * ctx->num_sms * UG);  // (32768 slots and more at 148 SMs)
     Pmax = std::max(UG, Pmax / UG * UG);
-    const int P = std::min(Pmax, (n + UG - 1) / UG * UG);
+    // Fewer ROIs than a unit a SM holds: as many units as ROIs or SMs, so that no CTA
+    // works through several slots while others have none (100 fits of 40 px: 1.84 ms
+    // instead of 2.02; at 16 and 24 px a round costs the same either way).
+    const int spread = std::min(n, ctx->num_sms) * UG;
+    const int P = std::min(Pmax, std::max((n + UG - 1) / UG * UG, spread));
     sp.U = P / UG;
     auto al = [](size_t v) { return (v + 1023) / 1024 * 1024; };
     const size_t b_a2 = al((size_t)(P / pl->G2) * a2_tile_bytes(pl->K1));
@@ -3034,15 +3240,15 @@ static int setup_pool(zola_ctx* ctx, zola_psf* p, WindowTables* w, int n, int pm
 }
 
 // Stages 1-3 (pupil DFT, window DFT, row blur) of every occupied slot.
-static void launch_stages123(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st) {
+static void launch_stages123(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st, bool dep = false) {
     prof_begin(ctx, 0, st);
-    launch_stage1(ctx, sp, F, st);
+    launch_stage1(ctx, sp, F, st, dep);
     prof_end(ctx, st);
     prof_begin(ctx, 1, st);
-    launch_stage2(ctx, sp, F, st);
+    launch_stage2(ctx, sp, F, st, dep);
     prof_end(ctx, st);
     prof_begin(ctx, 2, st);
-    k_stage3<<<unit_grid(ctx, sp), S3_THREADS, sp.s3, st>>>(sp.D, F);
+    launch_dependent(dep, k_stage3, unit_grid(ctx, sp), S3_THREADS, sp.s3, sp.D, F, st);
     prof_end(ctx, st);
     ctx->launches += 3;
 }
@@ -3384,29 +3590,30 @@ bool flow_shape(zola_ctx* ctx, zola_psf* p, WindowTables* w, FlowShape* out, dou
 // never leave the SM).  Smaller windows: the unit's maps go to shared memory
 // and its slots are summed together.  The two sum in different orders; the
 // choice depends on R alone so that a fit never depends on the batch it is in.
-static void issue_round(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st) {
-    launch_stages123(ctx, sp, F, st);
+static void issue_round(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st, bool dep) {
+    dep = dep && !ctx->profile;  // (the profile's events stand between the kernels)
+    launch_stages123(ctx, sp, F, st, dep);
     prof_begin(ctx, 3, st);
-    if (sp.pl->W >= S45_MIN_W)
-        k_stage45p<<<unit_grid(ctx, sp), S45_THREADS, sp.s45, st>>>(sp.D, F);
-    else
-        k_stage45s<<<unit_grid(ctx, sp), S45S_THREADS, sp.s45, st>>>(sp.D, F);
+    if (sp.pl->W >= S45_MIN_W) launch_dependent(dep, k_stage45p, unit_grid(ctx, sp), S45_THREADS, sp.s45, sp.D, F, st);
+    else launch_dependent(dep, k_stage45s, unit_grid(ctx, sp), S45S_THREADS, sp.s45, sp.D, F, st);
     prof_end(ctx, st);
     prof_begin(ctx, 7, st);
-    k_lm<<<(sp.D.P + 127) / 128, 128, 0, st>>>(sp.D, F);
+    launch_dependent(dep, k_lm, (sp.D.P + LM_SLOTS - 1) / LM_SLOTS, 8 * LM_SLOTS, 0, sp.D, F, st);
     prof_end(ctx, st);
     ctx->launches += 2;
 }
 
 // Four rounds: 20 launches whose arguments stay the same for the whole fit.
-static void issue_rounds(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st) {
-    for (int k = 0; k < 4; ++k) issue_round(ctx, sp, F, st);
+static void issue_rounds(zola_ctx* ctx, const SplitPool& sp, const FitIO& F, cudaStream_t st, bool dep) {
+    for (int k = 0; k < 4; ++k) issue_round(ctx, sp, F, st, dep);
 }
 
-// The four rounds captured once per fit as a CUDA graph and replayed between
-// the host's flag reads: one launch instead of 20 per block.  Not with the
-// context's kernel profiling on (its events bracket single launches); if the
-// capture fails the rounds are issued directly.
+// The four rounds of a mixed batch's class captured once per fit as a CUDA graph and
+// replayed between the host's flag reads: one launch instead of 20 per block.  Not with
+// the context's kernel profiling on (its events bracket single launches); if the
+// capture fails the rounds are issued directly.  A fit of one class issues its rounds
+// directly: with dependent launches a graph of them runs no faster (2.53 against 2.55
+// ms for 52 rounds, 0.72 against 0.58 ms for 9), and capturing one takes 150 us.
 struct RoundGraph {
     cudaGraphExec_t exec = nullptr;
     RoundGraph() = default;
@@ -3421,7 +3628,7 @@ struct RoundGraph {
             return;
         }
         const long long l0 = ctx->launches;
-        issue_rounds(ctx, sp, F, st);
+        issue_rounds(ctx, sp, F, st, false);
         ctx->launches = l0;
         if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) {
             cudaGetLastError();
@@ -3438,7 +3645,7 @@ struct RoundGraph {
             ctx->launches += 20;
             return;
         }
-        issue_rounds(ctx, sp, F, st);
+        issue_rounds(ctx, sp, F, st, false);
     }
 };
 
@@ -3468,6 +3675,10 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
     // inputs still arriving: the fit starts on the first chunk, and chunks are
     // handed to the pool as their copies complete
     int chunk = 0, navail = n, queue = 0;
+    if (feed && feed->n_chunks == 1) {  // all of them at once
+        ZOLA_CUDA_CHECK(cudaStreamWaitEvent(st, feed->ev[0], 0), ctx);
+        feed = nullptr;
+    }
     if (feed && feed->n_chunks > 0) {
         ZOLA_CUDA_CHECK(cudaStreamWaitEvent(st, feed->ev[0], 0), ctx);
         navail = feed->chunk_end[0];
@@ -3495,11 +3706,9 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
     const int max_rounds = (prm->max_iter + 2) * ((n + P - 1) / P + 1) + 8 + 4 * (feed ? feed->n_chunks : 0);
     int rounds = 0;
     const bool fused = ctx->split_mode == ZOLA_SPLIT_FUSED && fused_fits(*sp.pl);
-    RoundGraph graph;
-    if (!fused && !feed) graph.capture(ctx, sp, F, st);
     while (true) {
-        if (!fused && !feed) {
-            graph.run(ctx, sp, F, st);
+        if (!fused && (!feed || queue >= n)) {  // every ROI is in a slot or done: nothing left to refill
+            issue_rounds(ctx, sp, F, st, true);
         } else for (int k = 0; k < 4; ++k) {
             if (feed && queue < n) {  // idle slots take ROIs that arrived since
                 k_refill<<<(P + 127) / 128, 128, 0, st>>>(D, d_init, n, fp);
@@ -3516,7 +3725,7 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
                 ctx->launches += 2;
                 continue;
             }
-            issue_round(ctx, sp, F, st);
+            issue_round(ctx, sp, F, st, true);
         }
         rounds += 4;
         ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
@@ -3640,7 +3849,7 @@ int launch_fit_split_mixed(zola_ctx* ctx, int nc, MixedClass* mc, cudaStream_t s
                 for (int k = 0; k < 4; ++k) {  // idle slots take ROIs that arrived since
                     k_refill<<<(p.D.P + 127) / 128, 128, 0, cs>>>(p.D, mc[c].F.init, mc[c].F.n, mc[c].F.prm);
                     ctx->launches++;
-                    issue_round(ctx, p, mc[c].F, cs);
+                    issue_round(ctx, p, mc[c].F, cs, false);
                 }
             } else {
                 if (S[c].feed && !graphs[c].exec) graphs[c].capture(ctx, p, mc[c].F, cs);  // every ROI taken
