@@ -104,6 +104,9 @@ struct SplitDev {
     int* slot_roi;
     int* slot_phase;
     LMState* lm;
+    LMState* pack;  // k_pack_gather: the occupied slots of a draining pool
+    int* pack_roi;  // ROI and phase of each
+    int* n_packed;
     int* queue;    // next ROI to hand out
     int* active;   // occupied slots
     int* err;      // bounded-wait timeout flag
@@ -2952,6 +2955,45 @@ __global__ void k_refill(SplitDev P, const double* init, int n, FitParamsDev prm
 
 __global__ void k_set_int(int* p, int v) { *p = v; }
 
+// Once the ROI queue is empty the pool drains, and units of two or four slots with one
+// fit left cost as much as full ones.  k_pack_gather takes the occupied slots' states
+// into P.pack (any order: a fit does not depend on its slot) and empties the slots;
+// k_pack_scatter puts them back, into whole units while there are more than a unit a SM
+// of them, else evenly over the SMs.  Eight lanes a slot; 10 us for both at 16384.
+__global__ void __launch_bounds__(256) k_pack_gather(SplitDev P) {
+    const int slot = blockIdx.x * 32 + (threadIdx.x >> 3), l8 = threadIdx.x & 7, lead = threadIdx.x & 24;
+    const int roi = slot < P.P ? P.slot_roi[slot] : -1;
+    int o = 0;
+    if (roi >= 0 && l8 == 0) o = atomicAdd(P.n_packed, 1);
+    o = __shfl_sync(0xffffffffu, o, lead);
+    if (roi < 0) return;
+    const int phase = P.slot_phase[slot];
+    const double* a = (const double*)(P.lm + slot);
+    double* b = (double*)(P.pack + o);
+    for (int k = l8; k < (int)(sizeof(LMState) / 8); k += 8) b[k] = a[k];
+    __syncwarp(0xffu << lead);
+    if (l8 == 0) {
+        P.pack_roi[2 * o] = roi;
+        P.pack_roi[2 * o + 1] = phase;
+        P.slot_roi[slot] = -1;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_pack_scatter(SplitDev P, int sms) {
+    const int i = blockIdx.x * 32 + (threadIdx.x >> 3), l8 = threadIdx.x & 7, n = *P.n_packed;
+    if (i >= n) return;
+    const int UG = unit_slots(P.G1, P.G2), U = max((n + UG - 1) / UG, min(n, sms));
+    const int slot = i % U * UG + i / U;
+    const double* a = (const double*)(P.pack + i);
+    double* b = (double*)(P.lm + slot);
+    for (int k = l8; k < (int)(sizeof(LMState) / 8); k += 8) b[k] = a[k];
+    if (l8 == 0) {
+        P.slot_roi[slot] = P.pack_roi[2 * i];
+        P.slot_phase[slot] = P.pack_roi[2 * i + 1];
+    }
+}
+static_assert(sizeof(LMState) % 8 == 0, "packed by doubles");
+
 // ------------------------------------------------------- dataflow kernel ----
 // The whole fit in one cooperative launch: CTAs [first[s], first[s + 1]) run
 // stage s (pupil DFT, window DFT, row blur, column blur + sums, LM step) on the
@@ -3189,9 +3231,10 @@ static int setup_pool(zola_ctx* ctx, zola_psf* p, WindowTables* w, int n, int pm
     const size_t b_t = al((size_t)P * 4 * pl->R * pl->R * 4);
     const size_t b_lm = al((size_t)P * sizeof(LMState));
     const size_t b_sums = al((size_t)P * NSUM * 8);
+    const size_t b_pack = al((size_t)P * (sizeof(LMState) + 8) + 8);
     const size_t b_int = al((size_t)P * 8 + (size_t)sp.U * 4 + 64);
     const size_t b_clk = al(((size_t)3 * ctx->num_sms + 1) * 8);
-    const size_t total = b_a2 + b_a3 + b_a4 + b_t + b_lm + b_sums + b_clk + b_int;
+    const size_t total = b_a2 + b_a3 + b_a4 + b_t + b_lm + b_sums + b_pack + b_clk + b_int;
     if (need) {
         *need = total;
         return ZOLA_OK;
@@ -3213,6 +3256,10 @@ static int setup_pool(zola_ctx* ctx, zola_psf* p, WindowTables* w, int n, int pm
     D.tmaps = (float*)base; base += b_t;
     D.lm = (LMState*)base; base += b_lm;
     D.sums = (double*)base; base += b_sums;
+    D.pack = (LMState*)base;
+    D.pack_roi = (int*)(D.pack + P);
+    D.n_packed = D.pack_roi + 2 * P;
+    base += b_pack;
     D.evals = (unsigned long long*)base;
     D.clk = D.evals + 1;
     base += b_clk;
@@ -3251,6 +3298,24 @@ static void launch_stages123(zola_ctx* ctx, const SplitPool& sp, const FitIO& F,
     launch_dependent(dep, k_stage3, unit_grid(ctx, sp), S3_THREADS, sp.s3, sp.D, F, st);
     prof_end(ctx, st);
     ctx->launches += 3;
+}
+
+// Packs a draining pool when it is worth it: `held` slots were occupied or waited for
+// after the last packing, `active` are.  Between two blocks of rounds.  Never packing,
+// and packing at 0.3, 0.5, 0.7, 0.8 and 0.9 of `held`: a mixed batch of 100,000 takes
+// 87.2, 81.5, 80.3, 79.3, 78.9 and 78.9 ms, 9,000 fits of 24 px 12.9, 11.0, 10.9, 10.9,
+// 10.7 and 10.6, 3,001 of 40 px 13.0 and then 11.6 throughout.  A pool with a ROI or
+// less a SM has nothing to gain.
+static int pack_pool(zola_ctx* ctx, const SplitPool& sp, int active, int* held, cudaStream_t st) {
+    const SplitDev& D = sp.D;
+    const int UG = unit_slots(D.G1, D.G2);
+    if (*held <= ctx->num_sms || active > 0.8 * *held) return ZOLA_OK;
+    ZOLA_CUDA_CHECK(cudaMemsetAsync(D.n_packed, 0, sizeof(int), st), ctx);
+    k_pack_gather<<<(D.P + 31) / 32, 256, 0, st>>>(D);
+    k_pack_scatter<<<(active + 31) / 32, 256, 0, st>>>(D, std::min(ctx->num_sms, D.P / UG));
+    ctx->launches += 2;
+    *held = active;
+    return ZOLA_OK;
 }
 
 static int read_flags(zola_ctx* ctx, const SplitDev& D, cudaStream_t st, int* active, int* err, int* queue = nullptr) {
@@ -3704,7 +3769,7 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
     ctx->launches++;
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
     const int max_rounds = (prm->max_iter + 2) * ((n + P - 1) / P + 1) + 8 + 4 * (feed ? feed->n_chunks : 0);
-    int rounds = 0;
+    int rounds = 0, held = std::min(P, n);
     const bool fused = ctx->split_mode == ZOLA_SPLIT_FUSED && fused_fits(*sp.pl);
     while (true) {
         if (!fused && (!feed || queue >= n)) {  // every ROI is in a slot or done: nothing left to refill
@@ -3740,6 +3805,7 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
             if (navail <= queue && (rc = poll_feed(true))) return rc;
         }
         if (rounds > max_rounds) { ctx->err = "split fit: did not drain the ROI queue"; return ZOLA_E_TIMEOUT; }
+        if (queue >= n && !fused && (rc = pack_pool(ctx, sp, active, &held, st))) return rc;
     }
     if (trial) {  // device time per model evaluation of this pool size
         unsigned long long evals = 0;
@@ -3792,7 +3858,7 @@ int launch_fit_split_mixed(zola_ctx* ctx, int nc, MixedClass* mc, cudaStream_t s
     // first chunk; between blocks of rounds the host hands it the chunks that have
     // landed (the device count of arrived ROIs), and idle slots take them.
     struct State {
-        int rounds = 0, max_rounds = 0, chunk = 0, navail = 0, queue = 0;
+        int rounds = 0, max_rounds = 0, chunk = 0, navail = 0, queue = 0, held = 0;
         bool done = false, feed = false;
     };
     std::vector<State> S(nc);
@@ -3815,6 +3881,7 @@ int launch_fit_split_mixed(zola_ctx* ctx, int nc, MixedClass* mc, cudaStream_t s
         ctx->launches++;
         S[c].max_rounds = (F.prm.max_iter + 2) * ((F.n + D.P - 1) / D.P + 1) + 8 + (S[c].feed ? 4 * feeds[c].n_chunks : 0);
         S[c].done = F.n == 0;
+        S[c].held = std::min(D.P, F.n);
         if (!S[c].done && !S[c].feed) graphs[c].capture(ctx, sp[c], F, cs);
     }
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
@@ -3881,6 +3948,8 @@ int launch_fit_split_mixed(zola_ctx* ctx, int nc, MixedClass* mc, cudaStream_t s
             else if (S[c].rounds > S[c].max_rounds) {
                 ctx->err = "split fit: did not drain the ROI queue";
                 return ZOLA_E_TIMEOUT;
+            } else if (queue >= mc[c].F.n) {
+                if (int rc = pack_pool(ctx, sp[c], active, &S[c].held, ctx->mix_stream[c])) return rc;
             }
         }
     }
