@@ -153,6 +153,7 @@ int zola_ctx_destroy(zola_ctx* ctx) {
     if (ctx->calib_fit_area) cudaFree(ctx->calib_fit_area);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
+    if (ctx->h_post) cudaFreeHost(ctx->h_post);
     if (ctx->h_feed) cudaFreeHost(ctx->h_feed);
     if (ctx->h_tune) cudaFreeHost(ctx->h_tune);
     if (ctx->h_mix) cudaFreeHost(ctx->h_mix);

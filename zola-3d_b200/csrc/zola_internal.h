@@ -128,6 +128,8 @@ struct zola_ctx {
     int* d_counter = nullptr;
     int* d_status_word = nullptr;
     int* h_flags = nullptr;      // pinned host words read back by the split fit loop
+    int* h_post = nullptr;       // pinned ring the split fit's rounds report to
+    unsigned post_seq = 0;       // report numbers used so far
     int split_pool_max = 0;      // 0: size the split slot pool automatically
     bool round_graphs = true;    // replay a mixed batch's round-based kernels as CUDA graphs
     int split_mode = ZOLA_SPLIT_STAGED;  // ZOLA_SPLIT_STAGED, _FUSED or _FLOW
