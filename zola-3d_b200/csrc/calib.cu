@@ -893,7 +893,7 @@ int cal_setup(zola_psf* p, const zola_calib_data* cd, CalRun& run) {
                             std::min<size_t>(CAL_CLUSTERS, nbs * 256) * run.per_cluster};
     cudaError_t e = carve(&ctx->calib_area, &ctx->calib_bytes, q, bytes, 9);
     cudaStream_t st = ctx->stream;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(run.d_stacks, cd->stacks, nbs * RR * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = copy_in(ctx, run.d_stacks, cd->stacks, nbs * RR * 8, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(run.d_const, cd->dz, (size_t)ns * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && cd->photons)
         e = cudaMemcpyAsync(run.d_const + ns, cd->photons, nbs * 8, cudaMemcpyHostToDevice, st);

@@ -1114,10 +1114,10 @@ int detect_impl(zola_detector* d, const double* frames, const uint16_t* u16, con
     double* dout = (double*)(io + b_df + b_dc + b_du);
     cudaError_t e = cudaSuccess;
     if (u16) {
-        e = cudaMemcpyAsync(du, u16, SS * nframes * 2, cudaMemcpyHostToDevice, ctx->stream);
+        e = copy_in(ctx, du, u16, SS * nframes * 2, ctx->stream);
         if (e == cudaSuccess) rescale_u16(ctx, du, SS * nframes, rescale, df, ctx->stream);
     } else {
-        e = cudaMemcpyAsync(df, frames, SS * nframes * 8, cudaMemcpyHostToDevice, ctx->stream);
+        e = copy_in(ctx, df, frames, SS * nframes * 8, ctx->stream);
     }
     int rc = e == cudaSuccess ? detect_frames(d, df, nframes, room0, cap, cap, dout, dc, nullptr, ctx->stream) : ZOLA_OK;
     if (e == cudaSuccess && rc == ZOLA_OK) {

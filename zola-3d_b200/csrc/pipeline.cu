@@ -583,7 +583,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
         const int nf = std::min(FB, nframes - f0);
         V.nframes = nf;
         if (scmos) {
-            e = cudaMemcpyAsync(b_adu.p, adu + (size_t)f0 * SS, SS * nf * 4, cudaMemcpyHostToDevice, st);
+            e = copy_in(ctx, b_adu.p, adu + (size_t)f0 * SS, SS * nf * 4, st);
             if (e == cudaSuccess) {
                 k_pipe_scmos<<<ctx->num_sms * 8, 256, 0, st>>>((float*)b_adu.p, (double*)b_off.p, (double*)b_gain.p,
                                                               (double*)b_vg.p, SS, nf, (double*)b_img.p,
@@ -591,10 +591,10 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 ctx->launches++;
             }
         } else if (u16) {  // 2 bytes a pixel over the host link, photons made on the device
-            e = cudaMemcpyAsync(b_u16.p, u16 + (size_t)f0 * SS, SS * nf * 2, cudaMemcpyHostToDevice, st);
+            e = copy_in(ctx, b_u16.p, u16 + (size_t)f0 * SS, SS * nf * 2, st);
             if (e == cudaSuccess) rescale_u16(ctx, (const uint16_t*)b_u16.p, SS * nf, rescale, (double*)b_img.p, st);
         } else {
-            e = cudaMemcpyAsync(b_img.p, frames + (size_t)f0 * SS, SS * nf * 8, cudaMemcpyHostToDevice, st);
+            e = copy_in(ctx, b_img.p, frames + (size_t)f0 * SS, SS * nf * 8, st);
         }
         if (e == cudaSuccess) e = cudaMemsetAsync(b_mask.p, 0, SS * nf, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(b_ptr.p, 0, (size_t)nf * 4, st);

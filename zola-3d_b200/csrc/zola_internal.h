@@ -104,6 +104,7 @@ struct PoolTune {
     int trials = 0;
     bool done = false;
 };
+struct HostCopy;
 }  // namespace zola
 
 struct zola_ctx {
@@ -128,6 +129,8 @@ struct zola_ctx {
     int* d_counter = nullptr;
     int* d_status_word = nullptr;
     int* h_flags = nullptr;      // pinned host words read back by the split fit loop
+    zola::HostCopy* host_copy = nullptr;  // helpers of large pageable copies
+    char* h_stage = nullptr;     // pinned staging of small host-buffer fits
     int* h_post = nullptr;       // pinned ring the split fit's rounds report to
     unsigned post_seq = 0;       // report numbers used so far
     int split_pool_max = 0;      // 0: size the split slot pool automatically
@@ -250,6 +253,13 @@ int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* 
 int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_rois, const float* d_scmos,
                    const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
                    double* d_nll, int* d_status, int* d_iters, cudaStream_t st);
+
+// host_copy.cu: a context's copies from and to host memory of any kind.  As with
+// cudaMemcpyAsync, src may be written again when copy_in returns, and dst may be read when
+// st has been synchronised after copy_out.
+cudaError_t copy_in(zola_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
+cudaError_t copy_out(zola_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
+void host_copy_free(zola_ctx* ctx);
 
 // library.cu: normalised R x R images at x = y = 0 and depths zwat[0 .. n), to the host
 int library_psfs(zola_psf* psf, int R, const double* zwat, int n, double* out);
