@@ -401,32 +401,109 @@ __device__ int block_exclusive_scan(int v, int* wtot, int* total) {
 // the tmp that slice r sees at a pixel is the one of the last slice r' <= r with
 // a positive score there (0: none, or outside the border), which any thread can
 // find by itself: slices need no order, and only pixels that pass the first two
-// tests look at their column.  48 frames of 256^2 x 40 take 1.2 ms and two of
-// 130^2 x 12 take 6 us; one CTA a frame, slice after slice, took 6.4 ms and 375 us.
+// tests look at their column.
+//
+// Two kernels: k_det_look reads every score once and leaves one pixel in some
+// 200, which k_det_peaks tests in full.  48 frames of 256^2 x 40 take 340 + 515 us,
+// of which reading the scores alone is 160; in one kernel, 1.2 ms, the full tests'
+// registers halved the warps of the first look, and a third of the lanes ran most
+// of the instructions.  (One CTA a frame, slice after slice: 6.4 ms.)
 //
 // Scores of the FFT correlation are within eps (DetEps) of the direct sum's.  A
 // decision that eps could turn marks the frame in inexact[]; marked frames are taken again with directly summed
 // scores (again = 1, eps = 0).  inexact = nullptr: every score is the direct sum's.
 // bits: a bit per (slice, j, i), 32 values of i to a word; tot: peaks per slice.
+
+// First look, a warp a row: sets the bits of the pixels above the threshold that no
+// score within three pixels of the row or the column exceeds, with room for both
+// bounds and for the row's single precision.  56 pixels at a time, two a lane: one
+// in 20 passes the row's test, and 32 of those at a time read their column.
+__global__ void __launch_bounds__(256) k_det_look(DetView V, const double* score, const int* inexact, int again,
+                                                  unsigned* bits) {
+    const int f = blockIdx.z, r = blockIdx.y, SX = V.SX, SY = V.SY, dec = 3, lo = max(dec, V.R / 2);
+    const int i = lo + blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const bool approx = inexact && !again;
+    if (inexact && again && !inexact[f]) return;
+    if (i >= SX - lo) return;
+    const double* row = score + (((size_t)f * V.Z + r) * SX + i) * SY;
+    const int WX = (SX + 31) / 32, jend = SY - lo;
+    unsigned* out = bits + ((size_t)f * V.Z + r) * SY * WX + (i >> 5);
+    constexpr double SLACK = 3e-4;  // more than two eps (DET_EPS_MAX) and the rounding
+    __shared__ short keep[8][96];
+    short* mine = keep[threadIdx.x >> 5];
+    int n = 0;
+    auto column = [&]() {  // the first min(n, 32) pixels of the list
+        const int j = mine[lane];
+        double c[2 * dec + 1];
+#pragma unroll
+        for (int k = 0; k <= 2 * dec; ++k) c[k] = lane < n ? row[(ptrdiff_t)(k - dec) * SY + j] : 0.0;
+        bool stay = lane < n;
+#pragma unroll
+        for (int k = 0; k <= 2 * dec; ++k) {
+            const int ic = i + k - dec;
+            if (k != dec && ic >= lo && ic < SX - lo && c[k] > 0 && c[k] > c[dec] + SLACK) stay = false;
+        }
+        if (stay) atomicOr(out + (size_t)j * WX, 1u << (i & 31));
+        const int rest = max(n - 32, 0);
+        short t[2];
+        for (int k = 0; k < 2; ++k) t[k] = mine[min(32 + 32 * k + lane, 95)];
+        __syncwarp();
+        for (int k = 0; k < 2; ++k) mine[32 * k + lane] = t[k];
+        n = rest;
+        __syncwarp();
+    };
+    const float thr = approx ? (float)(V.thr - SLACK) : __double2float_rd(V.thr);
+    auto load = [&](int j) { return j >= lo - dec && j < jend + dec ? (float)row[j] : -INFINITY; };
+    float an = load(lo - 4 + 2 * lane), bn = load(lo - 3 + 2 * lane);
+    for (int j0 = lo; j0 < jend; j0 += 56) {
+        const int j = j0 - 4 + 2 * lane;
+        const float a = an, b = bn, m = fmaxf(a, b);
+        an = load(j + 56);
+        bn = load(j + 57);
+        const unsigned all = 0xffffffffu;
+        const float ml = __shfl_up_sync(all, m, 1), mr = __shfl_down_sync(all, m, 1);
+        const float bl = __shfl_up_sync(all, b, 2), ar = __shfl_down_sync(all, a, 2);
+        const float side = fmaxf(ml, mr), na = fmaxf(side, fmaxf(bl, b)), nb = fmaxf(side, fmaxf(ar, a));
+        const bool mid = lane >= 2 && lane < 30;
+        auto passes = [&](float v, float w, int jj) {
+            const bool beaten = w > v + (float)SLACK + 1e-6f * fabsf(v) && (approx || v > 0);
+            return mid && jj < jend && (approx ? v > thr : v >= thr) && !beaten;
+        };
+        const bool pa = passes(a, na, j), pb = passes(b, nb, j + 1);
+        const unsigned ba = __ballot_sync(all, pa), bb = __ballot_sync(all, pb), below = (1u << lane) - 1;
+        if (pa) mine[n + __popc(ba & below)] = (short)j;
+        n += __popc(ba);
+        if (pb) mine[n + __popc(bb & below)] = (short)(j + 1);
+        n += __popc(bb);
+        __syncwarp();
+        while (n >= 32) column();
+    }
+    if (n > 0) column();
+}
+
+// The full tests of the pixels that k_det_look left, a word of bits a lane.
 __global__ void __launch_bounds__(256) k_det_peaks(DetView V, const double* score, DetEps E, int* inexact, int again,
                                                    unsigned* bits, int* tot) {
     const int f = blockIdx.z, r = blockIdx.y, SX = V.SX, SY = V.SY, Z = V.Z, dec = 3, lo = max(dec, V.R / 2);
-    const int i = lo + blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int WX = (SX + 31) / 32, word = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
     const size_t SS = (size_t)SX * SY;
     const bool approx = inexact && !again;
     if (inexact && again && !inexact[f]) return;
+    unsigned* at_word = bits + ((size_t)f * Z + r) * SY * WX + word;
+    const unsigned seen = word < SY * WX ? *at_word : 0;
+    if (!__any_sync(0xffffffffu, seen != 0)) return;
     const double kf = approx ? E.k * __longlong_as_double((long long)E.amax[f]) : 0.0;
-    if (i >= SX - lo) return;
     const double* sc = score + (size_t)f * Z * SS;
-    const double* row = sc + (size_t)r * SS + (size_t)i * SY;
     const double* iv = approx ? E.isv + f * SS : nullptr;
     auto eps_at = [&](int ic, int jc) { return approx ? kf * fmax(iv[(size_t)ic * SY + jc], 0.0) + E.base : 0.0; };
-    const int WX = (SX + 31) / 32, jend = SY - lo;
-    int found = 0;
-    auto test = [&](int j) {  // every test of pixel (i, j); only lanes with a pixel come here
-        const double v = row[j], eps = eps_at(i, j);
-        if (!(v + eps > V.thr)) return;
-        bool unsure = !(v - eps > V.thr), peak = true;
+    // The tests of pixel (i, j) against its row and the column's scores, a lane a pixel.
+    auto test = [&](int i, int j, double& v, double& eps, bool& unsure) {
+        const double* row = sc + (size_t)r * SS + (size_t)i * SY;
+        v = row[j];
+        eps = eps_at(i, j);
+        if (!(v + eps > V.thr)) return false;
+        unsure = !(v - eps > V.thr);
+        bool peak = true;
         auto beats = [&](double w, double ew) {  // w against the candidate
             if (w - ew > v + eps) peak = false;
             else if (approx && w + ew >= v - eps) unsure = true;
@@ -445,7 +522,7 @@ __global__ void __launch_bounds__(256) k_det_peaks(DetView V, const double* scor
             const int ic = i + (k < dec ? -1 - k : k - dec + 1);
             if (ic >= lo && ic < SX - lo && cs[k] > ce[k] && cs[k] - ce[k] > v + eps) peak = false;
         }
-        if (!peak) return;
+        if (!peak) return false;
         if (!approx && !(v > 0)) {  // its own tmp is an earlier slice's, or 0
             double t = 0.0;
             for (int q = r - 1; q >= 0; --q) {
@@ -455,75 +532,81 @@ __global__ void __launch_bounds__(256) k_det_peaks(DetView V, const double* scor
                 for (int a = -dec; a <= dec; ++a) t = fmax(s[a], t);
                 break;
             }
-            if (v != t) return;
+            if (v != t) return false;
         }
-        // the tmp of (ic, j) as slice r sees it, against the candidate: zero, or seven scores' maximum
-        for (int k = 0; k < 2 * dec && peak; ++k) {
-            const int ic = i + (k < dec ? -1 - k : k - dec + 1);
-            bool none = true;
-            if (ic >= lo && ic < SX - lo) {
-                for (int q = r; q >= 0 && none; --q) {
-                    const double* s = sc + (size_t)q * SS + (size_t)ic * SY + j;
-                    const double e = eps_at(ic, j);
-                    if (*s > e) {
-                        none = false;
+        return true;
+    };
+    // Candidate (i, j) against the tmp of (ic, j) as slice r sees it, for the six ic: zero,
+    // or seven scores' maximum.  By the whole warp: a lane a slice, since the last slice
+    // with a positive score can be far below r, then a lane a score.  0: not a peak, 1: a
+    // peak, 2: a peak if the scores were exact.
+    auto against_tmp = [&](int i, int j, double v, double eps, bool unsure) {
+        bool beaten = false;
+        auto beats = [&](double w, double ew) {
+            if (w - ew > v + eps) beaten = true;
+            else if (approx && w + ew >= v - eps) unsure = true;
+        };
+        int at[2 * dec];  // that slice, or -1
+        double e[2 * dec];
+        unsigned open = 0;
 #pragma unroll
-                        for (int a = -dec; a <= dec; ++a) beats(s[a], eps_at(ic, j + a));
-                    } else if (approx && *s > -e) {
-                        unsure = true;
-                    }
+        for (int k = 0; k < 2 * dec; ++k) {
+            const int ic = i + (k < dec ? -1 - k : k - dec + 1);
+            at[k] = -1;
+            e[k] = 0.0;
+            if (ic >= lo && ic < SX - lo) {
+                open |= 1u << k;
+                e[k] = eps_at(ic, j);
+            }
+        }
+        for (int q0 = r; q0 >= 0 && open; q0 -= 32) {
+            double x[2 * dec];
+#pragma unroll
+            for (int k = 0; k < 2 * dec; ++k) {
+                const int ic = i + (k < dec ? -1 - k : k - dec + 1);
+                x[k] = (open >> k & 1) && q0 - lane >= 0 ? sc[(size_t)(q0 - lane) * SS + (size_t)ic * SY + j] : -INFINITY;
+            }
+#pragma unroll
+            for (int k = 0; k < 2 * dec; ++k) {
+                const unsigned pos = __ballot_sync(0xffffffffu, x[k] > e[k]);
+                if (approx && (open >> k & 1) && x[k] > -e[k] && (pos & ((2u << lane) - 1)) == 0) unsure = true;
+                if (pos) {
+                    at[k] = q0 - (__ffs(pos) - 1);
+                    open &= ~(1u << k);
                 }
             }
-            if (none) beats(0.0, 0.0);
         }
-        if (!peak) return;
-        if (approx && unsure) {
-            inexact[f] = 1;
-        } else {
-            atomicOr(&bits[(((size_t)f * Z + r) * SY + j) * WX + (i >> 5)], 1u << (i & 31));
-            ++found;
-        }
-    };
-    // First look: a warp takes 26 pixels of the row with three more on either side, and
-    // keeps those above the threshold that no neighbour in the row exceeds, in single
-    // precision with room for both bounds and the rounding.  About 1 in 20 pixels is
-    // left; these are tested 32 at a time.
-    __shared__ short keep[8][64];
-    short* mine = keep[threadIdx.x >> 5];
-    const float thr = approx ? (float)V.thr - 3e-4f : -INFINITY;
-    int n = 0;
-    auto load = [&](int j) { return j < jend + dec ? row[j] : (double)-INFINITY; };  // j >= lo - dec >= 0
-    double vn = load(lo - dec + lane);
-    for (int j0 = lo; j0 < jend; j0 += 26) {
-        const int j = j0 - dec + lane;
-        const double v = vn;
-        vn = load(j + 26);
-        const float vf = (float)v, top = vf + 3e-4f + 1e-6f * fabsf(vf);
-        bool stay = lane >= dec && lane < 32 - dec && j < jend && vf > thr && (approx || v > V.thr);
+        int z = -1, d = 0;
+        for (int p = lane; p < 2 * dec * (2 * dec + 1); p += 32) {
+            const int k = p / (2 * dec + 1), c = k < dec ? -1 - k : k - dec + 1;
 #pragma unroll
-        for (int a = -dec; a <= dec; ++a)
-            if (a != 0) {
-                const float w = __shfl_sync(0xffffffffu, vf, (lane + a) & 31);
-                if (w > top && (approx || v > 0)) stay = false;
-            }
-        const unsigned b = __ballot_sync(0xffffffffu, stay);
-        if (stay) mine[n + __popc(b & ((1u << lane) - 1))] = (short)j;
-        n += __popc(b);
-        __syncwarp();
-        const bool end = j0 + 26 >= jend;
-        if (n >= 32 || end) {
-            if (lane < n) test(mine[lane]);
-            __syncwarp();
-            const int left = max(n - 32, 0);
-            const short t = lane < left ? mine[32 + lane] : 0;
-            __syncwarp();
-            if (lane < left) mine[lane] = t;
-            n = left;
-            __syncwarp();
-            if (end && lane < n) test(mine[lane]);
+            for (int m = 0; m < 2 * dec; ++m)
+                if (m == k) z = at[m];
+            d = p - k * (2 * dec + 1) - dec;
+            if (z >= 0) beats(sc[(size_t)z * SS + (size_t)(i + c) * SY + j + d], eps_at(i + c, j + d));
+            else beats(0.0, 0.0);
+        }
+        if (__any_sync(0xffffffffu, beaten)) return 0;
+        return approx && __any_sync(0xffffffffu, unsure) ? 2 : 1;
+    };
+    unsigned left = seen, peaks = 0;
+    while (__any_sync(0xffffffffu, left != 0)) {
+        const int bit = left ? __ffs(left) - 1 : 0, i = word % WX * 32 + bit, j = word / WX;
+        double v = 0, eps = 0;
+        bool unsure = false;
+        unsigned alive = __ballot_sync(0xffffffffu, left && test(i, j, v, eps, unsure));
+        left &= left - 1;
+        for (; alive; alive &= alive - 1) {
+            const int k = __ffs(alive) - 1;
+            const int is = against_tmp(__shfl_sync(0xffffffffu, i, k), __shfl_sync(0xffffffffu, j, k),
+                                       __shfl_sync(0xffffffffu, v, k), __shfl_sync(0xffffffffu, eps, k),
+                                       __shfl_sync(0xffffffffu, unsure, k));
+            if (is == 1 && lane == k) peaks |= 1u << bit;
+            if (is == 2 && lane == 0) inexact[f] = 1;
         }
     }
-    found = __reduce_add_sync(0xffffffffu, found);
+    if (peaks != seen) *at_word = peaks;
+    const int found = __reduce_add_sync(0xffffffffu, __popc(peaks));
     if (lane == 0 && found) atomicAdd(&tot[(size_t)f * Z + r], found);
 }
 
@@ -1025,18 +1108,23 @@ int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap
             ctx->launches++;
         };
         const int lo = std::max(3, v.R / 2);
-        const dim3 pgrid((unsigned)std::max(1, (v.SX - 2 * lo + 7) / 8), v.Z, nf);
+        auto peaks = [&](int* marks, int again) {
+            const unsigned rows = (unsigned)std::max(1, (v.SX - 2 * lo + 7) / 8);
+            k_det_look<<<dim3(rows, v.Z, nf), 256, 0, st>>>(v, score, marks, again, bits);
+            const unsigned words = (unsigned)v.SY * ((v.SX + 31) / 32);
+            k_det_peaks<<<dim3((words + 255) / 256, v.Z, nf), 256, 0, st>>>(v, score, E, marks, again, bits, tot);
+            ctx->launches += 2;
+        };
         if (fft) {
             det_fft_scores(ctx, v, d->fft, fr, nf, isv, b, score, st);
-            k_det_peaks<<<pgrid, 256, 0, st>>>(v, score, E, inexact, 0, bits, tot);
+            peaks(inexact, 0);
             direct(inexact);  // the frames that the screening could not decide
             k_det_unmark<<<dim3(32, nf), 256, 0, st>>>(v, inexact, bits, tot);
-            k_det_peaks<<<pgrid, 256, 0, st>>>(v, score, E, inexact, 1, bits, tot);
-            ctx->launches += 3;
+            peaks(inexact, 1);
+            ctx->launches++;
         } else {
             direct(nullptr);
-            k_det_peaks<<<pgrid, 256, 0, st>>>(v, score, E, nullptr, 0, bits, tot);
-            ctx->launches++;
+            peaks(nullptr, 0);
         }
         int* cnt = d_counts + f0;
         k_det_emit<<<dim3(v.Z, nf), 128, 0, st>>>(v, score, bits, tot, cand, cnt);
