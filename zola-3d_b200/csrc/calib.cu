@@ -637,55 +637,65 @@ __global__ void k_cal_hess(CalView V, int nzr, int fit_sigma, int npar, const do
     H[(size_t)q * npar + p] = s;
 }
 
-// Damped solve (H + lambda max(diag H, 1e-12)) x = -g by a blocked Cholesky
-// factorisation of the matrix with -g as a last row (whose factor row is the forward
-// substitution), one CTA: 32 columns at a time, the diagonal block by one warp, the
-// panel a row a thread, the trailing matrix in 4 x 4 blocks from panels staged in
-// shared memory.  n = 393: 1.3 ms, a fifth of what the host took to assemble H and solve.  A: (n + 1) x n work space;
-// ok = 0 when the damped matrix is not positive definite.
+// Damped solve (H + lambda max(diag H, 1e-12)) x = -g.  The beads' parameters couple only
+// through the ng shared ones (modes and sigma), so a CTA a bead eliminates its pb
+// parameters (k_cal_bead), one CTA solves for the shared ones (k_cal_shared), and a CTA a
+// bead takes its own from them (k_cal_back).  45 modes and 5 beads of 61 slices, 393
+// parameters: 314 us; one factorisation of the whole matrix by one CTA, which fills the
+// blocks between beads, took 1270.
+//
+// The pieces are blocked Cholesky factorisations by one CTA: 32 columns at a time, the
+// diagonal block by one warp with a row in a lane's registers, the panel a row a thread,
+// the trailing matrix in 4 x 4 blocks from panels staged in shared memory.
 constexpr int CH_B = 32, CH_THREADS = 512, CH_ROWS = 256;
 constexpr int CH_SMEM = (CH_B * (CH_B + 1) + 2 * CH_ROWS * (CH_B + 2)) * 8 + 64;
-__global__ void __launch_bounds__(CH_THREADS) k_cal_solve(const double* H, const double* g, int n, double lambda, double* A,
-                                                          double* x, int* ok) {
-    extern __shared__ __align__(16) double ch_sm[];
-    double* dg = ch_sm;                          // [32][33]: the diagonal block
-    double* pa = dg + CH_B * (CH_B + 1);         // panel rows of the block rows, [row][34]
-    double* pc = pa + CH_ROWS * (CH_B + 2);      // panel rows of the block columns
+
+// Eliminates the first n columns of the lower triangle of A (rows x cols, row stride ld):
+// the factor in their place, the Schur complement in rows and columns n .. .  False when
+// a pivot is not positive.
+__device__ bool chol(double* A, int ld, int n, int rows, int cols, double* ch_sm) {
+    double* dg = ch_sm;                   // [32][33]: the diagonal block
+    double* pa = dg + CH_B * (CH_B + 1);  // panel rows of the block rows, [row][34]
+    double* pc = pa + CH_ROWS * (CH_B + 2);  // panel rows of the block columns
     int* bad = (int*)(pc + CH_ROWS * (CH_B + 2));
     constexpr int PS = CH_B + 2;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rows = n + 1;
-    for (size_t k = tid; k < (size_t)n * n; k += CH_THREADS) {
-        const int i = (int)(k / n), j = (int)(k - (size_t)i * n);
-        const double h = H[k];
-        A[k] = i == j ? h + lambda * fmax(h, 1e-12) : h;
-    }
-    for (int k = tid; k < n; k += CH_THREADS) A[(size_t)n * n + k] = -g[k];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) *bad = 0;
     __syncthreads();
     for (int k0 = 0; k0 < n; k0 += CH_B) {
         const int nb = min(CH_B, n - k0);
-        if (warp == 0) {  // the diagonal block, a row a lane
-            for (int j = 0; j < nb; ++j) dg[lane * (CH_B + 1) + j] = lane < nb ? A[(size_t)(k0 + lane) * n + k0 + j] : 0.0;
-            __syncwarp();
-            for (int j = 0; j < nb; ++j) {
-                double s = dg[lane * (CH_B + 1) + j];
-                for (int k = 0; k < j; ++k) s -= dg[lane * (CH_B + 1) + k] * dg[j * (CH_B + 1) + k];
-                const double piv = __shfl_sync(0xffffffffu, s, j);
-                if (!(piv > 0)) { if (lane == 0) *bad = 1; break; }
-                const double r = sqrt(piv);
-                if (lane >= j) dg[lane * (CH_B + 1) + j] = lane == j ? r : s / r;
-                __syncwarp();
+        if (warp == 0) {
+            double r[CH_B];
+#pragma unroll
+            for (int j = 0; j < CH_B; ++j)
+                r[j] = j < nb && lane < nb && j <= lane ? A[(size_t)(k0 + lane) * ld + k0 + j] : 0.0;
+            bool fine = true;
+#pragma unroll
+            for (int j = 0; j < CH_B; ++j) {
+                if (j >= nb) break;
+                const double piv = __shfl_sync(0xffffffffu, r[j], j);
+                if (!(piv > 0)) { fine = false; break; }
+                const double d = sqrt(piv);
+                r[j] = lane == j ? d : r[j] / d;
+#pragma unroll
+                for (int k = j + 1; k < CH_B; ++k) {
+                    const double c = __shfl_sync(0xffffffffu, r[j], k);
+                    if (lane >= k) r[k] -= r[j] * c;
+                }
             }
+#pragma unroll
+            for (int j = 0; j < CH_B; ++j) dg[lane * (CH_B + 1) + j] = r[j];
+            if (!fine && lane == 0) *bad = 1;
         }
         __syncthreads();
-        if (*bad) break;
+        if (*bad) return false;
         for (int k = tid; k < nb * nb; k += CH_THREADS) {
             const int i = k / nb, j = k - i * nb;
-            if (j <= i) A[(size_t)(k0 + i) * n + k0 + j] = dg[i * (CH_B + 1) + j];
+            if (j <= i) A[(size_t)(k0 + i) * ld + k0 + j] = dg[i * (CH_B + 1) + j];
         }
         for (int i = k0 + nb + tid; i < rows; i += CH_THREADS) {  // the panel below it
             double r[CH_B];
-            double* a = A + (size_t)i * n + k0;
+            double* a = A + (size_t)i * ld + k0;
 #pragma unroll
             for (int j = 0; j < CH_B; ++j) r[j] = j < nb ? a[j] : 0.0;
 #pragma unroll
@@ -699,15 +709,15 @@ __global__ void __launch_bounds__(CH_THREADS) k_cal_solve(const double* H, const
             }
         }
         __syncthreads();
-        // trailing rows i >= k0 + nb, columns k0 + nb <= j <= i (and j < n)
+        // trailing rows i >= k0 + nb, columns k0 + nb <= j <= i (and j < cols)
         for (int i0 = k0 + nb; i0 < rows; i0 += CH_ROWS)
-            for (int j0 = k0 + nb; j0 <= i0 + CH_ROWS - 1 && j0 < n; j0 += CH_ROWS) {
-                const int ni = min(CH_ROWS, rows - i0), nj = min(CH_ROWS, n - j0);
+            for (int j0 = k0 + nb; j0 <= i0 + CH_ROWS - 1 && j0 < cols; j0 += CH_ROWS) {
+                const int ni = min(CH_ROWS, rows - i0), nj = min(CH_ROWS, cols - j0);
                 __syncthreads();
                 for (int k = tid; k < CH_ROWS * CH_B; k += CH_THREADS) {
                     const int i = k / CH_B, j = k % CH_B;
-                    pa[i * PS + j] = i < ni && j < nb ? A[(size_t)(i0 + i) * n + k0 + j] : 0.0;
-                    if (j0 != i0) pc[i * PS + j] = i < nj && j < nb ? A[(size_t)(j0 + i) * n + k0 + j] : 0.0;
+                    pa[i * PS + j] = i < ni && j < nb ? A[(size_t)(i0 + i) * ld + k0 + j] : 0.0;
+                    if (j0 != i0) pc[i * PS + j] = i < nj && j < nb ? A[(size_t)(j0 + i) * ld + k0 + j] : 0.0;
                 }
                 __syncthreads();
                 const double* pj = j0 == i0 ? pa : pc;
@@ -732,39 +742,95 @@ __global__ void __launch_bounds__(CH_THREADS) k_cal_solve(const double* H, const
 #pragma unroll
                     for (int q = 0; q < 16; ++q) {
                         const int ii = i + q / 4, jj = j + q % 4;
-                        if (ii < ni && jj < nj && j0 + jj <= i0 + ii) A[(size_t)(i0 + ii) * n + j0 + jj] -= s[q];
+                        if (ii < ni && jj < nj && j0 + jj <= i0 + ii) A[(size_t)(i0 + ii) * ld + j0 + jj] -= s[q];
                     }
                 }
             }
         __syncthreads();
     }
-    if (*bad) {
-        if (tid == 0) *ok = 0;
-        return;
-    }
-    // back substitution, block by block: x = L^-T y, y = the last row
-    double* y = A + (size_t)n * n;
+    return true;
+}
+
+// x = L^-T y, block by block: L the factor of n columns in A, y is overwritten.
+__device__ void chol_back(const double* A, int ld, int n, double* y, double* x, double* ch_sm) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k1 = n; k1 > 0;) {
         const int k0 = (k1 - 1) / CH_B * CH_B, nb = k1 - k0;
         if (warp == 0) {
             double v = lane < nb ? y[k0 + lane] : 0.0;
             for (int j = nb - 1; j >= 0; --j) {
-                const double xj = __shfl_sync(0xffffffffu, v, j) / A[(size_t)(k0 + j) * n + k0 + j];
+                const double xj = __shfl_sync(0xffffffffu, v, j) / A[(size_t)(k0 + j) * ld + k0 + j];
                 if (lane == j) v = xj;
-                else if (lane < j) v -= A[(size_t)(k0 + j) * n + k0 + lane] * xj;
+                else if (lane < j) v -= A[(size_t)(k0 + j) * ld + k0 + lane] * xj;
             }
-            if (lane < nb) { dg[lane] = v; x[k0 + lane] = v; }
+            if (lane < nb) { ch_sm[lane] = v; x[k0 + lane] = v; }
         }
         __syncthreads();
         for (int i = tid; i < k0; i += CH_THREADS) {
             double v = y[i];
-            for (int j = 0; j < nb; ++j) v -= A[(size_t)(k0 + j) * n + i] * dg[j];
+            for (int j = 0; j < nb; ++j) v -= A[(size_t)(k0 + j) * ld + i] * ch_sm[j];
             y[i] = v;
         }
         __syncthreads();
         k1 = k0;
     }
-    if (tid == 0) *ok = 1;
+}
+
+// Bead blockIdx.x: its block of H, the shared parameters' rows and -g as rows below
+// (M = pb + ng + 1 of stride M), eliminated.  flags[0]: every pivot was positive.
+__global__ void __launch_bounds__(CH_THREADS) k_cal_bead(const double* H, const double* g, int n, int ng, int pb,
+                                                         double lambda, double* A, int* flags) {
+    extern __shared__ __align__(16) double ch_sm[];
+    const int M = pb + ng + 1, o = ng + blockIdx.x * pb;
+    A += (size_t)blockIdx.x * M * M;
+    for (int k = threadIdx.x; k < M * M; k += CH_THREADS) {
+        const int i = k / M, j = k - i * M;
+        if (j > i) continue;
+        double v = 0.0;
+        if (j < pb) v = i < pb ? H[(size_t)(o + i) * n + o + j] : i < M - 1 ? H[(size_t)(i - pb) * n + o + j] : -g[o + j];
+        if (i == j && i < pb) v += lambda * fmax(v, 1e-12);
+        A[k] = v;
+    }
+    __syncthreads();
+    if (!chol(A, M, pb, M, M - 1, ch_sm) && threadIdx.x == 0) atomicAnd(flags, 0);
+}
+
+// The shared parameters: their block of H plus the beads' Schur complements.  S: (ng + 1) x
+// ng work space.
+__global__ void __launch_bounds__(CH_THREADS) k_cal_shared(const double* H, const double* g, int n, int ng, int pb, int nb,
+                                                           double lambda, const double* A, double* S, double* x, int* flags) {
+    extern __shared__ __align__(16) double ch_sm[];
+    if (!*flags) return;
+    const int M = pb + ng + 1;
+    for (int k = threadIdx.x; k < (ng + 1) * ng; k += CH_THREADS) {
+        const int i = k / ng, j = k - i * ng;
+        if (j > i) continue;
+        double v = i < ng ? H[(size_t)i * n + j] : -g[j];
+        if (i == j) v += lambda * fmax(v, 1e-12);
+        for (int b = 0; b < nb; ++b) v += A[(size_t)b * M * M + (size_t)(pb + i) * M + pb + j];
+        S[k] = v;
+    }
+    __syncthreads();
+    if (!chol(S, ng, ng, ng + 1, ng, ch_sm)) {
+        if (threadIdx.x == 0) *flags = 0;
+        return;
+    }
+    chol_back(S, ng, ng, S + (size_t)ng * ng, x, ch_sm);
+}
+
+__global__ void __launch_bounds__(CH_THREADS) k_cal_back(int ng, int pb, double* A, double* x, const int* flags) {
+    extern __shared__ __align__(16) double ch_sm[];
+    if (!*flags) return;
+    const int M = pb + ng + 1;
+    A += (size_t)blockIdx.x * M * M;
+    double* y = A + (size_t)(M - 1) * M;
+    for (int j = threadIdx.x; j < pb; j += CH_THREADS) {
+        double v = y[j];
+        for (int i = 0; i < ng; ++i) v -= A[(size_t)(pb + i) * M + j] * x[i];
+        y[j] = v;
+    }
+    __syncthreads();
+    chol_back(A, M, pb, y, x + ng + blockIdx.x * pb, ch_sm);
 }
 
 }  // namespace zola
@@ -1059,8 +1125,9 @@ int zola_calib_fit(zola_psf* psf, const zola_calib_data* data, double* zernike, 
                          (void**)&d_g, (void**)&run.K.Q, (void**)&run.K.E, (void**)&run.K.T, (void**)&run.K.Ts,
                          (void**)&run.K.S};
     const size_t n2 = (size_t)npar * npar;
+    const size_t bead_rows = (size_t)pb + boff + 1;
     const size_t fb[] = {(nzr + 4) * nbs * RR * 8, nbs * RR * 8, nbs * RR * 8, nbs * ne * 8, n2 * 8,
-                         (n2 + npar) * 8, (2 * (size_t)npar + 1) * 8, nbs * DD * 16, nbs * WW * 16, nbs * RR * 8,
+                         (nb * bead_rows * bead_rows + (size_t)(boff + 1) * boff) * 8, (2 * (size_t)npar + 1) * 8, nbs * DD * 16, nbs * WW * 16, nbs * RR * 8,
                          nbs * RR * 8, nbs * 8};
     if (carve(&ctx->calib_fit_area, &ctx->calib_fit_bytes, fq, fb, 12) != cudaSuccess) {
         ctx->err = "zola_calib_fit: device memory";
@@ -1068,7 +1135,8 @@ int zola_calib_fit(zola_psf* psf, const zola_calib_data* data, double* zernike, 
     }
     const size_t gn_smem = ((size_t)GN_CHUNK * (gn_stride(nl) + 1) + 16 * FL_THREADS / 2) * 8;
     if (cudaFuncSetAttribute(k_cal_gn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gn_smem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cal_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_SMEM) != cudaSuccess) {
+        cudaFuncSetAttribute(k_cal_bead, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_cal_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_SMEM) != cudaSuccess) {
         ctx->err = "zola_calib_fit: shared memory";
         return ZOLA_E_CUDA;
     }
@@ -1119,10 +1187,15 @@ int zola_calib_fit(zola_psf* psf, const zola_calib_data* data, double* zernike, 
     auto solve = [&](const std::vector<double>& grad, double lambda, std::vector<double>& step, bool* ok) -> int {
         cudaStream_t st = ctx->stream;
         int flag = 0;
+        double *x = d_g + npar, *S = d_A + nb * bead_rows * bead_rows;
+        int* flags = (int*)(d_g + 2 * npar);
         cudaError_t e = cudaMemcpyAsync(d_g, grad.data(), (size_t)npar * 8, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0xff, sizeof(int), st);
         if (e == cudaSuccess) {
-            k_cal_solve<<<1, CH_THREADS, CH_SMEM, st>>>(d_H, d_g, npar, lambda, d_A, d_g + npar, (int*)(d_g + 2 * npar));
-            ctx->launches++;
+            k_cal_bead<<<nb, CH_THREADS, CH_SMEM, st>>>(d_H, d_g, npar, boff, pb, lambda, d_A, flags);
+            k_cal_shared<<<1, CH_THREADS, CH_SMEM, st>>>(d_H, d_g, npar, boff, pb, nb, lambda, d_A, S, x, flags);
+            k_cal_back<<<nb, CH_THREADS, CH_B * 8, st>>>(boff, pb, d_A, x, flags);
+            ctx->launches += 3;
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(step.data(), d_g + npar, (size_t)npar * 8, cudaMemcpyDeviceToHost, st);
