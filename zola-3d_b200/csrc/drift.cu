@@ -107,9 +107,14 @@ __device__ __forceinline__ void dit_stages(V (&x)[1 << NS], int lo, const float2
 #pragma unroll
         for (int i = 0; i < (1 << NS); ++i) {
             if (i >> s & 1) continue;
-            float2 w = __ldg(tw + (((i & ((1 << s) - 1)) << S0) + lo) * ts);
-            w.y *= -sign;
-            const float2 a = x[i], c = x[i | 1 << s], t = cmul_f(w, c);
+            const int m = ((i & ((1 << s) - 1)) << S0) + lo;
+            const float2 a = x[i], c = x[i | 1 << s];
+            float2 t = c;
+            if (S0 > 0 || m > 0) {  // (the table's first entry is 1)
+                float2 w = __ldg(tw + m * ts);
+                w.y *= -sign;
+                t = cmul_f(w, c);
+            }
             x[i] = make_float2(a.x + t.x, a.y + t.y);
             x[i | 1 << s] = make_float2(a.x - t.x, a.y - t.y);
         }
@@ -176,27 +181,28 @@ __host__ __device__ inline size_t plane_smem(int P1, int P2) { return (size_t)P1
 
 // x and y transforms of histogram plane blockIdx.x (z = S0 / 2 + blockIdx.x; the others
 // are empty) of bin blockIdx.y of the batch (windows x bins): xy[bin][plane][y][x].
-__global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_xy(DriftDev D, const float* hist, const float2* tw, float2* xy) {
+__global__ void __launch_bounds__(FFT_THREADS, 4) k_drift_fwd_xy(DriftDev D, const float* hist, const float2* tw, float2* xy) {
     extern __shared__ float2 plane[];
-    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1;
+    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1, lx = lg_of(P2);
     const size_t item = (size_t)blockIdx.y * D.S0 + blockIdx.x;
     const float* h = hist + item * S1 * S2;
     for (int e = threadIdx.x; e < P1 * P2; e += FFT_THREADS) {
-        const int y = e / P2, x = e - y * P2, yc = y - S1 / 2, xc = x - S2 / 2;
+        const int y = e >> lx, x = e & (P2 - 1), yc = y - S1 / 2, xc = x - S2 / 2;
         const bool in = yc >= 0 && yc < S1 && xc >= 0 && xc < S2;
         plane[y * RS + x] = make_float2(in ? h[yc * S2 + xc] : 0.f, 0.f);
     }
     __syncthreads();
-    dit(plane, lg_of(P2), S1, [&](int l, int k) { return (S1 / 2 + l) * RS + k; }, tw, -1.f);
+    dit(plane, lx, S1, [&](int l, int k) { return (S1 / 2 + l) * RS + k; }, tw, -1.f);
     dit(plane, lg_of(P1), P2, [&](int l, int k) { return k * RS + l; }, tw, -1.f);
     float2* out = xy + item * P1 * P2;
-    for (int e = threadIdx.x; e < P1 * P2; e += FFT_THREADS) out[e] = plane[e / P2 * RS + e % P2];
+    for (int e = threadIdx.x; e < P1 * P2; e += FFT_THREADS) out[e] = plane[(e >> lx) * RS + (e & (P2 - 1))];
 }
 
 // z transforms, 32 lines a CTA, times the Gaussian: spec[bin][z][y][x].
 constexpr int ZL = 32;
-__global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_z(DriftDev D, const float2* xy, const float2* tw,
-                                                             const float* gauss, float2* spec) {
+template <int LG>
+__global__ void __launch_bounds__(FFT_THREADS, LG == 8 ? 2 : 4) k_drift_fwd_z(DriftDev D, const float2* xy, const float2* tw,
+                                                                const float* gauss, float2* spec) {
     extern __shared__ float2 lines[];
     const int P0 = D.P0, S0 = D.S0, PP = D.P1 * D.P2, q0 = blockIdx.x * ZL, nl = min(ZL, PP - q0);
     const float2* in = xy + (size_t)blockIdx.y * S0 * PP;
@@ -206,7 +212,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_z(DriftDev D, const f
         lines[e] = zc >= 0 && zc < S0 && l < nl ? in[(size_t)zc * PP + q0 + l] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    dit(lines, lg_of(P0), ZL, [&](int l, int k) { return k * ZL + l; }, tw, -1.f);
+    dit_lines<LG>(lines, ZL, [&](int l, int k) { return k * ZL + l; }, tw, -1.f);
     for (int e = threadIdx.x; e < P0 * ZL; e += FFT_THREADS) {
         const int z = e / ZL, l = e % ZL;
         if (l >= nl) continue;
@@ -221,13 +227,14 @@ __global__ void __launch_bounds__(FFT_THREADS) k_drift_fwd_z(DriftDev D, const f
 
 // Plane z = blockIdx.x of F_p1 conj(F_p2) for pair first + blockIdx.y of window blockIdx.z
 // of the batch, its inverse x transforms, its inverse y transforms for the x that the crop
-// keeps, and the cropped plane: xy[window][pair][z][S1][S2].  66 pairs of 64^3 take 77 us
-// and their z pass 33, bound by L2 (64 KB of spectra a plane) and shared memory; product,
-// three axes and crop as five passes over whole cubes took 760.
-__global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_xy(DriftDev D, const float2* spec, const int* p1, const int* p2,
+// keeps, and the cropped plane: xy[window][pair][z][S1][S2].  66 pairs of 64^3 take 62 us
+// and their z pass 19, bound by L2 (64 KB of spectra a plane, 4.5 TB/s) and instructions
+// (78 with divisions for e / P2 and multiplications by twiddles of 1); product, three axes
+// and crop as five passes over whole cubes took 760.
+__global__ void __launch_bounds__(FFT_THREADS, 4) k_drift_inv_xy(DriftDev D, const float2* spec, const int* p1, const int* p2,
                                                               int first, const float2* tw, float2* xy) {
     extern __shared__ float2 plane[];
-    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1, PP = P1 * P2;
+    const int P1 = D.P1, P2 = D.P2, S1 = D.S1, S2 = D.S2, RS = P2 + 1, PP = P1 * P2, lx = lg_of(P2);
     const size_t PV = (size_t)D.P0 * PP;
     spec += (size_t)blockIdx.z * D.bins * PV + (size_t)blockIdx.x * PP;
     const float2* f1 = spec + p1[first + blockIdx.y] * PV;
@@ -235,22 +242,23 @@ __global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_xy(DriftDev D, const 
 #pragma unroll 4
     for (int e = threadIdx.x; e < PP; e += FFT_THREADS) {
         const float2 a = f1[e], b = f2[e];
-        plane[e / P2 * RS + e % P2] = make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)),
+        plane[(e >> lx) * RS + (e & (P2 - 1))] = make_float2(__fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)),
                                                   __fmaf_rn(a.y, b.x, -__fmul_rn(a.x, b.y)));
     }
     __syncthreads();
-    dit(plane, lg_of(P2), P1, [&](int l, int k) { return l * RS + k; }, tw, 1.f);
+    dit(plane, lx, P1, [&](int l, int k) { return l * RS + k; }, tw, 1.f);
     dit(plane, lg_of(P1), S2, [&](int l, int k) { return k * RS + crop_of(l, S2, P2); }, tw, 1.f);
     float2* out = xy + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * D.P0 + blockIdx.x) * S1 * S2;
     for (int e = threadIdx.x; e < S1 * S2; e += FFT_THREADS) {
-        const int b = e / S2, c = e - b * S2;
+        const int b = e >> (lx - 1), c = e & (S2 - 1);  // (P2 = 2 S2)
         out[e] = plane[crop_of(b, S1, P1) * RS + crop_of(c, S2, P2)];
     }
 }
 
 // Inverse z transforms of the cropped planes, 32 lines a CTA; result[pair] += the real
 // part at the z that the crop keeps, window after window of the batch.
-__global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_z(DriftDev D, const float2* xy, int first, int nwin,
+template <int LG>
+__global__ void __launch_bounds__(FFT_THREADS, LG == 8 ? 2 : 4) k_drift_inv_z(DriftDev D, const float2* xy, int first, int nwin,
                                                              const float2* tw, float* result) {
     extern __shared__ float2 lines[];
     const int P0 = D.P0, S0 = D.S0, SS = D.S1 * D.S2, q0 = blockIdx.x * ZL, nl = min(ZL, SS - q0);
@@ -260,12 +268,30 @@ __global__ void __launch_bounds__(FFT_THREADS) k_drift_inv_z(DriftDev D, const f
         for (int e = threadIdx.x; e < P0 * ZL; e += FFT_THREADS)
             lines[e] = e % ZL < nl ? in[(size_t)(e / ZL) * SS + q0 + e % ZL] : make_float2(0.f, 0.f);
         __syncthreads();
-        dit(lines, lg_of(P0), ZL, [&](int l, int k) { return k * ZL + l; }, tw, 1.f);
+        dit_lines<LG>(lines, ZL, [&](int l, int k) { return k * ZL + l; }, tw, 1.f);
         for (int e = threadIdx.x; e < S0 * ZL; e += FFT_THREADS) {
             const int a = e / ZL, l = e % ZL;
             if (l < nl) res[(size_t)a * SS + q0 + l] += lines[crop_of(a, S0, P0) * ZL + l].x;
         }
         __syncthreads();
+    }
+}
+
+// The z kernels of padded length P0 (a power of two up to 256).  A kernel a length: with
+// the lengths switched inside, the compiler kept the twiddles of all eight in registers
+// across k_drift_inv_z's windows (255 registers, one CTA an SM: 68 us a window of 12 bins
+// at 64^3 voxels instead of 19).
+template <class FN>
+static void with_z_kernels(int P0, const FN& fn) {
+    switch (P0) {
+        case 2: fn(k_drift_fwd_z<1>, k_drift_inv_z<1>); break;
+        case 4: fn(k_drift_fwd_z<2>, k_drift_inv_z<2>); break;
+        case 8: fn(k_drift_fwd_z<3>, k_drift_inv_z<3>); break;
+        case 16: fn(k_drift_fwd_z<4>, k_drift_inv_z<4>); break;
+        case 32: fn(k_drift_fwd_z<5>, k_drift_inv_z<5>); break;
+        case 64: fn(k_drift_fwd_z<6>, k_drift_inv_z<6>); break;
+        case 128: fn(k_drift_fwd_z<7>, k_drift_inv_z<7>); break;
+        default: fn(k_drift_fwd_z<8>, k_drift_inv_z<8>); break;
     }
 }
 
@@ -668,11 +694,14 @@ extern "C" int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crl
     k_drift_gauss<<<grid, 256, 0, st>>>(D, sfp[2], sfp[1], sfp[0], d_gauss);
     ctx->launches++;
     const size_t psm = plane_smem(D.P1, D.P2), zsm = (size_t)D.P0 * ZL * sizeof(float2);
+    decltype(&k_drift_fwd_z<1>) fwd_z = nullptr;
+    decltype(&k_drift_inv_z<1>) inv_z = nullptr;
+    with_z_kernels(D.P0, [&](auto f, auto i) { fwd_z = f, inv_z = i; });
     if (planes) {
         ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_fwd_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm), ctx);
         ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_inv_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm), ctx);
-        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_fwd_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
-        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_drift_inv_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(fwd_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
+        ZOLA_CUDA_CHECK(cudaFuncSetAttribute(inv_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm), ctx);
     }
     for (int w0 = 0; w0 < nwin; w0 += WB) {
         const int nw = std::min(WB, nwin - w0);
@@ -681,14 +710,12 @@ extern "C" int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crl
             ZOLA_CUDA_CHECK(cudaMemsetAsync(d_hist, 0, RV * bin * 4 * nw, st), ctx);
             k_drift_hist<<<hgrid, 256, 0, st>>>(D, d_win + w0, d_xyz, d_frame, n, d_hist, nullptr);
             k_drift_fwd_xy<<<dim3(D.S0, bin * nw), FFT_THREADS, psm, st>>>(D, d_hist, d_tw, d_fxy);
-            k_drift_fwd_z<<<dim3((D.P1 * D.P2 + ZL - 1) / ZL, bin * nw), FFT_THREADS, zsm, st>>>(D, d_fxy, d_tw, d_gauss,
-                                                                                               d_spec);
+            fwd_z<<<dim3((D.P1 * D.P2 + ZL - 1) / ZL, bin * nw), FFT_THREADS, zsm, st>>>(D, d_fxy, d_tw, d_gauss, d_spec);
             ctx->launches += 3;
             for (int first = 0; first < tot; first += CH) {
                 const int np = std::min(CH, tot - first);
                 k_drift_inv_xy<<<dim3(D.P0, np, nw), FFT_THREADS, psm, st>>>(D, d_spec, d_p1, d_p2, first, d_tw, d_corr);
-                k_drift_inv_z<<<dim3((D.S1 * D.S2 + ZL - 1) / ZL, np), FFT_THREADS, zsm, st>>>(D, d_corr, first, nw, d_tw,
-                                                                                             d_res);
+                inv_z<<<dim3((D.S1 * D.S2 + ZL - 1) / ZL, np), FFT_THREADS, zsm, st>>>(D, d_corr, first, nw, d_tw, d_res);
                 ctx->launches += 2;
             }
         } else {
