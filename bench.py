@@ -211,8 +211,9 @@ def detect_fit_config(z, ctx, torch, device, nframes, fp64_frames=0, seed=1):
     out["detect_only"] = {"frames": nframes, "frames_per_s": nframes / dt,
                           "fp64_tflops": out["detect_fp64_flops_per_frame"] * nframes / dt / 1e12,
                           "fp64_frac_of_issue": out["detect_fp64_flops_per_frame"] * nframes / dt / fp64_issue,
-                          "note": "host uint16 frames to candidate lists through zola_detect_u16; FP64 issue rate "
-                                  "= 148 SMs x 64 DFMA/clk x 1965 MHz (nominal)"}
+                          "note": "host uint16 frames to candidate lists through zola_detect_u16; flops of direct sums "
+                                  "for every pixel (FFTs screen them with far fewer, so the fraction can "
+                                  "exceed 1); FP64 issue rate = 148 SMs x 64 DFMA/clk x 1965 MHz (nominal)"}
     rows = {}
     for name, prec, nf in (("split", z.ZOLA_PREC_SPLIT, nframes), ("fp64", z.ZOLA_PREC_FP64, fp64_frames)):
         if nf <= 0:
