@@ -50,6 +50,7 @@ struct PipeView {
     const double* vmap;       // SX x SY sCMOS var/gain^2, or nullptr
     float* slot_v;            // slots x R x R sCMOS patches (with vmap)
     unsigned char* mask;      // nframes x SX x SY
+    unsigned* near_mask;      // nframes x SX x ceil(SY / 32): a bit per pixel whose R x R patch has a masked pixel
     const double* cand;       // nframes x cap x 7
     const int* counts;        // nframes
     const double* libpsf;     // Z x R x R (normalised library PSFs)
@@ -118,21 +119,61 @@ __device__ bool pipe_fitted(const PipeView& V, const double* img, int r, int ci,
     return maxp / B > V.max_snr && B > 0;
 }
 
+// near_mask from the mask, 32 rows of a frame a CTA: rows as words of bits, each the OR of
+// its R neighbours along the row, then of R rows.  Most of a list's candidates lie near a
+// mask late in a frame, and k_pipe_wave drops them by one bit (47 us a wave for 96 frames
+// of 256^2 at R = 40); looking through their patches, a warp each, was 540 of its 630 us.
+constexpr int PN_ROWS = 32, PN_THREADS = 256;
+static size_t near_smem(int SY, int R) { return (size_t)2 * (PN_ROWS + R - 1) * ((SY + 31) / 32) * sizeof(unsigned); }
+__global__ void __launch_bounds__(PN_THREADS) k_pipe_near(PipeView V) {
+    extern __shared__ unsigned pn_sm[];
+    const int f = blockIdx.y, SX = V.SX, SY = V.SY, R = V.R, h = R / 2, i0 = blockIdx.x * PN_ROWS;
+    if (V.done[f]) return;
+    const int WY = (SY + 31) / 32, rows = PN_ROWS + R - 1, lane = threadIdx.x & 31;
+    unsigned *raw = pn_sm, *wide = raw + rows * WY;
+    const unsigned char* mk = V.mask + (size_t)f * SX * SY;
+#pragma unroll 4
+    for (int q = threadIdx.x >> 5; q < rows * WY; q += PN_THREADS / 32) {
+        const int i = i0 - h + q / WY, j = q % WY * 32 + lane;
+        const unsigned b = __ballot_sync(0xffffffffu, i >= 0 && i < SX && j < SY && mk[(size_t)i * SY + j] != 0);
+        if (lane == 0) raw[q] = b;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < rows * WY; q += PN_THREADS) {
+        const int w = q % WY;
+        const unsigned* row = raw + q - w;
+        unsigned any = 0;
+        for (int d = -h; d < R - h; ++d) {  // the 32 bits from bit 32 w + d on
+            const int a = w + (d >> 5);
+            const unsigned lo = a >= 0 && a < WY ? row[a] : 0, hi = a + 1 >= 0 && a + 1 < WY ? row[a + 1] : 0;
+            any |= __funnelshift_r(lo, hi, d & 31);
+        }
+        wide[q] = any;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < PN_ROWS * WY; q += PN_THREADS) {
+        if (i0 + q / WY >= SX) continue;
+        unsigned any = 0;
+        for (int d = 0; d < R; ++d) any |= wide[q + d * WY];
+        V.near_mask[((size_t)f * SX + i0) * WY + q] = any;
+    }
+}
+
 // One wave's selection for one frame (one CTA): walking the candidates from the
 // frame's pointer, the first K (in candidate order) that need a fit under the
 // current mask get slots and their ROI (k_pipe_start adds the start).  limit = just
 // past the K-th (or the end).
-// 512 candidates at a time: a thread drops the ones outside the border or with a
-// masked centre, which late in a frame are nearly all; the rest are taken in order,
-// a warp each, until K are found.  (A thread a candidate for everything read its
-// 1,600 pixels one after the other: 2.8 ms a wave at R = 40.)
+// 512 candidates at a time: a thread drops the ones outside the border or with a masked
+// pixel in their patch, which late in a frame are nearly all; the rest are taken in
+// order, a warp each, until K are found: 90 us a wave at R = 40.  (A thread a candidate
+// for everything read its 1,600 pixels one after the other: 2.8 ms.)
 constexpr int PW_THREADS = 512, PW_WARPS = PW_THREADS / 32;
 __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
     const int f = blockIdx.x, SX = V.SX, SY = V.SY, R = V.R, h = R / 2, RR = R * R;
     if (V.done[f]) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double* img = V.fimg + (size_t)f * SX * SY;
-    const unsigned char* mk = V.mask + (size_t)f * SX * SY;
+    const unsigned* near_mask = V.near_mask + (size_t)f * SX * ((SY + 31) / 32);
     const double* cand = V.cand + (size_t)f * V.cap * 7;
     int* code_of = V.cand_slot + (size_t)f * V.cap;
     const int n = min(V.counts[f], V.cap);
@@ -144,7 +185,7 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
         if (i < n) {
             const int ci = (int)llrint(cand[(size_t)i * 7 + 2]), cj = (int)llrint(cand[(size_t)i * 7 + 3]);
             const bool in = pipe_inside(V, ci, cj);
-            look = in && mk[(size_t)ci * SY + cj] == 0;
+            look = in && !(near_mask[(size_t)ci * ((SY + 31) / 32) + (cj >> 5)] >> (cj & 31) & 1u);
             if (!look) code_of[i] = in ? -3 : -2;
         }
         const unsigned bal = __ballot_sync(0xffffffffu, look);
@@ -166,17 +207,7 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
             double maxp = 0;
             int code = -3;
             if (mine) {
-                bool masked = false;
-                for (int q0 = 0; q0 < RR && !masked; q0 += 256) {
-                    bool any = false;
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int q = q0 + 32 * u + lane;
-                        any |= q < RR && mk[corner + (size_t)(q / R) * SY + q % R] != 0;
-                    }
-                    masked = __any_sync(0xffffffffu, any);
-                }
-                if (!masked) code = pipe_fitted(V, img, r, ci, cj, &maxp) ? 0 : -1;
+                code = pipe_fitted(V, img, r, ci, cj, &maxp) ? 0 : -1;
                 if (lane == 0) {
                     code_of[k] = code;
                     V.cand_maxp[(size_t)f * V.cap + k] = maxp;
@@ -530,14 +561,16 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
     const int FB = std::max(1, std::min(nframes, prm->frames_per_batch > 0 ? prm->frames_per_batch : 1024));
     const size_t SS = (size_t)SX * SY, RR = (size_t)R * R;
     cudaStream_t st = ctx->stream;
+    ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_pipe_near, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)near_smem(SY, R)),
+                    ctx);
     const int K = prm->wave_fits > 0 ? prm->wave_fits : PIPE_WAVE_FITS;
     const int slot_cap = FB * K;
     Buf b_img, b_mask, b_cand, b_cnt, b_lib, b_rng, b_cslot, b_cmax, b_ptr, b_lim, b_done, b_ns, b_rois, b_init, b_sf,
         b_sc, b_out5, b_st, b_xyz, b_psi, b_mthr, b_acc, b_seq, b_nacc, b_dpsi, b_rows, b_fimg, b_adu, b_off, b_gain,
-        b_vg, b_sv, b_u16, b_list, b_nlist, b_var;
+        b_vg, b_sv, b_u16, b_list, b_nlist, b_var, b_near;
     cudaError_t e = cudaSuccess;
     auto A = [&](Buf& b, size_t bytes) { if (e == cudaSuccess) e = b.alloc(bytes); };
-    A(b_img, SS * FB * 8); A(b_var, SS * FB * 8); A(b_mask, SS * FB); A(b_cand, (size_t)FB * cap * 7 * 8); A(b_cnt, (size_t)FB * 4);
+    A(b_img, SS * FB * 8); A(b_var, SS * FB * 8); A(b_mask, SS * FB); A(b_near, (size_t)FB * SX * ((SY + 31) / 32) * 4); A(b_cand, (size_t)FB * cap * 7 * 8); A(b_cnt, (size_t)FB * 4);
     A(b_lib, lib.size() * 8); A(b_rng, range.size() * 8); A(b_cslot, (size_t)FB * cap * 4);
     A(b_cmax, (size_t)FB * cap * 8); A(b_ptr, (size_t)FB * 4); A(b_lim, (size_t)FB * 4); A(b_done, (size_t)FB * 4);
     A(b_ns, 64); A(b_nacc, 64);
@@ -565,7 +598,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
     V.SX = SX; V.SY = SY; V.R = R; V.cap = cap;
     V.dx = fit_psf->o.xystep; V.minZ = prm->minZ; V.maxZ = prm->maxZ; V.photon_thr = prm->photon_threshold;
     V.max_snr = prm->max_snr;
-    V.images = (double*)b_img.p; V.mask = (unsigned char*)b_mask.p; V.cand = (double*)b_cand.p;
+    V.images = (double*)b_img.p; V.mask = (unsigned char*)b_mask.p; V.near_mask = (unsigned*)b_near.p; V.cand = (double*)b_cand.p;
     V.fimg = scmos ? (double*)b_fimg.p : (double*)b_img.p;
     V.vmap = scmos ? (double*)b_vg.p : nullptr;
     V.slot_v = scmos ? (float*)b_sv.p : nullptr;
@@ -660,8 +693,9 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
             e = cudaMemsetAsync(b_ns.p, 0, 4, st);
             if (e == cudaSuccess) e = cudaMemsetAsync(b_nacc.p, 0, 4, st);
             if (e != cudaSuccess) return fail(e);
+            k_pipe_near<<<dim3((SX + PN_ROWS - 1) / PN_ROWS, nf), PN_THREADS, near_smem(SY, R), st>>>(V);
             k_pipe_wave<<<nf, PW_THREADS, 0, st>>>(V, K);
-            ctx->launches++;
+            ctx->launches += 2;
             int nslot = 0;
             e = cudaMemcpyAsync(&nslot, b_ns.p, 4, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
