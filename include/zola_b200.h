@@ -250,8 +250,8 @@ typedef struct {
     int cand_cap;             /* candidates stored per frame at the start (0: 8192); it grows to the
                                  longest list so that every frame walks its whole list */
     int frames_per_batch;     /* frames per device batch (0: 1024) */
-    int wave_fits;            /* candidates fitted ahead per frame and wave (0: 8); any value gives the
-                                 same rows as the reference's one-at-a-time walk */
+    int wave_fits;            /* candidates fitted ahead per frame and wave (0: 8, or more in split fits
+                                 of few frames); any value gives the same rows as the reference's one-at-a-time walk */
 } zola_loc_params;
 
 /* frames: nframes x SX x SY photons (double, first index x, already converted
