@@ -2420,6 +2420,20 @@ __host__ __device__ inline int s45s_nbuf(int W, int RP, int R, int UG) {
     return 2 * UG * 4 * RP <= 512 && s45s_smem(W, RP, R, UG, 2, s45s_groups(2)) <= 225 * 1024 ? 2 : 1;
 }
 
+// The pixels (and sCMOS terms) of a unit's ROIs, and A and B, on their way to L1 for
+// unit_sums, whose pixel loop waits for them otherwise.
+template <int NTG>
+__device__ __forceinline__ void prefetch_rois(const SplitDev& P, const FitIO& F, int unit, int tg) {
+    const int UG = unit_slots(P.G1, P.G2), per = NTG / UG, g = tg / per, RR = P.R * P.R, slot = unit * UG + g;
+    const int roi = P.slot_roi[slot];
+    if (roi < 0) return;
+    for (int k = (tg - g * per) * 32; k < RR; k += per * 32) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(F.rois + (size_t)roi * RR + k));
+        if (F.scmos) asm volatile("prefetch.global.L1 [%0];" ::"l"(F.scmos + (size_t)roi * RR + k));
+    }
+    if (tg == g * per) asm volatile("prefetch.global.L1 [%0];" ::"l"(P.lm[slot].trial + 3));
+}
+
 // The epilogue of one group of NTG threads (tg its thread index, bar_id its
 // barrier): the maps of each unit it owns from TMEM to shared memory (pixel
 // column j' = TMEM lane; 4 NTG / 512 maps a thread), then the unit's sums.
@@ -2439,6 +2453,7 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
         const uint32_t par = (uint32_t)((n / NB) & 1);
         ++n;
         if (NG == 2 && b != grp) continue;  // the other group's unit
+        prefetch_rois<NTG>(P, F, unit, tg);  // while the maps are on their way
         umma::mbar_wait(&acc[b], par, P.err);
         umma::fence_after_sync();
 #pragma unroll
