@@ -2443,7 +2443,7 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
                                               double (*nrm)[4], int* badw, uint64_t* acc, uint64_t* tfree) {
     constexpr int NG = SPLIT_THREADS / NTG;  // groups
     const int R = P.R, RP = P.RP, NT = 4 * RP, RR = R * R, UG = unit_slots(P.G1, P.G2), nc = UG * NT;
-    const int jp = tg & 127;
+    const int jp = tg & 127, lg8 = RP == 16 ? 1 : 2;  // (UG RP = 64: 16 or 32 rows a slot)
     int n = 0;
     bool abort = false;
     for (int tag = 0; !abort;) {
@@ -2453,6 +2453,8 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
         const uint32_t par = (uint32_t)((n / NB) & 1);
         ++n;
         if (NG == 2 && b != grp) continue;  // the other group's unit
+        unsigned live = 0;  // the unit's occupied slots
+        for (int g = 0; g < UG; ++g) live |= (P.slot_roi[unit * UG + g] >= 0 ? 1u : 0u) << g;
         prefetch_rois<NTG>(P, F, unit, tg);  // while the maps are on their way
         umma::mbar_wait(&acc[b], par, P.err);
         umma::fence_after_sync();
@@ -2465,7 +2467,7 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
                 uint32_t ad[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const int g = q / (RP / 8), h = (q - g * (RP / 8)) * 8;
+                    const int g = q >> lg8, h = (q & ((1 << lg8) - 1)) * 8;
                     ad[q] = tmem_lane_addr(tbase, b * nc + g * NT + map * RP + h);
                 }
                 float v[8][8];
@@ -2473,8 +2475,8 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
                 if (jp < R)
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        const int g = q / (RP / 8), h = (q - g * (RP / 8)) * 8;
-                        if (P.slot_roi[unit * UG + g] < 0) continue;
+                        const int g = q >> lg8, h = (q & ((1 << lg8) - 1)) * 8;
+                        if (!(live >> g & 1u)) continue;
                         float* dst = Tm + (size_t)(g * 4 + map) * RR;
 #pragma unroll
                         for (int u = 0; u < 8; ++u)
@@ -2482,7 +2484,7 @@ __device__ __forceinline__ void s45s_epilogue(const SplitDev& P, const FitIO& F,
                     }
             } else {
                 for (int g = 0; g < UG; ++g) {
-                    if (P.slot_roi[unit * UG + g] < 0) continue;
+                    if (!(live >> g & 1u)) continue;
                     float* dst = Tm + (size_t)(g * 4 + map) * RR;
                     for (int h = 0; h < RP; h += 16) {  // 16 columns a wait
                         const uint32_t ad[2] = {tmem_lane_addr(tbase, b * nc + g * NT + map * RP + h),
