@@ -894,6 +894,7 @@ struct CalRun {
     std::vector<double> par, res;
     double sigma = -1;
     size_t n_bead() const { return (size_t)V.nb * V.pb; }
+    size_t head() const { return (nz + n_bead() + 1) / 2 * 2; }  // GT and dGT are read as pairs
 };
 
 // Carve the buffers q[k] (bytes[k] each, 256-byte aligned) from a grow-only
@@ -953,7 +954,7 @@ int cal_setup(zola_psf* p, const zola_calib_data* cd, CalRun& run) {
     void** const q[] = {(void**)&run.d_par, (void**)&run.d_res, (void**)&run.d_phase, (void**)&run.d_slice,
                         (void**)&run.d_gphi, (void**)&run.d_gsum, (void**)&run.d_stacks, (void**)&run.d_const,
                         (void**)&run.scratch};
-    const size_t n_par = nz + run.n_bead() + 2 * WR, n_res = 2 + nz + run.n_bead();
+    const size_t n_par = run.head() + 2 * WR, n_res = 2 + nz + run.n_bead();
     const size_t bytes[] = {n_par * 8, n_res * 8, DD * 8, nbs * NOUT * 8, nbs * DD * 8, DD * 8, nbs * RR * 8,
                             (ns + (cd->photons ? nbs : 0)) * 8,
                             std::min<size_t>(CAL_CLUSTERS, nbs * 256) * run.per_cluster};
@@ -969,7 +970,7 @@ int cal_setup(zola_psf* p, const zola_calib_data* cd, CalRun& run) {
     V.dz = run.d_const;
     V.stacks = run.d_stacks;
     V.A0 = cd->photons ? run.d_const + ns : nullptr;
-    V.GT = run.d_par + nz + run.n_bead();
+    V.GT = run.d_par + run.head();
     V.dGT = V.GT + WR;
     return ZOLA_OK;
 }
@@ -979,7 +980,7 @@ int cal_upload(zola_psf* p, CalRun& run, const double* coef, double sigma, const
     zola_ctx* ctx = p->ctx;
     if (!(sigma > 0)) { ctx->err = "calibration: sigma must be positive"; return ZOLA_E_ARG; }
     const int R = run.V.R, W = run.V.W, DD = run.V.D * run.V.D;
-    const size_t head = run.nz + run.n_bead();
+    const size_t head = run.head();
     std::memcpy(run.par.data(), coef, run.nz * 8);
     std::memcpy(run.par.data() + run.nz, bead, run.n_bead() * 8);
     size_t n = head;
