@@ -106,16 +106,19 @@ __device__ inline CalWork cal_carve(char* base, int D, int W, int R) {
 }
 
 // Shared memory: reduction areas, transform buffer, a tile (pupil rows, or W rows of
-// an intensity and R rows of V1 by LINES columns), and the two transposed blur
-// matrices where they fit.
+// an intensity and R rows of V1 by LINES columns), and the transposed blur matrix where
+// it fits; its derivative is read through L1.  With both in shared memory and 128
+// registers two CTAs shared an SM; 85 registers spill next to nothing, and with three
+// the latency-bound kernels take 1.84 and 0.25 ms (k_cal_tangent, k_cal_eval) instead of
+// 2.07 and 0.28.
 constexpr int CAL_RED_BYTES = 2048;
-constexpr size_t CAL_G_SMEM = 64 * 1024;
+constexpr size_t CAL_G_SMEM = 32 * 1024;
 __host__ __device__ inline size_t cal_tile_bytes(int N, int D, int W, int R) {
     const size_t lines = 2048 / N, q = lines * (D | 1) * 16, x = (size_t)(W + R) * lines * 8;
     return cal_al(q > x ? q : x);
 }
 __host__ __device__ inline size_t cal_smem(int N, int D, int W, int R) {
-    const size_t g = (size_t)2 * W * R * 8;
+    const size_t g = (size_t)W * R * 8;
     return CAL_RED_BYTES + FL_SMEM + cal_tile_bytes(N, D, W, R) + (g <= CAL_G_SMEM ? g : 0);
 }
 
@@ -129,11 +132,10 @@ template <int NFFT>
 __device__ __forceinline__ CalSmem cal_begin(const CalView& V, char* smem) {
     CalSmem m{(double*)smem, (double2*)(smem + CAL_RED_BYTES), smem + CAL_RED_BYTES + FL_SMEM, V.GT, V.dGT};
     const int n = V.W * V.R;
-    if ((size_t)2 * n * 8 <= CAL_G_SMEM) {
+    if ((size_t)n * 8 <= CAL_G_SMEM) {
         double* g = (double*)(m.tile + cal_tile_bytes(NFFT, V.D, V.W, V.R));
-        for (int k = threadIdx.x; k < n; k += FL_THREADS) { g[k] = V.GT[k]; g[n + k] = V.dGT[k]; }
+        for (int k = threadIdx.x; k < n; k += FL_THREADS) g[k] = V.GT[k];
         m.GT = g;
-        m.dGT = g + n;
     }
     __syncthreads();
     return m;
@@ -228,11 +230,11 @@ __device__ __forceinline__ void cal_second(const CalView& V, const CalSmem& m, c
 
 // mode 0: NLL (+ model, psi), mode 1: NLL + adjoint.  One cluster per (bead, slice).
 // out_slice: per slice NOUT values; gphi: per slice the phase gradient, [b][a]; K: per
-// slice what the tangents need.  305 slices of 32 px, 45 modes, N = 128: 276 us (mode 1),
-// bound by the latency of its passes and barriers (74 clusters at once); the direct sums
+// slice what the tangents need.  305 slices of 32 px, 45 modes, N = 128: 248 us (mode 1),
+// bound by the latency of its passes and barriers (111 clusters at once); the direct sums
 // with one output a thread, read from the work area, took 993 us.
 template <int NFFT>
-__global__ void __launch_bounds__(FL_THREADS, 2) k_cal_eval(CalView V, const double* phase, const double* bead, int mode,
+__global__ void __launch_bounds__(FL_THREADS, 3) k_cal_eval(CalView V, const double* phase, const double* bead, int mode,
                                                             CalKeep K, char* scratch, size_t per_cluster,
                                                             double* out_slice, double* gphi, double* model,
                                                             double* psi_out) {
@@ -410,10 +412,10 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_cal_eval(CalView V, const dou
 // Tangent maps d mu / d theta_u of every slice: u < nzr Zernike modes 3 .. (Z: basis),
 // then sigma, x, y, z.  Items are (u, slice), a CTA each, from the fields that the
 // evaluation kept.  tan: per (u, bs) R x R.  46 directions x 305 slices of 32 px (N = 128):
-// 2.1 ms, bound by latency as k_cal_eval; repeating the forward model per direction with
+// 1.8 ms, bound by latency as k_cal_eval; repeating the forward model per direction with
 // direct sums took 30.3 ms.
 template <int NFFT>
-__global__ void __launch_bounds__(FL_THREADS, 2) k_cal_tangent(CalView V, CalKeep K, const double* bead, const double* Z,
+__global__ void __launch_bounds__(FL_THREADS, 3) k_cal_tangent(CalView V, CalKeep K, const double* bead, const double* Z,
                                                                int nzr, char* scratch, size_t per_cta, double* tan) {
     extern __shared__ __align__(256) char cal_sm[];
     using F = FftLines<NFFT>;
