@@ -5,9 +5,9 @@
 // bound by the FP64 pipe (256^2 px, R = 40, 40 slices: 8.4 GFLOP, 310 us a frame
 // at 27 TFLOP/s).  On an MX x MY grid with M >= S + R/2 the circular correlation
 // equals it (both halos fall into the same zero padding), and costs about
-// 0.2 GFLOP a frame: 43 us for that frame, 19 in the columns and 23 in the rows,
+// 0.2 GFLOP a frame: 30 us for that frame, 17 in the columns and 13 in the rows,
 // which are bound by the L2 traffic and latency of T, the spectra and the scores
-// (46 and 40 bytes a point; 13% of the FP64 rate).  These scores only screen the candidates: detect.cu takes
+// (46 and 40 bytes a point; 18% of the FP64 rate).  These scores only screen the candidates: detect.cu takes
 // its decisions with the error bound below, and computes the rows it returns by
 // the direct sum.
 //
@@ -38,16 +38,26 @@ namespace zola {
 // A line length M = R0 R1 R2 [R3] and how a CTA runs it, all known at compile
 // time: radices behind a run-time switch put the operands in local memory and
 // cost eight integer instructions to each floating-point one (57 and 69 us for
-// the two inverse passes of two 256^2 frames, against 38 and 46 us).
+// the two inverse passes of two 256^2 frames, against 38 and 46 us at the time).
 template <int R0, int R1, int R2, int R3>
 struct Len {
     static constexpr int M = R0 * R1 * R2 * R3, NP = R3 > 1 ? 4 : 3;
     static constexpr int LEAST = R3 > 1 ? R3 : R2;  // radices come largest first
-    // lines a CTA: the most of 8, 4, 2, 1 that leave room for two or three CTAs of 80 registers a thread
-    static constexpr int LG = M / LEAST * 8 <= 400 ? 3 : (M / LEAST * 4 <= 400 ? 2 : (M / LEAST * 2 <= 512 ? 1 : 0));
-    static constexpr int THREADS = ((M / LEAST << LG) + 31) / 32 * 32;
-    static constexpr int CTAS = 768 / THREADS > 1 ? 768 / THREADS : 1;
-    static constexpr int SMEM = (M << LG) * (int)sizeof(double2);
+};
+
+// A CTA's share: 1 << MOST lines, or fewer so that it has at most 400 threads (512 for
+// two), and as many CTAs an SM as leave 56 registers a thread.  Columns are read and
+// written along the lines and take 8; rows are read along the points, and the fewer
+// lines the longer the runs: 2.  The inverse passes of two 256^2 frames take 33 + 27 us;
+// rows with 4 lines and with 1 take 29 and 35, and with 8 lines and 80 registers, two
+// CTAs an SM, the passes took 38 + 46.
+template <class L, int MOST>
+struct Share : L {
+    static constexpr int T = L::M / L::LEAST;
+    static constexpr int LG = MOST >= 3 && T * 8 <= 400 ? 3 : MOST >= 2 && T * 4 <= 400 ? 2 : MOST >= 1 && T * 2 <= 512 ? 1 : 0;
+    static constexpr int THREADS = ((T << LG) + 31) / 32 * 32;
+    static constexpr int CTAS = 1152 / THREADS > 16 ? 16 : (1152 / THREADS > 1 ? 1152 / THREADS : 1);
+    static constexpr int SMEM = (L::M << LG) * (int)sizeof(double2);
 };
 
 // One pass of the CTA's lines, radix R, NS = product of the earlier radices.
@@ -207,7 +217,6 @@ static bool fft_dim(int n, FftDim* out) {
         using L = Len<a, b, c, d>;                                        \
         if (L::M >= n && (best.M == 0 || L::M < best.M)) {                \
             best.M = L::M;                                                \
-            best.lines = 1 << L::LG;                                      \
         }                                                                 \
     }
     FFT_LENGTHS(X)
@@ -226,22 +235,23 @@ static void with_len(int M, const FN& fn) {
     }
 }
 
-static unsigned fft_tiles(const FftDim& f, int lines) { return (unsigned)((lines + f.lines - 1) / f.lines); }
 
-// Launch kernel<length M>(...) on grid; kernels are templates, so each gets a functor.
-#define FFT_LAUNCHER(name)                                                                                        \
+// Launch kernel<length M>(...) on grid, grid.x = the lines; kernels are templates, so each
+// gets a functor.
+#define FFT_LAUNCHER(name, MOST)                                                                                  \
     template <class... ARGS>                                                                                      \
     static void launch_##name(int M, dim3 grid, cudaStream_t st, ARGS... args) {                                  \
         with_len(M, [&](auto len) {                                                                               \
-            using L = decltype(len);                                                                              \
+            using L = Share<decltype(len), MOST>;                                                                 \
+            grid.x = (grid.x + (1u << L::LG) - 1) >> L::LG;                                                       \
             cudaFuncSetAttribute(k_##name<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);              \
             k_##name<L><<<grid, L::THREADS, L::SMEM, st>>>(args...);                                              \
         });                                                                                                       \
     }
-FFT_LAUNCHER(fft_rows_fwd)
-FFT_LAUNCHER(fft_cols_fwd)
-FFT_LAUNCHER(fft_cols_inv)
-FFT_LAUNCHER(fft_rows_inv)
+FFT_LAUNCHER(fft_rows_fwd, 1)
+FFT_LAUNCHER(fft_cols_fwd, 3)
+FFT_LAUNCHER(fft_cols_inv, 3)
+FFT_LAUNCHER(fft_rows_inv, 1)
 
 void det_fft_free(DetFft& p) {
     if (p.d_tab) cudaFree(p.d_tab);
@@ -270,8 +280,8 @@ void det_fft_build(zola_ctx* ctx, const DetView& v, DetFft& p) {
     }
     if (ok) {
         cudaStream_t st = ctx->stream;
-        launch_fft_rows_fwd(q.y.M, dim3(fft_tiles(q.y, v.R), 1, q.pairs), st, q.twy(), v.psf0, v.R, v.R, 1, v.Z, A);
-        launch_fft_cols_fwd(q.x.M, dim3(fft_tiles(q.x, q.y.M), 1, q.pairs), st, q.twx(), A, v.R, v.R / 2, q.y.M,
+        launch_fft_rows_fwd(q.y.M, dim3((unsigned)(v.R), 1, q.pairs), st, q.twy(), v.psf0, v.R, v.R, 1, v.Z, A);
+        launch_fft_cols_fwd(q.x.M, dim3((unsigned)(q.y.M), 1, q.pairs), st, q.twx(), A, v.R, v.R / 2, q.y.M,
                             1.0 / (double)MM, 1, q.K());
         ctx->launches += 2;
         ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
@@ -303,14 +313,14 @@ void det_fft_scores(zola_ctx* ctx, const DetView& v, const DetFft& p, const doub
     const size_t SS = (size_t)v.SX * v.SY;
     double2* F = (double2*)scratch;                 // spectra of the frames
     double2* T = F + (size_t)MX * MY * nf;          // row transforms, then the inverse column transforms
-    launch_fft_rows_fwd(MY, dim3(fft_tiles(p.y, v.SX), 1, nf), st, p.twy(), frames, v.SX, v.SY, 0, 0, T);
-    launch_fft_cols_fwd(MX, dim3(fft_tiles(p.x, MY), 1, nf), st, p.twx(), T, v.SX, 0, MY, 1.0, 0, F);
+    launch_fft_rows_fwd(MY, dim3((unsigned)(v.SX), 1, nf), st, p.twy(), frames, v.SX, v.SY, 0, 0, T);
+    launch_fft_cols_fwd(MX, dim3((unsigned)(MY), 1, nf), st, p.twx(), T, v.SX, 0, MY, 1.0, 0, F);
     ctx->launches += 2;
     for (int f0 = 0; f0 < nf; f0 += FS) {
         const int n = std::min(FS, nf - f0);
-        launch_fft_cols_inv(MX, dim3(fft_tiles(p.x, MY), p.pairs, n), st, p.twx(), F + (size_t)f0 * MX * MY, p.K(), v.SX,
+        launch_fft_cols_inv(MX, dim3((unsigned)(MY), p.pairs, n), st, p.twx(), F + (size_t)f0 * MX * MY, p.K(), v.SX,
                             MY, T);
-        launch_fft_rows_inv(MY, dim3(fft_tiles(p.y, v.SX), p.pairs, n), st, p.twy(), T, v, isv + f0 * SS,
+        launch_fft_rows_inv(MY, dim3((unsigned)(v.SX), p.pairs, n), st, p.twy(), T, v, isv + f0 * SS,
                             score + (size_t)f0 * v.Z * SS);
         ctx->launches += 2;
     }

@@ -176,13 +176,13 @@ struct DetView {
     const double* norm;  // SX x SY box counts (normImage)
 };
 
-// detect_fft.cu: line transforms of M points, `lines` of them a CTA, and a
+// detect_fft.cu: line transforms of M points, and a
 // detector's twiddles and library spectra.
 constexpr int DET_FFT_MIN_R = 14;  // see det_fft_wanted
 constexpr size_t DET_FFT_MAX_LIBRARY = (size_t)512 << 20;  // bytes of library spectra a detector may hold
 constexpr size_t DET_FFT_T_BYTES = (size_t)56 << 20;       // column transforms in flight (see frames_together)
 struct FftDim {
-    int M = 0, lines = 0;
+    int M = 0;
 };
 struct DetFft {
     FftDim x, y;
