@@ -132,13 +132,10 @@ int zola_ctx_create(int device, zola_ctx** out) {
     // the host-buffer calls and stays non-blocking.
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamDefault) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->feed_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&c->d_counter, 64 * sizeof(int)) != cudaSuccess) {
+        cudaStreamCreateWithFlags(&c->feed_stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete c;
         return ZOLA_E_CUDA;
     }
-    c->d_status_word = c->d_counter + 32;
-    cudaMemset(c->d_counter, 0, 64 * sizeof(int));
     *out = c;
     return ZOLA_OK;
 }
@@ -151,7 +148,6 @@ int zola_ctx_destroy(zola_ctx* ctx) {
     if (ctx->io) cudaFree(ctx->io);
     if (ctx->calib_area) cudaFree(ctx->calib_area);
     if (ctx->calib_fit_area) cudaFree(ctx->calib_fit_area);
-    if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
     if (ctx->h_post) cudaFreeHost(ctx->h_post);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -387,7 +383,7 @@ namespace {
 int fit_dev_impl(zola_ctx* ctx, zola_psf* psf, int R, const float* d_rois, const float* d_scmos,
                  const double* d_init5, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
                  double* d_nll, int* d_status, int* d_iters, void* stream, const zola::RoiFeed* feed = nullptr,
-                 const int* d_avail = nullptr) {
+                 const int* d_avail = nullptr, bool direct = false) {
     if (!ctx || !psf) return ZOLA_E_ARG;
     if (psf->ctx != ctx) return set_err(ctx, ZOLA_E_ARG, "psf belongs to another context");
     if (!check_fit_params(ctx, prm)) return ZOLA_E_ARG;
@@ -404,8 +400,21 @@ int fit_dev_impl(zola_ctx* ctx, zola_psf* psf, int R, const float* d_rois, const
                                 st, feed, d_avail);
     if (feed && feed->n_chunks > 0)  // the FP64 form needs every input before it starts
         ZOLA_CUDA_CHECK(cudaStreamWaitEvent(st, feed->ev[feed->n_chunks - 1], 0), ctx);
-    return launch_fit_f64(ctx, psf, w, d_rois, d_scmos, d_init5, n, prm, d_out5, d_crlb5, d_nll, d_status, d_iters, st);
+    return launch_fit_f64(ctx, psf, w, d_rois, d_scmos, d_init5, n, prm, d_out5, d_crlb5, d_nll, d_status, d_iters, st,
+                          direct);
 }
+
+}  // namespace
+
+namespace zola {
+int fit_frames_dev(zola_ctx* ctx, zola_psf* psf, int R, const float* d_rois, const float* d_scmos, const double* d_init5,
+                   int n, const zola_fit_params* prm, double* d_out5, int* d_status, cudaStream_t st) {
+    return fit_dev_impl(ctx, psf, R, d_rois, d_scmos, d_init5, n, prm, d_out5, nullptr, nullptr, d_status, nullptr, st,
+                        nullptr, nullptr, true);
+}
+}  // namespace zola
+
+namespace {
 
 int mixed_dev_impl(zola_ctx* ctx, const zola_fit_class* classes, int nclass, cudaStream_t st,
                    const zola::RoiFeed* feeds);

@@ -16,6 +16,19 @@
 // The forward field uses the reference's (cos q, sin r) pair (PSFPhase.java:565-569)
 // so evanescent tables built with resetKz are reproduced; derivatives assume
 // q == r, which holds for the fit tables (kz = 0 where evanescent).
+//
+// Two forms of the sums.  FFTs (eval_maps) serve the models and most fits of
+// zola_fit_batch.  Where the last bit matters the partial DFTs are summed directly, every
+// sum in a fixed order (direct_maps): a fit that meets a flat or singular likelihood (z = 0
+// of a PSF that is the same above and below focus, where rounding decides which way it
+// turns) amplifies the 1e-15 between the two forms to nanometres, or to the other side of
+// focus.  So a fit of zola_fit_batch is taken again, from its start, by direct sums when
+// the FFT form does not bring it to convergence in F64_TRIAL evaluations, or meets a point
+// where one of x, y, z has less than F64_WEAK of the largest one's Fisher information (z
+// within 3 nm of such a focus).  The frame pipeline, whose candidates mostly run long, fits
+// by direct sums at once, and its rows take direct models.  Of 250,000 fits of six PSFs, from good, poor and z = 0 starts, the others end
+// within 1.3e-10 of the direct form's in every parameter and bound, after as many
+// evaluations.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,6 +52,13 @@ struct F64Work {
     double* T;   // 4 * R*R: the CTA's rows of map m start at T + m * nt
     int nt;      // pixels of the CTA's rows
 };
+struct DirectWork {
+    double2* Q;  // D*D
+    double2* S;  // 3 * D*W
+    double* I;   // 4 * W*W
+    double* J;   // 4 * R*W
+    double* T;   // 4 * R*R
+};
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -49,6 +69,9 @@ __host__ __device__ inline size_t f64_work_bytes(int D, int W, int R) {
     b += align_up((size_t)4 * R * R * 8, 256);
     return b;
 }
+__host__ __device__ inline size_t direct_work_bytes(int D, int W, int R) {
+    return f64_work_bytes(D, W, R) + align_up((size_t)D * D * 16, 256) + align_up((size_t)4 * W * W * 8, 256);
+}
 
 __device__ inline F64Work f64_carve(char* base, int D, int W, int R) {
     F64Work w{};
@@ -57,6 +80,11 @@ __device__ inline F64Work f64_carve(char* base, int D, int W, int R) {
     w.J = (double*)(base + o);  o += align_up((size_t)4 * R * W * 8, 256);
     w.T = (double*)(base + o);
     return w;
+}
+__device__ inline DirectWork direct_carve(char* base, int D, int W, int R) {
+    const F64Work f = f64_carve(base, D, W, R);
+    base += f64_work_bytes(D, W, R);
+    return DirectWork{(double2*)base, f.S, (double*)(base + align_up((size_t)D * D * 16, 256)), f.J, f.T};
 }
 
 // Shared memory: reduction areas, transform buffer, one tile of the
@@ -278,6 +306,322 @@ __global__ void __launch_bounds__(F64_THREADS, 2) model_f64_kernel(PsfView P, Wi
     cl.sync();  // no CTA leaves while another may read its shared memory
 }
 
+// ------------------------------------------------------------------------
+// The direct form: partial DFT sums in the order of their terms, so that a result never
+// depends on how the work is shared.  The threads of a cluster share every pass.
+constexpr int DIRECT_THREADS = 512;
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 cmadd(double2 acc, double2 a, double2 b) {
+    acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+    acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+    return acc;
+}
+
+// The four blurred maps as eval_maps, into w.T (map m from m R R on); every thread of the
+// cluster.  Bound by the latency of its operands in L2 and by the barriers: 60 us an
+// evaluation at N = 128, W = 64 by eight CTAs.  Two outputs a thread: one takes 5.6
+// instead of 6.0 ms for 800 fits of 24 px, of which a few go on by direct sums, but twice
+// as long where the fits fill the chip; with four it is 7.3 ms.  Tiles of columns kept in
+// shared memory by a CTA take 5.4 ms, and a quarter more for a movie.
+__device__ void direct_maps(const Cluster& cl, const PsfView& P, const WinView& Wn, const DirectWork& w, double x,
+                            double y, double zoil, double zwat, bool derivs) {
+    const int D = P.D, W = Wn.W, R = Wn.R, t0 = cl.rank * DIRECT_THREADS + threadIdx.x, nt = cl.size * DIRECT_THREADS;
+    for (int idx = t0; idx < D * D; idx += nt) {
+        const int a = idx / D, b = idx - a * D;
+        const double pup = P.pupil[idx];
+        double2 q2 = make_double2(0.0, 0.0);
+        if (pup != 0.0) {
+            const double pp = P.kx[a] * x + P.ky[b] * y + P.phase[idx];
+            const double q = pp + P.kz[idx] * zwat - P.kzoil[idx] * zoil;
+            const double r = pp + P.kz[idx] * zwat * P.isim[idx] - P.kzoil[idx] * zoil * P.isimoil[idx];
+            q2 = make_double2(pup * cos(q), pup * sin(r));
+        }
+        w.Q[idx] = q2;
+    }
+    cl.sync();
+    // first contraction over pupil columns b: rows a0 and a0 + 1 of one column j
+    constexpr int TA = 2;
+    double2 *S = w.S, *Sy = S + (size_t)D * W, *Sz = Sy + (size_t)D * W;
+    for (int idx = t0; idx < (D + TA - 1) / TA * W; idx += nt) {
+        const int a0 = idx / W * TA, j = idx % W;
+        double2 s[TA], sy[TA], sz[TA];
+        const double2* q_[TA];
+        const double* kz_[TA];
+#pragma unroll
+        for (int t = 0; t < TA; ++t) {
+            s[t] = sy[t] = sz[t] = make_double2(0, 0);
+            q_[t] = w.Q + (size_t)min(a0 + t, D - 1) * D;
+            kz_[t] = P.kz + (size_t)min(a0 + t, D - 1) * D;
+        }
+        const double2* crow = Wn.C + (size_t)j * D;
+#pragma unroll 4
+        for (int b = 0; b < D; ++b) {
+            const double2 c = crow[b];
+            const double ky = P.ky[b];
+#pragma unroll
+            for (int t = 0; t < TA; ++t) {
+                const double2 qc = cmul(q_[t][b], c);
+                s[t].x += qc.x; s[t].y += qc.y;
+                if (derivs) {
+                    const double kz = kz_[t][b];
+                    sy[t].x -= ky * qc.y; sy[t].y += ky * qc.x;   // (i ky) q c
+                    sz[t].x -= kz * qc.y; sz[t].y += kz * qc.x;   // (i kz) q c
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < TA; ++t) {
+            if (a0 + t >= D) break;
+            const size_t o = (size_t)(a0 + t) * W + j;
+            S[o] = s[t];
+            if (derivs) { Sy[o] = sy[t]; Sz[o] = sz[t]; }
+        }
+    }
+    cl.sync();
+    // second contraction over pupil rows a, then intensities: rows i0 and i0 + 1 of one column j
+    double *I0 = w.I, *I1 = I0 + (size_t)W * W, *I2 = I1 + (size_t)W * W, *I3 = I2 + (size_t)W * W;
+    for (int idx = t0; idx < W / TA * W; idx += nt) {
+        const int i0 = idx / W * TA, j = idx % W;
+        double2 e[TA], ex[TA], ey[TA], ez[TA];
+#pragma unroll
+        for (int t = 0; t < TA; ++t) e[t] = ex[t] = ey[t] = ez[t] = make_double2(0, 0);
+        const double2* c_ = Wn.C + (size_t)i0 * D;
+#pragma unroll 4
+        for (int a = 0; a < D; ++a) {
+            const double2 s = S[(size_t)a * W + j];
+            double2 sy = make_double2(0, 0), sz = make_double2(0, 0);
+            double kx = 0;
+            if (derivs) { sy = Sy[(size_t)a * W + j]; sz = Sz[(size_t)a * W + j]; kx = P.kx[a]; }
+#pragma unroll
+            for (int t = 0; t < TA; ++t) {
+                const double2 c = c_[(size_t)t * D + a];
+                const double2 cs = cmul(c, s);
+                e[t].x += cs.x; e[t].y += cs.y;
+                if (derivs) {
+                    ex[t].x -= kx * cs.y; ex[t].y += kx * cs.x;
+                    ey[t] = cmadd(ey[t], c, sy);
+                    ez[t] = cmadd(ez[t], c, sz);
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < TA; ++t) {
+            const size_t o = (size_t)(i0 + t) * W + j;
+            I0[o] = e[t].x * e[t].x + e[t].y * e[t].y;
+            if (derivs) {
+                I1[o] = 2.0 * (e[t].x * ex[t].x + e[t].y * ex[t].y);
+                I2[o] = 2.0 * (e[t].x * ey[t].x + e[t].y * ey[t].y);
+                I3[o] = 2.0 * (e[t].x * ez[t].x + e[t].y * ez[t].y);
+            }
+        }
+    }
+    cl.sync();
+    // blur along the first index (two rows i' of one column j), then along the second
+    const int nm = derivs ? 4 : 1, hp = R / 2;
+    for (int idx = t0; idx < nm * hp * W; idx += nt) {
+        const int m = idx / (hp * W), rem = idx - m * hp * W, ip = rem / W * 2, j = rem % W;
+        const double *Im = w.I + (size_t)m * W * W + j, *g = Wn.G + (size_t)ip * W;
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll 8
+        for (int i = 0; i < W; ++i) {
+            const double v = Im[(size_t)i * W];
+            s0 = fma(g[i], v, s0);
+            s1 = fma(g[W + i], v, s1);
+        }
+        w.J[((size_t)m * R + ip) * W + j] = s0;
+        w.J[((size_t)m * R + ip + 1) * W + j] = s1;
+    }
+    cl.sync();
+    for (int idx = t0; idx < nm * R * R; idx += nt) {
+        const int row = idx / R, jp = idx - row * R;
+        const double *g = Wn.GT + jp, *Jm = w.J + (size_t)row * W;
+        double s = 0.0;
+#pragma unroll 8
+        for (int j = 0; j < W; ++j) s = fma(g[(size_t)j * R], Jm[j], s);
+        w.T[idx] = s;
+    }
+    cl.sync();
+}
+
+// Sums over n pixels, pixel k to thread k mod 512: pix(k, v) adds a pixel's terms; end(v)
+// closes a thread's sums.  Every CTA forms them for itself.  red: 17 NV doubles.
+template <int NV, class PIX, class END>
+__device__ __forceinline__ void direct_sums(int n, double* red, double (&out)[NV], const PIX& pix, const END& end) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+    for (int k = threadIdx.x; k < n; k += DIRECT_THREADS) pix(k, v);
+    end(v);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        double x = v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) red[warp * NV + k] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double s = 0.0;
+        for (int w = 0; w < DIRECT_THREADS / 32; ++w) s += red[w * NV + threadIdx.x];
+        red[DIRECT_THREADS / 32 * NV + threadIdx.x] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = red[DIRECT_THREADS / 32 * NV + k];
+    __syncthreads();
+}
+
+__device__ __forceinline__ void direct_norm(const double* T, int RR, bool derivs, double* red, double (&s)[4]) {
+    direct_sums<4>(RR, red, s, [&](int k, double (&v)[4]) {
+        double t0 = T[k];
+        double sg = t0 < 0 ? -1.0 : 1.0;
+        v[0] += fabs(t0);
+        if (derivs) {
+            v[1] += sg * T[RR + k];
+            v[2] += sg * T[2 * RR + k];
+            v[3] += sg * T[3 * RR + k];
+        }
+    }, [](double (&)[4]) {});
+}
+
+// CTAs a cluster of the direct form for n items: as the window has work for, and fewer
+// where the items alone fill the chip.
+static int direct_cluster(const zola_ctx* ctx, int W, int n) {
+    int c = W >= 64 ? 8 : (W >= 32 ? 4 : 2);
+    while (c > 1 && (long long)n * c > ctx->num_sms) c /= 2;
+    return c;
+}
+
+// The models of model_f64_kernel (without a list) in the direct form.
+__global__ void __launch_bounds__(DIRECT_THREADS, 1) model_direct_kernel(PsfView P, WinView Wn, const double* xyz, int n,
+                                                                      double* out, double* dout, char* gscratch,
+                                                                      size_t per_cluster) {
+    __shared__ double red[17 * 4];
+    const Cluster cl;
+    const DirectWork w = direct_carve(gscratch + cl.id() * per_cluster, P.D, Wn.W, Wn.R);
+    const int RR = Wn.R * Wn.R;
+    const double* T = w.T;
+    const bool derivs = dout != nullptr;
+    for (int m = cl.id(); m < n; m += cl.count()) {
+        direct_maps(cl, P, Wn, w, xyz[3 * m], xyz[3 * m + 1], P.zfocus, xyz[3 * m + 2], derivs);
+        double s[4];
+        direct_norm(T, RR, derivs, red, s);
+        for (int k = cl.rank * DIRECT_THREADS + threadIdx.x; k < RR; k += cl.size * DIRECT_THREADS) {
+            double t0 = T[k];
+            double sg = t0 < 0 ? -1.0 : 1.0;
+            double psi = fabs(t0) / s[0];
+            out[(size_t)m * RR + k] = psi;
+            if (derivs)
+                for (int d = 0; d < 3; ++d)
+                    dout[((size_t)m * 3 + d) * RR + k] = (sg * T[(d + 1) * RR + k] - psi * s[d + 1]) / s[0];
+        }
+        // (T is written again behind four cluster barriers)
+    }
+}
+
+// The fits of ROIs list[0 .. *n_dev), or of all n without a list, in the direct form.  FP64
+// movies of 13 to 30 frames take 32 (20 frames, 16 px), 88 to 123 (22 to 26 px) and 490 ms
+// (38 px); with fits by FFTs, whose rows are not the same, 24, 46 to 58 and 147, and
+// with direct sums by one CTA a fit 42, 159 to 194 and 888.
+__global__ void __launch_bounds__(DIRECT_THREADS, 1) fit_direct_kernel(PsfView P, WinView Wn, const float* rois,
+                                                                    const float* scmos, const double* init, int n,
+                                                                    const int* list, const int* n_dev, FitParamsDev prm,
+                                                                    double* out5, double* crlb5, double* nll_out,
+                                                                    int* st_out, int* it_out, char* gscratch,
+                                                                    size_t per_cluster, int* counter, int least,
+                                                                    int most) {
+    __shared__ double red[17 * F64_NRED];
+    __shared__ LMState st;  // every CTA of the cluster steps its own copy, from the same sums
+    __shared__ int item, go;
+    const Cluster cl;
+    const DirectWork w = direct_carve(gscratch + cl.id() * per_cluster, P.D, Wn.W, Wn.R);
+    const int RR = Wn.R * Wn.R, items = list ? min(n, *n_dev) : n;
+    const double* T = w.T;
+    if (items < least || items > most) return;  // (a launch with clusters of another size takes them)
+    for (;;) {
+        if (cl.rank == 0 && threadIdx.x == 0) item = atomicAdd(counter, 1);
+        cl.sync();
+        const int i = cl.size > 1 ? cl.read(&item, 0) : item;
+        if (i >= items) break;
+        const int r = list ? list[i] : i;
+        const float* d = rois + (size_t)r * RR;
+        const float* sv = scmos ? scmos + (size_t)r * RR : nullptr;
+        if (threadIdx.x == 0) {
+            for (int q = 0; q < 5; ++q) st.trial[q] = init[5 * (size_t)r + q];
+            lm_clamp(st.trial, prm);
+            st.status = 0;  // nothing evaluated yet
+        }
+        __syncthreads();
+        do {
+            double th[5], s[4], v[F64_NRED];
+            for (int q = 0; q < 5; ++q) th[q] = st.trial[q];
+            direct_maps(cl, P, Wn, w, th[0], th[1], P.zfocus, th[2], true);
+            direct_norm(T, RR, true, red, s);
+            const double A = th[3], B = th[4];
+            bool bad = false;
+            direct_sums<F64_NRED>(RR, red, v, [&](int k, double (&v)[F64_NRED]) {
+                double t0 = T[k];
+                double sg = t0 < 0 ? -1.0 : 1.0;
+                double psi = fabs(t0) / s[0];
+                double j[5];
+                for (int q = 0; q < 3; ++q) j[q] = A * (sg * T[(q + 1) * RR + k] - psi * s[q + 1]) / s[0];
+                j[3] = psi;
+                j[4] = 1.0;
+                double mu = A * psi + B + (sv ? (double)sv[k] : 0.0);
+                if (!(mu > 0.0)) { bad = true; return; }
+                double dk = (double)d[k];
+                v[0] += dk > 0 ? mu - dk - dk * log(mu / dk) : mu;
+                double wg = 1.0 - dk / mu, wh = dk / (mu * mu), wf = 1.0 / mu;
+                int o = 1;
+#pragma unroll
+                for (int q = 0; q < 5; ++q) v[o + q] += wg * j[q];
+                o = 6;
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+#pragma unroll
+                    for (int r = 0; r <= q; ++r) {
+                        v[o] += wh * j[q] * j[r];
+                        v[o + 15] += wf * j[q] * j[r];
+                        ++o;
+                    }
+            }, [&](double (&v)[F64_NRED]) {
+                if (bad) v[0] = INFINITY;
+                bad = false;
+            });
+            if (threadIdx.x == 0) {
+                double H[25], F[25];
+                int o = 6;
+                for (int q = 0; q < 5; ++q)
+                    for (int r = 0; r <= q; ++r) {
+                        H[q * 5 + r] = H[r * 5 + q] = v[o];
+                        F[q * 5 + r] = F[r * 5 + q] = v[o + 15];
+                        ++o;
+                    }
+                if (st.status == 0) {
+                    for (int q = 0; q < 5; ++q) st.th[q] = th[q];
+                    lm_start(st, v[0], v + 1, H, F, prm);
+                } else {
+                    lm_update(st, v[0], v + 1, H, F, prm);
+                }
+                go = lm_propose(st, prm) ? 1 : 0;
+            }
+            __syncthreads();
+        } while (go);
+        if (cl.rank == 0 && threadIdx.x == 0) {
+            for (int q = 0; q < 5; ++q) out5[5 * (size_t)r + q] = st.th[q];
+            if (nll_out) nll_out[r] = st.nll;
+            if (st_out) st_out[r] = st.status;
+            if (it_out) it_out[r] = st.evals;
+            if (crlb5) lm_crlb(st.F, crlb5 + 5 * (size_t)r);
+        }
+        cl.sync();  // item is written again
+    }
+    cl.sync();  // no CTA leaves while another may read its shared memory
+}
+
 // Likelihood, gradient, Gauss-Newton Hessian and Fisher matrix at theta.
 // sv (nullable): the ROI's sCMOS term var/gain^2, added to the mean
 // (process/cpu/Localization.java:1132).
@@ -333,12 +677,20 @@ __device__ void eval_lik_f64(const Cluster& cl, const PsfView& P, const WinView&
         }
 }
 
+// The trial of every fit; those that go on by direct sums (see above) are listed for
+// fit_direct_kernel.  12 evaluations: one to three fits in a hundred go on, and the longer
+// the trial, the further the others' rounding travels.  1e-4: with 1e-6 the fits that do
+// not go on end up to 7e-11 from the direct form's, with 1e-4 3e-12; 1e-2 takes three times
+// as many fits of a saddle-point PSF along.
+constexpr int F64_TRIAL = 12;
+constexpr double F64_WEAK = 1e-4;
 template <int NFFT>
 __global__ void __launch_bounds__(F64_THREADS, 2) fit_f64_kernel(PsfView P, WinView Wn, const float* rois,
                                                                  const float* scmos, const double* init, int n,
                                                                  FitParamsDev prm, double* out5, double* crlb5,
                                                                  double* nll_out, int* st_out, int* it_out,
-                                                                 char* gscratch, size_t per_cluster, int* counter) {
+                                                                 char* gscratch, size_t per_cluster, int* counter,
+                                                                 int* list, int* listed) {
     extern __shared__ __align__(256) char smem_raw[];
     double* red = (double*)smem_raw;  // reduction area
     __shared__ LMState st;            // every CTA of the cluster steps its own copy, from the same sums
@@ -372,35 +724,41 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fit_f64_kernel(PsfView P, WinV
                     lm_update(st, nll, g, H, F, prm);
                 }
                 go = lm_propose(st, prm) ? 1 : 0;
+                if (fmin(F[0], fmin(F[6], F[12])) < F64_WEAK * fmax(F[0], fmax(F[6], F[12]))) {
+                    st.status = ZOLA_FIT_MAXITER;
+                    go = 0;
+                }
             }
             __syncthreads();
         } while (go);
         if (cl.rank == 0 && threadIdx.x == 0) {
-            for (int q = 0; q < 5; ++q) out5[5 * r + q] = st.th[q];
-            if (nll_out) nll_out[r] = st.nll;
-            if (st_out) st_out[r] = st.status;
-            if (it_out) it_out[r] = st.evals;
-            if (crlb5) lm_crlb(st.F, crlb5 + 5 * r);
+            if (st.status != ZOLA_FIT_CONVERGED) {
+                list[atomicAdd(listed, 1)] = r;
+            } else {
+                for (int q = 0; q < 5; ++q) out5[5 * r + q] = st.th[q];
+                if (nll_out) nll_out[r] = st.nll;
+                if (st_out) st_out[r] = st.status;
+                if (it_out) it_out[r] = st.evals;
+                if (crlb5) lm_crlb(st.F, crlb5 + 5 * r);
+            }
         }
         cl.sync();  // roi is written again
     }
     cl.sync();  // no CTA leaves while another may read its shared memory
 }
 
-// Launch configuration for n ROIs or models: as many clusters as run at once (at
-// most `most`).  attr and cfg live as long as the launch.
+// Launch configuration for n ROIs or models in clusters of C CTAs: as many clusters as run
+// at once (at most `most`).  attr and cfg live as long as the launch.
 template <class K>
-static cudaError_t f64_config(K kernel, const zola_psf* p, const WindowTables* w, int n, long long most, cudaStream_t st,
+static cudaError_t f64_config(K kernel, int C, int threads, size_t smem, int n, long long most, cudaStream_t st,
                               cudaLaunchAttribute* attr, cudaLaunchConfig_t* cfg, int* clusters) {
-    const int C = f64_cluster(p->N, w->W);
-    const size_t smem = f64_smem(p->N, p->D, w->W, w->R);
     *cfg = cudaLaunchConfig_t();
     attr->id = cudaLaunchAttributeClusterDimension;
     attr->val.clusterDim.x = C;
     attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
     cfg->attrs = attr;
     cfg->numAttrs = 1;
-    cfg->blockDim = dim3(F64_THREADS);
+    cfg->blockDim = dim3(threads);
     cfg->gridDim = dim3(C);
     cfg->dynamicSmemBytes = smem;
     cfg->stream = st;
@@ -423,7 +781,8 @@ int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* 
         cudaLaunchAttribute attr;
         cudaLaunchConfig_t cfg;
         int clusters = 0;
-        cudaError_t e = f64_config(kernel, p, w, n, n, st, &attr, &cfg, &clusters);
+        cudaError_t e = f64_config(kernel, f64_cluster(p->N, w->W), F64_THREADS, f64_smem(p->N, p->D, w->W, w->R), n, n, st, &attr,
+                                   &cfg, &clusters);
         if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) { rc = ZOLA_E_CUDA; return; }
         prof_begin(ctx, 6, st);
         if (e == cudaSuccess)
@@ -438,31 +797,129 @@ int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* 
     return ZOLA_OK;
 }
 
-int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_rois, const float* d_scmos,
-                   const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
-                   double* d_nll, int* d_status, int* d_iters, cudaStream_t st) {
+int launch_model_direct(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n, double* d_out,
+                        double* d_dout, cudaStream_t st) {
     if (n <= 0) return ZOLA_OK;
-    const size_t per_cluster = f64_work_bytes(p->D, w->W, w->R);
-    FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
+    const size_t per_cluster = direct_work_bytes(p->D, w->W, w->R);
     WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
-    ZOLA_CUDA_CHECK(cudaMemsetAsync(ctx->d_counter, 0, sizeof(int), st), ctx);
-    int rc = ZOLA_OK;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg;
+    int clusters = 0;
+    cudaError_t e = f64_config(model_direct_kernel, direct_cluster(ctx, w->W, n), DIRECT_THREADS, 0, n, n, st, &attr, &cfg, &clusters);
+    if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) return ZOLA_E_CUDA;
+    prof_begin(ctx, 6, st);
+    if (e == cudaSuccess)
+        e = cudaLaunchKernelEx(&cfg, model_direct_kernel, p->view, wv, d_xyz, n, d_out, d_dout, (char*)ctx->scratch,
+                               per_cluster);
+    prof_end(ctx, st);
+    if (e != cudaSuccess) { ctx->err = std::string("model: ") + cudaGetErrorString(e); return ZOLA_E_CUDA; }
+    ctx->launches++;
+    return ZOLA_OK;
+}
+
+// The kernels of an FP64 fit with their work in area(bytes): counters, the list of fits that
+// go on by direct sums, and the clusters' work areas.  room (0: whatever is asked for) bounds
+// it: fewer clusters and a shorter list then, and the ROIs in as many pieces as the list
+// needs.  direct: no trial by FFTs.
+struct F64Fit {
+    const float *rois, *scmos;
+    const double* init;
+    int n;
+    double *out5, *crlb5, *nll;
+    int *status, *iters;
+};
+template <class AREA>
+static cudaError_t fit_f64_launch(zola_ctx* ctx, const zola_psf* p, const WindowTables* w, const F64Fit& F,
+                                  FitParamsDev fp, bool direct, size_t room, cudaStream_t st, const AREA& area) {
+    const size_t per_fft = f64_work_bytes(p->D, w->W, w->R), per_direct = direct_work_bytes(p->D, w->W, w->R);
+    constexpr size_t HEAD = 256;
+    constexpr int PIECE = 1 << 20;
+    const WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
+    cudaError_t e = cudaSuccess;
+    int piece = direct ? F.n : std::min(F.n, PIECE);
+    if (!direct && room) {  // what one work area leaves; too little for a list: direct sums
+        const size_t left = (room - HEAD - per_direct) / 256 * 256 / sizeof(int);
+        if (left < 4096) direct = true;
+        else piece = (int)std::min<size_t>(piece, left);
+        if (direct) piece = F.n;
+    }
+    const size_t list_b = direct ? 0 : align_up((size_t)piece * sizeof(int), 256);
+    const size_t most = room ? room - HEAD - list_b : 0;
+    // The direct form: with n known, the clusters that suit it; for a list, a launch each with
+    // large, small and single-CTA clusters, of which the list's length picks one (3,000 fits of
+    // 16 px that all go on: 90 ms by clusters of four, 21 by single CTAs).
+    struct { int ctas, least, most, clusters; cudaLaunchAttribute attr; cudaLaunchConfig_t cfg; } D[3];
+    int nd = 0, cd = 0;
+    if (direct) {
+        D[nd++] = {direct_cluster(ctx, w->W, piece), 0, piece};
+    } else {
+        const int big = direct_cluster(ctx, w->W, 1), to[3] = {ctx->num_sms / 4, ctx->num_sms, piece};
+        for (int c = big, k = 0, from = 1; k < 3; from = to[k] + 1, ++k) {
+            D[nd++] = {c, from, to[k]};
+            c = k == 0 ? std::min(c, 2) : 1;
+        }
+    }
+    cudaLaunchAttribute attr_f;
+    cudaLaunchConfig_t cfg_f;
+    int cf = 0;
+    for (int k = 0; k < nd && e == cudaSuccess; ++k) {
+        e = f64_config(fit_direct_kernel, D[k].ctas, DIRECT_THREADS, 0, std::min(piece, D[k].most),
+                       room ? most / per_direct : piece, st, &D[k].attr, &D[k].cfg, &D[k].clusters);
+        cd = std::max(cd, D[k].clusters);
+    }
+    if (e != cudaSuccess) return e;
     with_fft(p->N, [&](auto nfft) {
         auto kernel = fit_f64_kernel<decltype(nfft)::value>;
-        cudaLaunchAttribute attr;
-        cudaLaunchConfig_t cfg;
-        int clusters = 0;
-        cudaError_t e = f64_config(kernel, p, w, n, n, st, &attr, &cfg, &clusters);
-        if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) { rc = ZOLA_E_CUDA; return; }
-        prof_begin(ctx, 5, st);
-        if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, kernel, p->view, wv, d_rois, d_scmos, d_init, n, fp, d_out5, d_crlb5, d_nll,
-                                   d_status, d_iters, (char*)ctx->scratch, per_cluster, ctx->d_counter);
-        prof_end(ctx, st);
-        if (e != cudaSuccess) { ctx->err = std::string("fit: ") + cudaGetErrorString(e); rc = ZOLA_E_CUDA; }
+        if (!direct)
+            e = f64_config(kernel, f64_cluster(p->N, w->W), F64_THREADS, f64_smem(p->N, p->D, w->W, w->R), piece,
+                           room ? most / per_fft : piece, st, &attr_f, &cfg_f, &cf);
+        char* base = e == cudaSuccess ? area(HEAD + list_b + std::max(cf * per_fft, cd * per_direct)) : nullptr;
+        if (!base) return;
+        int *counters = (int*)base, *list = (int*)(base + HEAD);  // FFT queue, list, direct queue
+        char* work = base + HEAD + list_b;
+        FitParamsDev trial = fp;
+        trial.max_iter = std::min(fp.max_iter, F64_TRIAL);
+        const size_t RR = (size_t)w->R * w->R;
+        for (int a = 0; a < F.n && e == cudaSuccess; a += piece) {
+            const int n = std::min(piece, F.n - a);
+            const float *rois = F.rois + a * RR, *scmos = F.scmos ? F.scmos + a * RR : nullptr;
+            const double* init = F.init + 5 * (size_t)a;
+            double *out5 = F.out5 + 5 * (size_t)a, *crlb5 = F.crlb5 ? F.crlb5 + 5 * (size_t)a : nullptr,
+                   *nll = F.nll ? F.nll + a : nullptr;
+            int *status = F.status ? F.status + a : nullptr, *iters = F.iters ? F.iters + a : nullptr;
+            e = cudaMemsetAsync(counters, 0, 3 * sizeof(int), st);
+            if (!direct && e == cudaSuccess) {
+                e = cudaLaunchKernelEx(&cfg_f, kernel, p->view, wv, rois, scmos, init, n, trial, out5, crlb5, nll, status,
+                                       iters, work, per_fft, counters, list, counters + 1);
+                ctx->launches++;
+            }
+            for (int k = 0; k < nd && e == cudaSuccess; ++k) {
+                e = cudaLaunchKernelEx(&D[k].cfg, fit_direct_kernel, p->view, wv, rois, scmos, init, n,
+                                       direct ? (const int*)nullptr : (const int*)list, (const int*)(counters + 1), fp,
+                                       out5, crlb5, nll, status, iters, work, per_direct, counters + 2, D[k].least,
+                                       D[k].most);
+                ctx->launches++;
+            }
+        }
     });
-    if (rc) return rc;
-    ctx->launches++;
+    return e;
+}
+
+int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_rois, const float* d_scmos,
+                   const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
+                   double* d_nll, int* d_status, int* d_iters, cudaStream_t st, bool direct) {
+    if (n <= 0) return ZOLA_OK;
+    FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
+    const F64Fit F{d_rois, d_scmos, d_init, n, d_out5, d_crlb5, d_nll, d_status, d_iters};
+    bool room = true;
+    prof_begin(ctx, 5, st);
+    const cudaError_t e = fit_f64_launch(ctx, p, w, F, fp, direct, 0, st, [&](size_t bytes) {
+        room = ensure_scratch(ctx, bytes, ctx->err) == 0;
+        return room ? (char*)ctx->scratch : nullptr;
+    });
+    prof_end(ctx, st);
+    if (!room) return ZOLA_E_CUDA;
+    if (e != cudaSuccess) { ctx->err = std::string("fit: ") + cudaGetErrorString(e); return ZOLA_E_CUDA; }
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
     return ZOLA_OK;
 }
@@ -581,34 +1038,16 @@ extern "C" int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois,
     }
     char* base = (char*)noalloc_scratch(ctx->device, ctx->err);
     if (!base) return ZOLA_E_CUDA;
-    const size_t per_cluster = f64_work_bytes(psf->D, w->W, w->R);
-    int* counter = (int*)base;
-    char* work = base + 256;
-    const size_t room = NOALLOC_SCRATCH_BYTES - 256;
-    // The windows that are refused: those whose field, transform and intensity planes
-    // would not fit the array together (the FFT form itself keeps fewer planes).
-    const size_t D = psf->D, W = w->W, planes = (D * D + 3 * D * W) * 16 + (4 * W * W + 4 * R * W + 4 * (size_t)R * R) * 8;
-    if (per_cluster > room || planes > room) {
-        ctx->err = "zola_fit_batch_noalloc: one block's work area (" + std::to_string(std::max(planes, per_cluster)) +
+    const size_t per_cluster = direct_work_bytes(psf->D, w->W, w->R);
+    if (per_cluster > NOALLOC_SCRATCH_BYTES - 256) {
+        ctx->err = "zola_fit_batch_noalloc: one block's work area (" + std::to_string(per_cluster) +
                    " bytes for this ROI size) exceeds the 64 MiB static scratch";
         return ZOLA_E_ARG;
     }
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
-    WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
-    if (e == cudaSuccess)
-        with_fft(psf->N, [&](auto nfft) {
-            auto kernel = fit_f64_kernel<decltype(nfft)::value>;
-            cudaLaunchAttribute attr;
-            cudaLaunchConfig_t cfg;
-            int clusters = 0;
-            e = f64_config(kernel, psf, w, n, (long long)(room / per_cluster), st, &attr, &cfg, &clusters);
-            if (e != cudaSuccess) return;
-            e = cudaLaunchKernelEx(&cfg, kernel, psf->view, wv, d_rois, (const float*)nullptr, d_init5, n, fp, d_out5,
-                                   d_crlb5, d_nll, d_status, d_iters, work, per_cluster, counter);
-            ctx->launches++;
-        });
+    const F64Fit F{d_rois, nullptr, d_init5, n, d_out5, d_crlb5, d_nll, d_status, d_iters};
+    const cudaError_t e = fit_f64_launch(ctx, psf, w, F, fp, false, NOALLOC_SCRATCH_BYTES, st, [&](size_t) { return base; });
     if (e != cudaSuccess) {
         ctx->err = std::string("zola_fit_batch_noalloc: ") + cudaGetErrorString(e);
         return ZOLA_E_CUDA;

@@ -4,8 +4,9 @@
 // The starts of the pipeline's fits are refined against these images, and a split fit's
 // path depends on the last bit of its start: with a library from the FFT form of the same
 // model (fit_f64.cu), 1e-15 away, four of a hundred localizations of 40 px ended up to
-// 10 nm elsewhere on the flat floor of their likelihood.  So this form stays as it is,
-// and a detector gives the same localizations whatever the FP64 fit does.
+// 10 nm elsewhere on the flat floor of their likelihood.  So this form stays as it is, and
+// a movie's fits start from the same bits whatever form the model takes.  (Its FP64 fits
+// are as sensitive by themselves; fit_f64.cu takes them by direct sums too.)
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -436,7 +436,8 @@ __global__ void k_take_acc(int n, const int* acc_slot, const double* theta, doub
 }
 
 // chi2 and CRLB of the accepted localizations (psi, dpsi evaluated at their
-// fitted positions, in acceptance-list order).  A warp a row; a thread a row read
+// fitted positions by direct sums, in acceptance-list order: at z = 0 of a PSF that is the
+// same above and below focus the z bound is made of the derivatives' last bits).  A warp a row; a thread a row read
 // its 4 R^2 model values one after the other (2.0 ms for 100 rows at R = 40).
 __global__ void __launch_bounds__(128) k_pipe_rows(PipeView V, int n, const int* acc_slot, const int* acc_seq,
                                                    const int* status, const double* theta, const double* psi,
@@ -717,11 +718,8 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                 if (rc) return rc;
                 k_pipe_start<<<(nslot + 3) / 4, 128, 0, st>>>(V, nslot);
                 ctx->launches++;
-                rc = scmos ? zola_fit_batch_scmos_dev(ctx, fit_psf, R, (float*)b_rois.p, (float*)b_sv.p,
-                                                      (double*)b_init.p, nslot, &fp, (double*)b_out5.p, nullptr,
-                                                      nullptr, (int*)b_st.p, nullptr, st)
-                           : zola_fit_batch_dev(ctx, fit_psf, R, (float*)b_rois.p, (double*)b_init.p, nslot, &fp,
-                                                (double*)b_out5.p, nullptr, nullptr, (int*)b_st.p, nullptr, st);
+                rc = fit_frames_dev(ctx, fit_psf, R, (float*)b_rois.p, V.slot_v, (double*)b_init.p, nslot, &fp,
+                                    (double*)b_out5.p, (int*)b_st.p, st);
                 if (rc) return rc;
                 // psi at the fitted positions the walk may accept (its model masks)
                 k_take_xyz<<<(nslot + 127) / 128, 128, 0, st>>>(nslot, (double*)b_out5.p, (double*)b_xyz.p);
@@ -756,7 +754,9 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
                                                                (double*)b_xyz.p);
                 ctx->launches++;
                 // the walk has used psi; its buffer now takes the accepted positions' models
-                rc = zola_psf_model_dev(fit_psf, R, (double*)b_xyz.p, nacc, (double*)b_psi.p, (double*)b_dpsi.p, st);
+                WindowTables* wt = get_window(fit_psf, R, ctx->err);
+                if (!wt) return ZOLA_E_ARG;
+                rc = launch_model_direct(ctx, fit_psf, wt, (double*)b_xyz.p, nacc, (double*)b_psi.p, (double*)b_dpsi.p, st);
                 if (rc) return rc;
                 k_pipe_rows<<<(nacc + 3) / 4, 128, 0, st>>>(V, nacc, (int*)b_acc.p, (int*)b_seq.p, (int*)b_st.p,
                                                                 (double*)b_out5.p, (double*)b_psi.p,

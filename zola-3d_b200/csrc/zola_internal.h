@@ -126,8 +126,6 @@ struct zola_ctx {
     size_t calib_bytes = 0;
     void* calib_fit_area = nullptr;  // the calibration LM's tangents, Gram blocks and model (grow-only)
     size_t calib_fit_bytes = 0;
-    int* d_counter = nullptr;
-    int* d_status_word = nullptr;
     int* h_flags = nullptr;      // pinned host words read back by the split fit loop
     zola::HostCopy* host_copy = nullptr;  // helpers of large pageable copies
     char* h_stage = nullptr;     // pinned staging of small host-buffer fits
@@ -250,9 +248,17 @@ void blur_matrix(int R, int W, double sigma, std::vector<double>& G, std::vector
 int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n,
                      double* d_out, double* d_dout, cudaStream_t st, const int* d_list = nullptr,
                      const int* d_count = nullptr);
+// The same with every sum in a fixed order (see fit_f64.cu).
+int launch_model_direct(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* d_xyz, int n, double* d_out,
+                        double* d_dout, cudaStream_t st);
+// direct: every sum in a fixed order from the start.
 int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_rois, const float* d_scmos,
                    const double* d_init, int n, const zola_fit_params* prm, double* d_out5, double* d_crlb5,
-                   double* d_nll, int* d_status, int* d_iters, cudaStream_t st);
+                   double* d_nll, int* d_status, int* d_iters, cudaStream_t st, bool direct = false);
+
+// capi.cu: the frame pipeline's fits (with sCMOS patches when d_scmos is not null); FP64 ones by direct sums.
+int fit_frames_dev(zola_ctx* ctx, zola_psf* psf, int R, const float* d_rois, const float* d_scmos, const double* d_init5,
+                   int n, const zola_fit_params* prm, double* d_out5, int* d_status, cudaStream_t st);
 
 // host_copy.cu: a context's copies from and to host memory of any kind.  As with
 // cudaMemcpyAsync, src may be written again when copy_in returns, and dst may be read when
