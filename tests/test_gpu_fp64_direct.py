@@ -44,6 +44,18 @@ ROWS = [
     (5, 8, -114.32692908356226, 42.567855001469326, 1), (5, 13, -707.4590199848801, 15.157021123722558, 1),
 ]
 
+# bounds of x, y, z, A and B at z = -0.4, -0.1, 0.2 and 0.7 um: saddle-point PSF at 16 px, tetrapod at 32
+CURVES = [
+    (0.007868305689257699, 0.007922431316582936, 0.01882294879580033, 0.04078725005365519, 2.4689880921895866),
+    (0.005461397099965699, 0.005460581283804652, 0.03988488471251728, 0.0332764243269475, 1.9942218007470385),
+    (0.005994802256941714, 0.006017662628759339, 0.022740739160277332, 0.034469653129589176, 2.0699863839537946),
+    (0.013612420594048158, 0.013599980672872408, 0.028550771135346296, 0.07081896749957957, 4.3431914621636585),
+    (0.014001708899311426, 0.00628155679810523, 0.049978319419405615, 0.04260048680692021, 2.2433393029672795),
+    (0.00942903903344569, 0.006721259601168433, 0.034954083140892725, 0.03282525767306106, 1.7224912344024401),
+    (0.006903436329235402, 0.009140991826916035, 0.025556560018025438, 0.0322894701249691, 1.693882068994273),
+    (0.00776725138744841, 0.019450453318943642, 0.023130768564555176, 0.0427080773063525, 2.2490631311078926),
+]
+
 
 def test_fits_around_a_symmetric_focus(zpkg, ctx):
     """Starts at z = 0, 0.05 and -0.1 um: the depths and bounds of FITS to 1e-9, after as many evaluations."""
@@ -79,6 +91,16 @@ def test_movie_with_fits_that_do_not_converge(zpkg, ctx):
     det.close()
     lib.close()
     fit.close()
+
+
+def test_crlb_curves(zpkg, ctx):
+    """CURVES to 1e-11: central differences of 0.5 nm magnify the models' rounding, 1e-16, by up to 1e7."""
+    got = []
+    for N, R, zern in ((64, 16, saddle_zernike()), (128, 32, tetrapod_zernike())):
+        psf = zpkg.PSF(ctx, zpkg.optics(size_fft=N, **OPTICS), zern)
+        got.append(psf.crlb_curve(R, [-0.4, -0.1, 0.2, 0.7]))
+        psf.close()
+    assert np.allclose(np.concatenate(got), CURVES, rtol=1e-11, atol=0)
 
 
 @pytest.mark.parametrize("N,R,n", [(8, 4, 5), (16, 8, 3), (32, 14, 40), (64, 16, 1), (64, 30, 160), (128, 6, 37),

@@ -136,7 +136,9 @@ struct CrlbScan {
                         ctx);
         WindowTables* w = get_window(psf, R, ctx->err);
         if (!w) return ZOLA_E_ARG;
-        int rc = launch_model_f64(ctx, psf, w, d_xyz.p, 7 * n, d_psi.p, nullptr, st);
+        // (direct sums: steps of h magnify the models' rounding 1e7-fold, and the search compares
+        // bounds that are the same above and below a symmetric focus)
+        int rc = launch_model_direct(ctx, psf, w, d_xyz.p, 7 * n, d_psi.p, nullptr, st);
         if (rc) return rc;
         k_center_fisher<<<n, CF_THREADS, 0, st>>>(d_psi.p, (int)RR, photons, bg, h, ha, d_F.p);
         ctx->launches++;
