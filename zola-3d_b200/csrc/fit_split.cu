@@ -3808,6 +3808,17 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
             for (auto& e : ctx->tune_ev) ZOLA_CUDA_CHECK(cudaEventCreate(&e), ctx);
         ZOLA_CUDA_CHECK(cudaEventRecord(ctx->tune_ev[0], st), ctx);
     }
+    // The rounds are issued one ahead of their reports, so the loop ends, well or not, with a
+    // round on st that still looks for occupied slots in the context's scratch.  It is waited
+    // for: the context's next call may use the scratch on another stream, where those kernels
+    // would take what they find there for slots.  (A host-buffer call that ends well
+    // synchronises st itself, behind the copies of its results.)
+    struct Idle {
+        cudaStream_t st;
+        bool wait = true;
+        ~Idle() { if (wait) cudaStreamSynchronize(st); }
+    } idle{st};
+    const bool host_call = feed != nullptr;
     // inputs still arriving: the fit starts on the first chunk, and chunks are
     // handed to the pool as their copies complete
     int chunk = 0, navail = n, queue = 0;
@@ -3898,6 +3909,8 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
         ZOLA_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx->tune_ev[0], ctx->tune_ev[1]), ctx);
         if (evals > 0) pool_record(ctx, pkey, pool, ms * 1e6 / (double)evals);
     }
+    idle.wait = false;
+    if (!host_call) ZOLA_CUDA_CHECK(cudaStreamSynchronize(st), ctx);
     return ZOLA_OK;
 }
 
