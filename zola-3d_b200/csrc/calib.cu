@@ -114,7 +114,7 @@ __device__ inline CalWork cal_carve(char* base, int D, int W, int R) {
 constexpr int CAL_RED_BYTES = 2048;
 constexpr size_t CAL_G_SMEM = 32 * 1024;
 __host__ __device__ inline size_t cal_tile_bytes(int N, int D, int W, int R) {
-    const size_t lines = 2048 / N, q = lines * (D | 1) * 16, x = (size_t)(W + R) * lines * 8;
+    const size_t lines = fl_lines(N), q = lines * (D | 1) * 16, x = (size_t)(W + R) * lines * 8;
     return cal_al(q > x ? q : x);
 }
 __host__ __device__ inline size_t cal_smem(int N, int D, int W, int R) {

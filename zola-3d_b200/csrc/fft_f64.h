@@ -81,25 +81,28 @@ __device__ inline void dft(double2 (&x)[R]) {
     }
 }
 
-// N-point lines, N a power of two: 2048 / N lines at once, 256 threads, a 32 KB
+// N-point lines, N a power of two: fl_lines(N) lines at once, 256 threads, a 32 KB
 // buffer [point][line].  A thread owns one radix-8 or two radix-4 butterflies a
-// pass, its operands stay in registers over the barrier, and it ends with eight
-// outputs, always the same (point, line) for a given thread, so that results of
+// pass (one at N = 4, where a line has no more and there are only as many lines as
+// threads), its operands stay in registers over the barrier, and it ends with eight
+// outputs (four at N = 4), always the same (point, line) for a given thread, so that results of
 // several transforms can be combined in registers.  The lane index runs over the
 // lines first: shared-memory accesses are conflict-free and few twiddles differ.
 constexpr int FL_THREADS = 256, FL_OUT = 8;
+__host__ __device__ constexpr int fl_lines(int N) { return N < 8 ? FL_THREADS : 2048 / N; }
 template <int N_>
 struct FftLines {
-    static constexpr int N = N_, LINES = 2048 / N_;
+    static constexpr int N = N_, LINES = fl_lines(N_);
     static constexpr int R0 = N == 4 || N == 16 ? 4 : 8, R1 = N <= 8 ? 1 : (N <= 32 || N == 128 ? 4 : 8),
                          R2 = N <= 64 ? 1 : (N == 512 ? 8 : 4), R3 = N == 1024 ? 4 : 1;
     static_assert(R0 * R1 * R2 * R3 == N, "4 .. 1024 points");
+    static_assert(LINES <= FL_THREADS && LINES * N <= FL_OUT * FL_THREADS, "a line a thread");
 };
 constexpr size_t FL_SMEM = 2048 * sizeof(double2);
 
 template <class F, int SIGN, int R, int NS, class LD, class ST>
 __device__ __forceinline__ void fl_pass(double2* sm, const double2* tw, const LD& ld, const ST& st) {
-    constexpr int B = 8 / R;  // butterflies a thread
+    constexpr int B = F::LINES * F::N / (FL_THREADS * R);  // butterflies a thread
     constexpr bool first = NS == 1, last = NS * R == F::N;
     constexpr unsigned nb = F::N / R, JS = FL_THREADS / F::LINES;
     const unsigned line = threadIdx.x % F::LINES, j0 = threadIdx.x / F::LINES;
@@ -172,7 +175,7 @@ struct Cluster {
 // CTAs a cluster, by the window's columns (LINES at a time); never by the number of
 // ROIs, so that a result does not depend on its batch.
 __host__ __device__ inline int f64_cluster(int N, int W) {
-    const int t = W / (2048 / N);
+    const int t = W / fl_lines(N);
     return t >= 4 ? 4 : (t >= 2 ? 2 : 1);
 }
 

@@ -92,7 +92,7 @@ __device__ inline DirectWork direct_carve(char* base, int D, int W, int R) {
 // pupil field (LINES rows of D | 1) or of an intensity map (W x LINES), and the
 // transposed blur matrix (W x R) when it is small enough.
 __host__ __device__ inline size_t f64_tile_bytes(int N, int D, int W) {
-    const size_t lines = 2048 / N, q = lines * (D | 1) * 16, x = (size_t)W * lines * 8;
+    const size_t lines = fl_lines(N), q = lines * (D | 1) * 16, x = (size_t)W * lines * 8;
     return align_up(q > x ? q : x, 256);
 }
 __host__ __device__ inline size_t f64_smem(int N, int D, int W, int R) {
