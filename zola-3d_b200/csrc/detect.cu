@@ -182,8 +182,9 @@ struct DetEps {
 };
 
 // In place: sum -> variance of the box, sq -> isv.  With marks, inexact[f] is set
-// where a pixel of frame f is not finite or its bound exceeds DET_EPS_MAX (camera
-// frames have 1e-8 and less), the slack of k_det_peaks' first look.
+// where a pixel of frame f is not finite or the bound of a score that a candidate is
+// compared with exceeds DET_EPS_MAX (camera frames have 1e-8 and less), the slack of
+// k_det_look.
 constexpr double DET_EPS_MAX = 1e-4;
 __global__ void __launch_bounds__(256) k_det_var(DetView V, double* sum, double* sq, DetEps E, int* inexact) {
     const size_t SS = (size_t)V.SX * V.SY;
@@ -196,7 +197,8 @@ __global__ void __launch_bounds__(256) k_det_var(DetView V, double* sum, double*
         sum[f * SS + k] = v;
         sq[f * SS + k] = w;
         const int i = (int)(k / V.SY), j = (int)(k - (size_t)i * V.SY);
-        if (i >= lo && i < V.SX - lo && j >= lo && j < V.SY - lo) bad |= !(kf * w + E.base < DET_EPS_MAX);
+        // (k_det_look compares candidates with the three columns on either side of the inner part)
+        if (i >= lo && i < V.SX - lo && j >= lo - 3 && j < V.SY - lo + 3) bad |= !(kf * w + E.base < DET_EPS_MAX);
     }
     if (inexact && bad) inexact[f] = 1;
 }
