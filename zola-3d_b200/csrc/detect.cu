@@ -31,6 +31,7 @@
 #include <cmath>
 #include <vector>
 
+#include "det_bound.h"
 #include "zola_internal.h"
 
 namespace zola {
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(32) k_det_colsum(DetView V, const double* rows
 }
 
 // Bound of |FFT score - directly summed score| at a pixel: k max|pixel| /
-// sqrt(varImage) + base (det_fft_eps).
+// sqrt(varImage) + base (det_fft_bound).
 struct DetEps {
     double k, base;
     const unsigned long long* amax;  // bits of max|pixel| per frame (k_det_rowsum)
@@ -901,18 +902,6 @@ __global__ void __launch_bounds__(256) k_det_gather(DetView V, const double* can
 // 156 / 161, 196 / 165; 48 frames of 256^2 x 40 at R = 40 18.6 ms / 4.8 ms.
 bool det_fft_wanted(const DetView& v) { return v.thr >= 1e-3 && v.R >= DET_FFT_MIN_R; }
 
-// Bound of |FFT score - directly summed score| = k max|pixel| / sqrt(varImage) + base.
-// Three transforms with relative 2-norm errors of at most 5 u log2(Mx My) each (u = 2^-53),
-// ||img|| <= sqrt(Sx Sy) max|pixel|, ||psf0|| = R sqrt(varPSF), and |FFT(psf0)| <= R ||psf0||
-// (the inverse transform's part); the direct sum's own rounding, at most R^2 u sum |img psf0|;
-// and a few roundings of the score's scaling, |score| <= R^2 / sqrt(Mx My).
-static void det_fft_eps(const DetView& v, const DetFft& p, double* k, double* base) {
-    const double u = std::ldexp(1.0, -53), R = v.R;
-    const double fft = 15 * u * std::log2((double)p.x.M * p.y.M) * (1 + R) * std::sqrt((double)v.SX * v.SY) * R;
-    *k = (fft + u * R * R * R * R) * v.inv_m;
-    *base = 32 * u * (1 + R * R * v.inv_m);
-}
-
 }  // namespace zola
 
 // ------------------------------------------------------------------ host ----
@@ -985,6 +974,7 @@ int zola_detector_create(zola_psf* psf, int SX, int SY, int R, double minZ, doub
     v.thr = thr; v.zstep = step; v.dx = psf->o.xystep;
     v.psf0 = d->d_lib; v.varpsf = d->d_lib + psf0.size(); v.norm = d->d_lib + psf0.size() + varpsf.size();
     det_fft_build(ctx, v, d->fft);
+    d->fft.pair = det_pair_ratio(varpsf.data(), number);
     *out = d;
     return ZOLA_OK;
 }
@@ -1084,7 +1074,7 @@ int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap
         k_det_rowsum<<<dim3((v.SX + VR_ROWS - 1) / VR_ROWS, nf), VR_THREADS, VR_SMEM, st>>>(v, fr, rowsum, rowsq, amax);
         k_det_colsum<<<dim3((v.SY + 31) / 32, nf), 32, 0, st>>>(v, rowsum, rowsq, var, isv);
         DetEps E{0, 0, amax, isv};
-        if (fft) det_fft_eps(v, d->fft, &E.k, &E.base);
+        if (fft) det_fft_bound(v.SX, v.SY, v.R, d->fft.x.M, d->fft.y.M, v.inv_m, d->fft.pair, &E.k, &E.base);
         k_det_var<<<dim3((unsigned)std::min<size_t>((SS + 255) / 256, 256), nf), 256, 0, st>>>(v, var, isv, E,
                                                                                               fft ? inexact : nullptr);
         ctx->launches += 3;

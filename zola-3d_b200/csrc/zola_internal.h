@@ -185,6 +185,7 @@ struct FftDim {
 struct DetFft {
     FftDim x, y;
     int pairs = 0;
+    double pair = 1.0;         // det_pair_ratio of the library
     double2* d_tab = nullptr;  // twiddles of x and y, then the spectra of the slice pairs
     const double2* twx() const { return d_tab; }
     const double2* twy() const { return d_tab + x.M; }
