@@ -1,4 +1,4 @@
-"""The detection's error bound (csrc/det_bound.h), compiled by the host compiler."""
+"""The detection's error bound and open ranks (csrc/det_bound.h), compiled by the host compiler."""
 import ctypes
 import math
 import os
@@ -20,11 +20,13 @@ extern "C" double pair_ratio(const double* v, int Z) { return zola::det_pair_rat
 extern "C" void fft_bound(int SX, int SY, int R, int MX, int MY, double m, double p, double* kb) {
     zola::det_fft_bound(SX, SY, R, MX, MY, m, p, kb, kb + 1);
 }
+extern "C" int tie(double s, double next, double e) { return zola::det_tie(s, next, e); }
 """)
     subprocess.check_call(["g++", "-O2", "-shared", "-fPIC", "-I", CSRC, "-o", str(lib), str(src)])
     b = ctypes.CDLL(str(lib))
     b.pair_ratio.restype = ctypes.c_double
     b.fft_bound.argtypes = [ctypes.c_int] * 5 + [ctypes.c_double] * 2 + [ctypes.c_void_p]
+    b.tie.argtypes = [ctypes.c_double] * 3
     return b
 
 
@@ -72,3 +74,27 @@ def test_pair_ratio_ignores_empty_slices(bound):
     for v, want in (([1.0], 1.0), ([1.0, 0.0], 1.0), ([4.0, 1.0, 1.0], math.sqrt(5)), ([1.0, 1.0, 9.0, 0.25], math.sqrt(37))):
         a = np.array(v)
         assert bound.pair_ratio(a.ctypes.data_as(ctypes.c_void_p), len(a)) == pytest.approx(want)
+
+
+def _runs(bound, s, eps_max):
+    run, runs = 0, [0]
+    for a, b in zip(s[:-1], s[1:]):
+        run += not bound.tie(a, b, eps_max)
+        runs.append(run)
+    return runs
+
+
+def test_open_ranks_are_closed_under_their_bounds(bound):
+    """Scores of different runs are certain against each other, whatever the bounds in between: a wide bound beside
+    narrow ones on either side, then random lists."""
+    cases = [([1.00, 0.99, 0.95], [0.10, 0.001, 0.001]), ([1.00, 0.97, 0.96], [0.001, 0.001, 0.10])]
+    rng = np.random.default_rng(5)
+    for _ in range(200):
+        n = int(rng.integers(2, 40))
+        cases.append((np.sort(rng.uniform(0, 1, n))[::-1], 10.0 ** rng.uniform(-5, -1.5, n)))
+    for s, e in cases:
+        runs = _runs(bound, list(map(float, s)), float(max(e)))
+        for a in range(len(s)):
+            for b in range(a + 1, len(s)):
+                assert runs[a] == runs[b] or s[a] - s[b] > e[a] + e[b]
+    assert len(set(_runs(bound, [1.00, 0.99, 0.95], 0.10))) == 1  # (0.99 and 0.95 are certain, 1.00 and 0.95 are not)

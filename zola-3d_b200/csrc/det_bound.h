@@ -1,5 +1,5 @@
 // What the FFT correlation of the detection may decide by itself: the bound of its
-// scores' error.  Plain arithmetic, host and device.
+// scores' error, and the ranks that it leaves open.  Plain arithmetic, host and device.
 #pragma once
 
 #include <cmath>
@@ -38,5 +38,10 @@ DET_FN void det_fft_bound(int SX, int SY, int R_, int MX, int MY, double inv_m, 
     *k = (fft + u * R * R * R * R) * inv_m;
     *base = 32 * u * (1 + R * R * inv_m);
 }
+
+// Whether two scores next to each other in the order of the screening belong to one run
+// of open ranks.  eps_max: the largest bound in the list, so that scores of different runs
+// are more than any two bounds apart, whichever of a run's they are.
+DET_FN bool det_tie(double s, double next, double eps_max) { return s - next <= 2 * eps_max; }
 
 }  // namespace zola

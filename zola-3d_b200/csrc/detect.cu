@@ -803,8 +803,8 @@ __host__ __device__ inline int det_pow2(int n) {
 // list position.  gs / gid: global sort keys (det_pow2(cap) per frame) or nullptr
 // for the shared-memory form.
 // D.count (nullable): where screening scores next to each other in the order are
-// too close for it to be certain, both candidates are listed (D.frame, D.index) and
-// the pair is marked (D.tie[f][rank]: rank and rank + 1).  k_det_ties orders them.
+// too close for it to be certain (det_tie), both candidates are listed (D.frame, D.index)
+// and the pair is marked (D.tie[f][rank]: rank and rank + 1).  k_det_ties orders them.
 struct DetTies {
     int *count, *frame, *index;
     unsigned char* tie;
@@ -812,6 +812,7 @@ struct DetTies {
 __global__ void __launch_bounds__(1024) k_det_sort(DetView V, const double* cand, const int* counts, int* order, double* gs,
                                                    int* gid, DetEps E, const int* inexact, DetTies D) {
     extern __shared__ double smraw[];
+    __shared__ unsigned long long eps_bits;
     const int f = blockIdx.x, n = min(counts[f], V.cap);
     const int P2 = det_pow2(n);
     double* s = gs ? gs + (size_t)f * det_pow2(V.cap) : smraw;
@@ -821,7 +822,19 @@ __global__ void __launch_bounds__(1024) k_det_sort(DetView V, const double* cand
         if (t < n) { s[t] = c[(size_t)t * 7]; id[t] = t; }
         else { s[t] = -INFINITY; id[t] = 0x7fffffff; }
     }
+    if (threadIdx.x == 0) eps_bits = 0;
     __syncthreads();
+    // the largest bound of the list (positive: its bits are in its order)
+    const bool screened = D.count && !inexact[f];
+    if (screened) {
+        const double kf = E.k * __longlong_as_double((long long)E.amax[f]);
+        double m = 0.0;
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const double* r = c + (size_t)t * 7;
+            m = fmax(m, kf * fmax(E.isv[((size_t)f * V.SX + (int)r[2]) * V.SY + (int)r[3]], 0.0) + E.base);
+        }
+        atomicMax(&eps_bits, (unsigned long long)__double_as_longlong(m));
+    }
     // bitonic network: "before" = higher score, then earlier in the list
     for (int size = 2; size <= P2; size <<= 1)
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -838,17 +851,12 @@ __global__ void __launch_bounds__(1024) k_det_sort(DetView V, const double* cand
             }
             __syncthreads();
         }
-    const double kf = D.count && !inexact[f] ? E.k * __longlong_as_double((long long)E.amax[f]) : -1.0;
-    auto eps = [&](int p) {
-        const double* t = c + (size_t)p * 7;
-        return kf * fmax(E.isv[((size_t)f * V.SX + (int)t[2]) * V.SY + (int)t[3]], 0.0) + E.base;
-    };
+    __syncthreads();
+    const double eps_max = __longlong_as_double((long long)eps_bits);
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         order[(size_t)f * V.cap + t] = id[t];
         if (!D.count) continue;
-        // most gaps exceed every bound (DET_EPS_MAX)
-        const bool tie = kf >= 0 && t + 1 < n && s[t] - s[t + 1] <= 2 * DET_EPS_MAX &&
-                         s[t] - s[t + 1] <= eps(id[t]) + eps(id[t + 1]);
+        const bool tie = screened && t + 1 < n && det_tie(s[t], s[t + 1], eps_max);
         D.tie[(size_t)f * V.cap + t] = tie;
         if (tie) {  // (the middle of a longer run is listed twice, with the same result)
             const int o = atomicAdd(D.count, 2);
@@ -860,7 +868,8 @@ __global__ void __launch_bounds__(1024) k_det_sort(DetView V, const double* cand
 }
 
 // Orders each run of marked ranks by the direct scores (ties by list position): a
-// thread a run, nearly always a pair.  Scores outside a run are certain against it.
+// thread a run, nearly always a pair.  Scores outside a run are certain against it
+// (det_tie).
 __global__ void __launch_bounds__(256) k_det_ties(DetView V, const double* cand, const int* counts, int* order,
                                                   const unsigned char* tie) {
     const int f = blockIdx.y, n = min(counts[f], V.cap);
