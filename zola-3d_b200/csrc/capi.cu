@@ -148,6 +148,7 @@ int zola_ctx_destroy(zola_ctx* ctx) {
     if (ctx->io) cudaFree(ctx->io);
     if (ctx->calib_area) cudaFree(ctx->calib_area);
     if (ctx->calib_fit_area) cudaFree(ctx->calib_fit_area);
+    if (ctx->drift_area) cudaFree(ctx->drift_area);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
     if (ctx->h_post) cudaFreeHost(ctx->h_post);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);

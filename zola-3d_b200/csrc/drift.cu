@@ -631,7 +631,7 @@ extern "C" int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crl
     for (int t = 0; t < bin - 1; ++t)
         for (int s = t + 1; s < bin; ++s) { p1.push_back(t); p2.push_back(s); }
     const int tot = (int)p1.size();
-    // device buffers, carved from the context's scratch: localizations, pairs, twiddles, the
+    // device buffers, carved from one area: localizations, pairs, twiddles, the
     // Gaussian, spectra, what the pairs of a chunk need at once, the summed correlations
     const bool planes = (size_t)D.P1 * D.P2 <= PLANE_MAX;
     const size_t per_pair = planes ? (size_t)D.P0 * D.S1 * D.S2 : PV;
@@ -660,12 +660,27 @@ extern "C" int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crl
     auto want = [&](size_t bytes) { const size_t o = need; need += (bytes + 255) / 256 * 256; return o; };
     const size_t o_xyz = want((size_t)24 * n), o_frame = want((size_t)4 * n), o_p1 = want((size_t)4 * tot),
                  o_p2 = want((size_t)4 * tot), o_tw = want(FFT_LMAX / 2 * sizeof(float2)), o_gauss = want(PV * 4),
-                 o_drift = want((size_t)24 * tot), o_win = want(nwin * sizeof(DriftWin)), o_hist = want(RV * bin * 4 * WB),
+                 o_drift = want((size_t)24 * tot), o_win = want(nwin * sizeof(DriftWin)), o_hist = want(planes ? RV * bin * 4 * WB : 0),
                  o_fxy = want(planes ? (size_t)D.S0 * D.P1 * D.P2 * bin * WB * sizeof(float2) : 0),
                  o_spec = want(PV * bin * WB * sizeof(float2)), o_corr = want(tot > 0 ? per_pair * CH * WB * sizeof(float2) : 0),
                  o_res = want(RV * tot * sizeof(float));
-    if (ensure_scratch(ctx, need, ctx->err)) return ZOLA_E_CUDA;
-    char* base = (char*)ctx->scratch;
+    // The area is one of its own (the context's scratch may be at work on another stream).  Up
+    // to DRIFT_KEEP it stays with the context: to allocate and free 120 MB takes 2 to 4 ms of
+    // a call of 20.  A job of long windows takes several GB and gives them back.
+    constexpr size_t DRIFT_KEEP = (size_t)256 << 20;
+    DevBuf<char> large;
+    char* base = (char*)ctx->drift_area;
+    if (need > DRIFT_KEEP) {
+        ZOLA_CUDA_CHECK(large.alloc(need), ctx);
+        base = large.p;
+    } else if (need > ctx->drift_bytes) {
+        if (base) cudaFree(base);
+        ctx->drift_area = nullptr;
+        ctx->drift_bytes = 0;
+        ZOLA_CUDA_CHECK(cudaMalloc(&ctx->drift_area, need), ctx);
+        ctx->drift_bytes = need;
+        base = (char*)ctx->drift_area;
+    }
     double *d_xyz = (double*)(base + o_xyz), *d_drift = (double*)(base + o_drift);
     int *d_frame = (int*)(base + o_frame), *d_p1 = (int*)(base + o_p1), *d_p2 = (int*)(base + o_p2);
     float2 *d_tw = (float2*)(base + o_tw), *d_fxy = (float2*)(base + o_fxy), *d_spec = (float2*)(base + o_spec),

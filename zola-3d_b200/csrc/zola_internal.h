@@ -126,6 +126,8 @@ struct zola_ctx {
     size_t calib_bytes = 0;
     void* calib_fit_area = nullptr;  // the calibration LM's tangents, Gram blocks and model (grow-only)
     size_t calib_fit_bytes = 0;
+    void* drift_area = nullptr;  // buffers of drift jobs up to a limit
+    size_t drift_bytes = 0;
     int* h_flags = nullptr;      // pinned host words read back by the split fit loop
     zola::HostCopy* host_copy = nullptr;  // helpers of large pageable copies
     char* h_stage = nullptr;     // pinned staging of small host-buffer fits
