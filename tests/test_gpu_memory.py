@@ -26,3 +26,20 @@ def test_drift_gives_its_buffers_back(zpkg):
     job = lambda bins: zpkg.drift(ctx, xyz, fr, cr, pixel_nm=10.0, bins=bins, max_drift_um=1.28)  # noqa: E731
     assert _kept(lambda: job(6), lambda: job(2)) < 64 << 20
     ctx.close()
+
+
+@pytest.mark.parametrize("derivs", [False, True])
+def test_large_model_calls_give_their_buffers_back(zpkg, derivs):
+    """Models of 0.6 GB: the same as in small calls, and no more is kept than a call of 256 MB keeps (in steps of
+    64 MB, and as much for what else may move)."""
+    ctx = zpkg.Context(0)
+    psf = zpkg.PSF(ctx, zpkg.optics(size_fft=64, **OPTICS), astig_zernike())
+    xyz = np.random.default_rng(1).uniform(-0.3, 0.3, (73000 // (4 if derivs else 1), 3))
+    got = []
+    kept = _kept(lambda: got.append(psf.model(32, xyz, derivs=derivs)), lambda: psf.model(32, xyz[:10], derivs=derivs))
+    assert kept < 384 << 20
+    pick = np.r_[0:7, len(xyz) - 7:len(xyz)]
+    few, many = psf.model(32, xyz[pick], derivs=derivs), got[0]
+    for a, b in zip(few, many) if derivs else [(few, many)]:
+        assert np.array_equal(a, b[pick])
+    ctx.close()

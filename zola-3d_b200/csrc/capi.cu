@@ -278,10 +278,14 @@ int zola_psf_model_prec(zola_psf* psf, int R, const double* xyz, int n, double* 
     if (R < 4 || R % 2 || R > psf->N) return set_err(ctx, ZOLA_E_ARG, "ROI side must be even, >= 4 and <= the pupil grid");
     if (n == 0) return ZOLA_OK;
     cudaSetDevice(ctx->device);
-    // positions, models and derivatives in the context's grow-only staging area
-    const size_t rr = (size_t)R * R, nx = ((size_t)3 * n + 31) / 32 * 32;
-    if (ensure_io(ctx, (nx + rr * n * (dout ? 4 : 1)) * sizeof(double))) return ZOLA_E_CUDA;
-    double* dx = (double*)ctx->io;
+    // positions, models and derivatives in the context's staging area, which never shrinks;
+    // what it has no room for and is above MODEL_KEEP is allocated for the call
+    constexpr size_t MODEL_KEEP = (size_t)256 << 20;
+    const size_t rr = (size_t)R * R, nx = ((size_t)3 * n + 31) / 32 * 32, need = nx + rr * n * (dout ? 4 : 1);
+    DevBuf<double> large;
+    if (need * sizeof(double) > std::max(MODEL_KEEP, ctx->io_bytes)) ZOLA_CUDA_CHECK(large.alloc(need), ctx);
+    else if (ensure_io(ctx, need * sizeof(double))) return ZOLA_E_CUDA;
+    double* dx = large.p ? large.p : (double*)ctx->io;
     double* d_psi = dx + nx;
     double* d_der = dout ? d_psi + rr * n : nullptr;
     ZOLA_CUDA_CHECK(cudaMemcpyAsync(dx, xyz, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream), ctx);
