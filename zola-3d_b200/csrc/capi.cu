@@ -136,6 +136,16 @@ int zola_ctx_create(int device, zola_ctx** out) {
         delete c;
         return ZOLA_E_CUDA;
     }
+    cudaMemPoolProps pool{};
+    pool.allocType = cudaMemAllocationTypePinned;
+    pool.location.type = cudaMemLocationTypeDevice;
+    pool.location.id = device;
+    unsigned long long keep = (unsigned long long)64 << 20;
+    if (cudaMemPoolCreate(&c->pool, &pool) != cudaSuccess ||
+        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        delete c;
+        return ZOLA_E_CUDA;
+    }
     *out = c;
     return ZOLA_OK;
 }
@@ -149,6 +159,7 @@ int zola_ctx_destroy(zola_ctx* ctx) {
     if (ctx->calib_area) cudaFree(ctx->calib_area);
     if (ctx->calib_fit_area) cudaFree(ctx->calib_fit_area);
     if (ctx->drift_area) cudaFree(ctx->drift_area);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
     if (ctx->h_post) cudaFreeHost(ctx->h_post);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);

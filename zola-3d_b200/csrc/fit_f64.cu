@@ -748,6 +748,36 @@ __global__ void __launch_bounds__(F64_THREADS, 2) fit_f64_kernel(PsfView P, WinV
     cl.sync();  // no CTA leaves while another may read its shared memory
 }
 
+// Device memory for a launch on st.  Windows whose direct form takes 192 KB have it from
+// the context's pool, in the order of the stream, so that their models and fits may run on
+// several streams at once, beside other users of the scratch, and be captured at any time
+// (they once had no memory but a CTA's shared one).  Larger windows share the scratch.
+struct F64Area {
+    zola_ctx* ctx;
+    cudaStream_t st;
+    bool own;
+    void* p = nullptr;
+    bool failed = false;
+    F64Area(zola_ctx* c, const zola_psf* psf, const WindowTables* w, cudaStream_t s)
+        : ctx(c), st(s), own(direct_work_bytes(psf->D, w->W, w->R) <= 192 * 1024) {}
+    F64Area(const F64Area&) = delete;
+    F64Area& operator=(const F64Area&) = delete;
+    ~F64Area() { if (p) cudaFreeAsync(p, st); }
+    char* get(size_t bytes) {
+        if (!own) {
+            failed = ensure_scratch(ctx, bytes, ctx->err) != 0;
+            return failed ? nullptr : (char*)ctx->scratch;
+        }
+        const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, ctx->pool, st);
+        if (e == cudaSuccess) return (char*)p;
+        failed = true;
+        p = nullptr;
+        ctx->err = std::string("work area: ") + cudaGetErrorString(e);
+        cudaGetLastError();
+        return nullptr;
+    }
+};
+
 // Launch configuration for n ROIs or models in clusters of C CTAs: as many clusters as run
 // at once (at most `most`).  attr and cfg live as long as the launch.
 template <class K>
@@ -777,6 +807,7 @@ int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* 
     const size_t per_cluster = f64_work_bytes(p->D, w->W, w->R);
     WinView wv{w->R, w->W, w->d_C, w->d_G, w->d_GT};
     int rc = ZOLA_OK;
+    F64Area area(ctx, p, w, st);
     with_fft(p->N, [&](auto nfft) {
         auto kernel = model_f64_kernel<decltype(nfft)::value>;
         cudaLaunchAttribute attr;
@@ -784,11 +815,11 @@ int launch_model_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const double* 
         int clusters = 0;
         cudaError_t e = f64_config(kernel, f64_cluster(p->N, w->W), F64_THREADS, f64_smem(p->N, p->D, w->W, w->R), n, n, st, &attr,
                                    &cfg, &clusters);
-        if (e == cudaSuccess && ensure_scratch(ctx, per_cluster * (size_t)clusters, ctx->err)) { rc = ZOLA_E_CUDA; return; }
+        char* work = e == cudaSuccess ? area.get(per_cluster * (size_t)clusters) : nullptr;
+        if (area.failed) { rc = ZOLA_E_CUDA; return; }
         prof_begin(ctx, 6, st);
         if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, kernel, p->view, wv, d_xyz, n, d_out, d_dout, (char*)ctx->scratch, per_cluster,
-                                   d_list, d_count);
+            e = cudaLaunchKernelEx(&cfg, kernel, p->view, wv, d_xyz, n, d_out, d_dout, work, per_cluster, d_list, d_count);
         prof_end(ctx, st);
         if (e != cudaSuccess) { ctx->err = std::string("model: ") + cudaGetErrorString(e); rc = ZOLA_E_CUDA; }
     });
@@ -912,14 +943,12 @@ int launch_fit_f64(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d_r
     if (n <= 0) return ZOLA_OK;
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
     const F64Fit F{d_rois, d_scmos, d_init, n, d_out5, d_crlb5, d_nll, d_status, d_iters};
-    bool room = true;
+    F64Area area(ctx, p, w, st);
     prof_begin(ctx, 5, st);
-    const cudaError_t e = fit_f64_launch(ctx, p, w, F, fp, direct, 0, st, [&](size_t bytes) {
-        room = ensure_scratch(ctx, bytes, ctx->err) == 0;
-        return room ? (char*)ctx->scratch : nullptr;
-    });
+    const cudaError_t e =
+        fit_f64_launch(ctx, p, w, F, fp, direct, 0, st, [&](size_t bytes) { return area.get(bytes); });
     prof_end(ctx, st);
-    if (!room) return ZOLA_E_CUDA;
+    if (area.failed) return ZOLA_E_CUDA;
     if (e != cudaSuccess) { ctx->err = std::string("fit: ") + cudaGetErrorString(e); return ZOLA_E_CUDA; }
     ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
     return ZOLA_OK;

@@ -122,6 +122,7 @@ struct zola_ctx {
     // results of one call; never overlaps scratch)
     void* io = nullptr;
     size_t io_bytes = 0;
+    cudaMemPool_t pool = nullptr;  // work areas of small windows' FP64 models and fits
     void* calib_area = nullptr;  // calibration work buffers (grow-only, reused by every call)
     size_t calib_bytes = 0;
     void* calib_fit_area = nullptr;  // the calibration LM's tangents, Gram blocks and model (grow-only)
