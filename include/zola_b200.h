@@ -371,8 +371,9 @@ ZOLA_API int zola_drift(zola_ctx* ctx, const double* xyz_nm, const double* crlb_
  * prepares them); the call itself allocates nothing.  It makes the PSF's
  * device current, as the other entry points do.  Its first call on a device
  * (and its first call after that device's context was destroyed and created
- * again, e.g. by cudaDeviceReset) looks up the array's device address; make
- * that first call before any stream capture.  ROI sizes whose per-block work area exceeds the array are
+ * again, e.g. by cudaDeviceReset) looks up the array's device address and loads
+ * the kernels of every pupil grid, which may allocate; make that first call
+ * before any stream capture.  ROI sizes whose per-block work area exceeds the array are
  * rejected with ZOLA_E_ARG; large windows run on fewer blocks.  All calls share
  * the array: calls that overlap on the GPU race, so serialise them. */
 ZOLA_API int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois, const double* d_init5, int n,

@@ -1007,10 +1007,37 @@ void* current_context() {
     return c;
 }
 
+// Every kernel that a call may need, of every pupil grid, launched once on no ROIs: a
+// kernel's first launch loads it, and may enlarge the stacks, which takes device memory (2 MB
+// for one grid of seven).  base: the array.
+cudaError_t noalloc_load(const zola_psf& p, const zola::WindowTables& w, char* base, cudaStream_t st) {
+    using namespace zola;
+    PsfView P = p.view;
+    P.D = 4;
+    const WinView wv{4, 4, w.d_C, w.d_G, w.d_GT};  // (its tables are at least as large)
+    const FitParamsDev fp{};
+    int* counter = (int*)base;
+    cudaError_t e = cudaMemsetAsync(counter, 0, 3 * sizeof(int), st);
+    for (int N = 4; N <= 1024 && e == cudaSuccess; N *= 2)
+        with_fft(N, [&](auto nfft) {
+            auto kernel = fit_f64_kernel<decltype(nfft)::value>;
+            const size_t smem = f64_smem(N, P.D, wv.W, wv.R);
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return;
+            kernel<<<1, F64_THREADS, smem, st>>>(P, wv, nullptr, nullptr, nullptr, 0, fp, nullptr, nullptr, nullptr, nullptr,
+                                                 nullptr, base + 256, 0, counter, nullptr, nullptr);
+            e = cudaGetLastError();
+        });
+    if (e != cudaSuccess) return e;
+    fit_direct_kernel<<<1, DIRECT_THREADS, 0, st>>>(P, wv, nullptr, nullptr, nullptr, 0, nullptr, nullptr, fp, nullptr,
+                                                    nullptr, nullptr, nullptr, nullptr, base + 256, 0, counter + 2, 0, 0);
+    return cudaGetLastError();
+}
+
 // Device address of the scratch array in the current context (host code must
 // not use the array's name as a device pointer).  Looked up once per device
-// and context; the caller has made the device current.
-void* noalloc_scratch(int device, std::string& err) {
+// and context, when *fresh is set; the caller has made the device current.
+void* noalloc_scratch(int device, std::string& err, bool* fresh) {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     if (device < 0 || device >= 64) {
         err = "zola_fit_batch_noalloc: device index out of range";
@@ -1018,7 +1045,8 @@ void* noalloc_scratch(int device, std::string& err) {
     }
     void* c = current_context();
     NoallocEntry& e = g_noalloc[device];
-    if (!e.ptr || c != e.context) {
+    *fresh = !e.ptr || c != e.context;
+    if (*fresh) {
         void* p = nullptr;
         cudaError_t rc = cudaGetSymbolAddress(&p, g_fit_noalloc_scratch);
         if (rc != cudaSuccess || !p) {
@@ -1066,7 +1094,8 @@ extern "C" int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois,
         ctx->err = "zola_fit_batch_noalloc: cudaSetDevice failed";
         return ZOLA_E_CUDA;
     }
-    char* base = (char*)noalloc_scratch(ctx->device, ctx->err);
+    bool fresh = false;
+    char* base = (char*)noalloc_scratch(ctx->device, ctx->err, &fresh);
     if (!base) return ZOLA_E_CUDA;
     const size_t per_cluster = direct_work_bytes(psf->D, w->W, w->R);
     if (per_cluster > NOALLOC_SCRATCH_BYTES - 256) {
@@ -1077,7 +1106,9 @@ extern "C" int zola_fit_batch_noalloc(zola_psf* psf, int R, const float* d_rois,
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     FitParamsDev fp{prm->zmin, prm->zmax, prm->xymax, prm->tol_xyz, prm->step_xy, prm->step_z, prm->max_iter};
     const F64Fit F{d_rois, nullptr, d_init5, n, d_out5, d_crlb5, d_nll, d_status, d_iters};
-    const cudaError_t e = fit_f64_launch(ctx, psf, w, F, fp, false, NOALLOC_SCRATCH_BYTES, st, [&](size_t) { return base; });
+    cudaError_t e = fresh ? noalloc_load(*psf, *w, base, st) : cudaSuccess;
+    if (e == cudaSuccess)
+        e = fit_f64_launch(ctx, psf, w, F, fp, false, NOALLOC_SCRATCH_BYTES, st, [&](size_t) { return base; });
     if (e != cudaSuccess) {
         ctx->err = std::string("zola_fit_batch_noalloc: ") + cudaGetErrorString(e);
         return ZOLA_E_CUDA;
