@@ -85,9 +85,45 @@ __device__ inline double warp_max(double v) {
     return v;
 }
 
+// getAandB's sums over the patch at `corner`, by one warp: *A of the pixels whose library
+// PSF is not under thr and *B of those under it, pixel after pixel in the order of getAandB's
+// loop (the even lanes add up B and the odd ones A); returns the number under thr.
+__device__ int pipe_sums(const PipeView& V, const double* img, const double* psf, size_t corner, double thr, double* A,
+                         double* B) {
+    const double* vm = V.vmap;
+    const int R = V.R, RR = R * R, SY = V.SY, lane = threadIdx.x & 31;
+    auto pixel = [&](int k, bool& low) {
+        if (k >= RR) return 0.0;
+        const size_t px = corner + (size_t)(k / R) * SY + k % R;
+        low = psf[k] < thr;
+        return img[px] - (vm ? vm[px] : 0.0);
+    };
+    bool low = false;
+    double v = pixel(lane, low), sum = 0;
+    int cb = 0;
+    for (int k0 = 0; k0 < RR; k0 += 32) {
+        const unsigned lows = __ballot_sync(0xffffffffu, low);
+        const double cur = v;
+        low = false;
+        v = pixel(k0 + 32 + lane, low);  // on its way while this one is added up
+        const unsigned mine = (lane & 1) ? ~lows : lows;
+        cb += __popc(lows);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            const double x = __shfl_sync(0xffffffffu, cur, q);
+            sum += (mine >> q & 1u) ? x : 0.0;
+        }
+    }
+    *B = __shfl_sync(0xffffffffu, sum, 0);
+    *A = __shfl_sync(0xffffffffu, sum, 1);
+    return cb;
+}
+
 // Whether a candidate is fitted (maxPatch / B > maxSNR and B > 0), by one warp, with B
 // of getAandB: the mean of the pixels whose library PSF of slice r is under 10% of its
-// maximum, of the patch minus the sCMOS term when there is one (:1119-1211).
+// maximum, of the patch minus the sCMOS term when there is one (:1119-1211).  The lanes'
+// own sums decide wherever the rounding of any order of the sum leaves no doubt (a sum of
+// n terms is off by at most n u times the sum of their magnitudes), and pipe_sums else.
 __device__ bool pipe_fitted(const PipeView& V, const double* img, int r, int ci, int cj, double* maxp_) {
     const double* vm = V.vmap;
     const int R = V.R, RR = R * R, SY = V.SY, lane = threadIdx.x & 31;
@@ -103,20 +139,36 @@ __device__ bool pipe_fitted(const PipeView& V, const double* img, int r, int ci,
     maxi = warp_max(maxi);
     maxp = warp_max(maxp);
     const double thr = maxi * 0.1;
-    double B = 0;
+    double B = 0, mag = 0;
     int cb = 0;
 #pragma unroll 4
     for (int k = lane; k < RR; k += 32) {
         const size_t px = corner + (size_t)(k / R) * SY + k % R;
         const bool low = psf[k] < thr;
-        B += low ? img[px] - (vm ? vm[px] : 0.0) : 0.0;
+        const double x = low ? img[px] - (vm ? vm[px] : 0.0) : 0.0;
+        B += x;
+        mag += fabs(x);
         cb += low;
     }
     B = warp_sum(B);
+    mag = warp_sum(mag);
     cb = __reduce_add_sync(0xffffffffu, cb);
-    B = cb != 0 ? B / cb : 0.0;
     *maxp_ = maxp;
-    return maxp / B > V.max_snr && B > 0;
+    auto fitted = [&](double b) { return maxp / b > V.max_snr && b > 0; };
+    if (cb == 0) return fitted(0.0);
+    // both orders' sums and the roundings of the mean and the ratio, with room to spare; the
+    // test is monotone in b on either side of zero
+    const double err = 4e-16 * (RR + 8) * mag / cb, lo = B / cb - err, hi = B / cb + err;
+    const double s_lo = V.max_snr * (1 - 1e-15), s_hi = V.max_snr * (1 + 1e-15);
+    if (hi <= 0) return false;
+    if (lo > 0) {
+        const double a = maxp / lo, b = maxp / hi;
+        if (fmin(a, b) > fmax(s_lo, s_hi)) return true;
+        if (fmax(a, b) < fmin(s_lo, s_hi)) return false;
+    }
+    double A;
+    pipe_sums(V, img, psf, corner, thr, &A, &B);
+    return fitted(B / cb);
 }
 
 // near_mask from the mask, 32 rows of a frame a CTA: rows as words of bits, each the OR of
@@ -252,47 +304,22 @@ __global__ void __launch_bounds__(PW_THREADS) k_pipe_wave(PipeView V, int K) {
 }
 
 // Starts of the wave's slots: the candidates' refined offsets, loc.init(A, B, -dx, -dy,
-// range[r] + dz), and getAandB's A and B (pipe_fitted's B).  A warp a slot; the even lanes
-// add up B and the odd ones A, pixel after pixel: a split fit's path depends on the last
-// bit of its start, so the sums keep the order of getAandB's loop.  (40 px: 1,600 adds,
+// range[r] + dz), and getAandB's A and B.  A warp a slot: a split fit's path depends on the
+// last bit of its start, so the sums keep the order of getAandB's loop.  (40 px: 1,600 adds,
 // one after the other, about 30 us for a wave of 768 slots.)
 __global__ void __launch_bounds__(128) k_pipe_start(PipeView V, int n) {
     const int s = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (s >= n) return;
     const double* row = V.cand + ((size_t)V.slot_frame[s] * V.cap + V.slot_cand[s]) * 7;
-    const double* vm = V.vmap;
-    const int R = V.R, RR = R * R, SY = V.SY;
+    const int R = V.R, RR = R * R;
     const int r = (int)llrint(row[1]), ci = (int)llrint(row[2]), cj = (int)llrint(row[3]);
-    const double* img = V.fimg + (size_t)V.slot_frame[s] * V.SX * SY;
-    const size_t corner = (size_t)(ci - R / 2) * SY + (cj - R / 2);
+    const double* img = V.fimg + (size_t)V.slot_frame[s] * V.SX * V.SY;
     const double* psf = V.libpsf + (size_t)r * RR;
     double maxi = -INFINITY;
 #pragma unroll 4
     for (int k = lane; k < RR; k += 32) maxi = fmax(maxi, psf[k]);
-    const double thr = warp_max(maxi) * 0.1;
-    auto pixel = [&](int k, bool& low) {
-        if (k >= RR) return 0.0;
-        const size_t px = corner + (size_t)(k / R) * SY + k % R;
-        low = psf[k] < thr;
-        return img[px] - (vm ? vm[px] : 0.0);
-    };
-    bool low = false;
-    double v = pixel(lane, low), sum = 0;
-    int cb = 0;
-    for (int k0 = 0; k0 < RR; k0 += 32) {
-        const unsigned lows = __ballot_sync(0xffffffffu, low);
-        const double cur = v;
-        low = false;
-        v = pixel(k0 + 32 + lane, low);  // on its way while this one is added up
-        const unsigned mine = (lane & 1) ? ~lows : lows;
-        cb += __popc(lows);
-#pragma unroll
-        for (int q = 0; q < 32; ++q) {
-            const double x = __shfl_sync(0xffffffffu, cur, q);
-            sum += (mine >> q & 1u) ? x : 0.0;
-        }
-    }
-    double B = __shfl_sync(0xffffffffu, sum, 0), A = __shfl_sync(0xffffffffu, sum, 1);
+    double A, B;
+    const int cb = pipe_sums(V, img, psf, (size_t)(ci - R / 2) * V.SY + (cj - R / 2), warp_max(maxi) * 0.1, &A, &B);
     if (lane != 0) return;
     B = cb != 0 ? B / cb : 0.0;
     A -= (double)(RR - cb) * B;
