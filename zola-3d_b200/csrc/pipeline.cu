@@ -542,15 +542,15 @@ struct Buf {
 };
 
 // Speculative fits per frame and wave: 8, and up to 64 in split fits of few frames.  A round
-// of a split fit costs nearly the same until every SM has a unit or two (200 slots at a
-// window of 128, 600 at 64, 1,500 at 32), and more fits a wave make fewer waves; beyond
+// of a split fit costs nearly the same until every SM has a unit or two (4 slots for 3 SMs
+// at a window of 128, 4 an SM at 64, 10 at 32), and more fits a wave make fewer waves; beyond
 // that, the fits of candidates that an acceptance of the same wave masks are not free.
-// At 8 and at this rule's: 2 frames of 40 px 42 and 21 ms, 12 of them 56 and 46, 6 of 24 px
+// At 8 and at this rule's (148 SMs): 2 frames of 40 px 42 and 21 ms, 12 of them 56 and 46, 6 of 24 px
 // 56 and 30, 20 of 16 px 35 and 18; 96 frames of 40 px at 8, 12 and 16: 146, 160 and 176.
 constexpr int PIPE_WAVE_FITS = 8, PIPE_WAVE_MAX = 64;
-int wave_fits(int R, int N, int frames, int precision) {
+int wave_fits(int sms, int R, int N, int frames, int precision) {
     if (precision != ZOLA_PREC_SPLIT) return PIPE_WAVE_FITS;
-    const int W = window_size(R, N), slots = W >= 128 ? 200 : W >= 64 ? 600 : 1500;
+    const int W = window_size(R, N), slots = W >= 128 ? 4 * sms / 3 : W >= 64 ? 4 * sms : 10 * sms;
     return std::max(PIPE_WAVE_FITS, std::min(PIPE_WAVE_MAX, slots / frames));
 }
 // Candidates stored per frame at the start of a call: a 256 x 256 frame against a
@@ -602,7 +602,7 @@ int localize_impl(zola_ctx* ctx, zola_detector* det, zola_psf* fit_psf, const do
     cudaStream_t st = ctx->stream;
     ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_pipe_near, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)near_smem(SY, R)),
                     ctx);
-    const int K = prm->wave_fits > 0 ? prm->wave_fits : wave_fits(R, fit_psf->N, FB, prm->precision);
+    const int K = prm->wave_fits > 0 ? prm->wave_fits : wave_fits(ctx->num_sms, R, fit_psf->N, FB, prm->precision);
     const int slot_cap = FB * K;
     Buf b_img, b_mask, b_cand, b_cnt, b_lib, b_rng, b_cslot, b_cmax, b_ptr, b_lim, b_done, b_ns, b_rois, b_init, b_sf,
         b_sc, b_out5, b_st, b_xyz, b_psi, b_mthr, b_acc, b_seq, b_nacc, b_dpsi, b_rows, b_fimg, b_adu, b_off, b_gain,
