@@ -49,6 +49,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 
 #include "lm.h"
 #include "umma.h"
@@ -3381,11 +3382,13 @@ static int ensure_post(zola_ctx* ctx) {
     return ZOLA_OK;
 }
 
-// Waits for report `seq` of a fit that runs on st.
-static int wait_post(zola_ctx* ctx, unsigned seq, cudaStream_t st, int* active, int* err, int* queue) {
+// Waits for report `seq` of a fit that runs on st; between looks the thread gives its core
+// away where the application asked the device's waits to (cudaDeviceScheduleYield).
+static int wait_post(zola_ctx* ctx, unsigned seq, cudaStream_t st, bool yield, int* active, int* err, int* queue) {
     const int* w = ctx->h_post + 4 * (seq % POST_RING);
     for (unsigned spin = 1;; ++spin) {
         if ((unsigned)__atomic_load_n(w + 3, __ATOMIC_ACQUIRE) == seq) break;
+        if (yield) std::this_thread::yield();
         if (spin % 4096) continue;
         const cudaError_t e = cudaStreamQuery(st);
         if (e == cudaErrorNotReady) continue;
@@ -3855,8 +3858,12 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
     const bool fused = ctx->split_mode == ZOLA_SPLIT_FUSED && fused_fits(*sp.pl);
     // With every ROI on the device the rounds are issued one ahead of their reports
     // (post_state); otherwise, and with the profile's events between the kernels, four at
-    // a time with the flags read after them.
-    const bool posted = !fused && !feed && !ctx->profile;
+    // a time with the flags read after them.  So too where the application asked that waits
+    // for this device block (cudaDeviceScheduleBlockingSync): a report is polled for, and its
+    // round is over before a sleeping thread is back.
+    unsigned sched = 0;
+    ZOLA_CUDA_CHECK(cudaGetDeviceFlags(&sched), ctx);
+    const bool posted = !fused && !feed && !ctx->profile && !(sched & cudaDeviceScheduleBlockingSync);
     if (posted) {
         if ((rc = ensure_post(ctx))) return rc;
         sp.D.post = ctx->h_post;
@@ -3887,7 +3894,8 @@ int launch_fit_split(zola_ctx* ctx, zola_psf* p, WindowTables* w, const float* d
         rounds += posted ? 1 : 4;
         ZOLA_CUDA_CHECK(cudaGetLastError(), ctx);
         int active, err;
-        rc = posted ? wait_post(ctx, D.post_base + (unsigned)rounds, st, &active, &err, &queue)
+        rc = posted ? wait_post(ctx, D.post_base + (unsigned)rounds, st, (sched & cudaDeviceScheduleYield) != 0, &active, &err,
+                                &queue)
                     : read_flags(ctx, D, st, &active, &err, &queue);
         if (rc) return rc;
         if (err) { ctx->err = "split fit: a bounded device wait timed out"; return ZOLA_E_TIMEOUT; }
