@@ -200,7 +200,7 @@ def detect_fit_config(z, ctx, torch, device, nframes, fp64_frames=0, seed=1):
     out = {"workload": "256x256 uint16 frames, Poisson(5) tetrapod emitters, R = 40, 0.1 um library over +-2 um; "
                        "host frames in and localization rows out",
            "frames": nframes, "emitters": int(m), "library_slices": det.nz,
-           "detect_fp64_flops_per_frame": 2.0 * S * S * R * R * det.nz, "h2d_bytes_per_frame": S * S * 2}
+           "detect_fp64_flops_per_frame": detect_flops(S, S, R, det.nz), "h2d_bytes_per_frame": S * S * 2}
     # detection alone (uint16 frames in, candidate lists out), after a warm-up call of
     # the same size (it sizes the staging and scratch areas)
     det.detect_u16(frames)
@@ -211,9 +211,9 @@ def detect_fit_config(z, ctx, torch, device, nframes, fp64_frames=0, seed=1):
     out["detect_only"] = {"frames": nframes, "frames_per_s": nframes / dt,
                           "fp64_tflops": out["detect_fp64_flops_per_frame"] * nframes / dt / 1e12,
                           "fp64_frac_of_issue": out["detect_fp64_flops_per_frame"] * nframes / dt / fp64_issue,
-                          "note": "host uint16 frames to candidate lists through zola_detect_u16; flops of direct sums "
-                                  "for every pixel (FFTs screen them with far fewer, so the fraction can "
-                                  "exceed 1); FP64 issue rate = 148 SMs x 64 DFMA/clk x 1965 MHz (nominal)"}
+                          "note": "host uint16 frames to candidate lists through zola_detect_u16; flops of the "
+                                  "FFT correlation that scores every pixel (5 n log2 n a line); FP64 issue rate = "
+                                  "148 SMs x 64 DFMA/clk x 1965 MHz (nominal)"}
     rows = {}
     for name, prec, nf in (("split", z.ZOLA_PREC_SPLIT, nframes), ("fp64", z.ZOLA_PREC_FP64, fp64_frames)):
         if nf <= 0:
@@ -573,6 +573,42 @@ def flops_per_eval(R, N):
     return 3 * 8 * W * D * D + 4 * 8 * W * W * D
 
 
+def line_flops(n):
+    return 5.0 * n * np.log2(n)
+
+
+def fft_eval_flops(R, N):
+    """The same evaluation as the FP64 form computes it: line transforms of N points, then the two blurs."""
+    W, D = window(R, N), disk_rows(N)
+    return (3 * D + 4 * W) * line_flops(N) + 8 * (R * W * W + R * R * W)
+
+
+def direct_eval_flops(R, N):
+    """The same evaluation by direct sums, with the two blurs."""
+    W = window(R, N)
+    return flops_per_eval(R, N) + 8 * (R * W * W + R * R * W)
+
+
+def fp64_fit_flops(R, N, status, evals, trial=12):
+    """Operations of FP64 fits: the FFT form for the first `trial` evaluations, and all of them again by direct sums
+    where a fit has not converged by then."""
+    again = (status != 1) | (evals > trial)
+    return fft_eval_flops(R, N) * np.minimum(evals, trial).sum() + direct_eval_flops(R, N) * evals[again].sum()
+
+
+def detect_flops(SX, SY, R, slices):
+    """Operations of one frame's scores: line transforms along both axes of the padded frame, and back for each pair of
+    library slices, with the product of the spectra and the scaling."""
+    lengths = sorted(a * b * c * d for a, b, c, d in (
+        (4, 4, 4, 1), (5, 4, 4, 1), (6, 4, 4, 1), (5, 5, 4, 1), (6, 5, 4, 1), (8, 4, 4, 1), (6, 6, 4, 1), (6, 5, 5, 1),
+        (8, 5, 4, 1), (6, 6, 5, 1), (8, 6, 4, 1), (8, 5, 5, 1), (6, 6, 6, 1), (8, 6, 5, 1), (8, 8, 4, 1), (8, 6, 6, 1),
+        (8, 8, 5, 1), (8, 8, 6, 1), (8, 8, 8, 1)))
+    MX, MY = (next(m for m in lengths if m >= n + R // 2) for n in (SX, SY))
+    both = SX * line_flops(MY) + MY * line_flops(MX)
+    pairs = (slices + 1) // 2
+    return float(both + pairs * (both + 6 * MX * MY) + 3 * slices * SX * SY)
+
+
 def theta_err(a, b, zsym):
     """|a - b| per ROI and parameter, |z| compared for z-symmetric PSFs."""
     d = np.abs(a - b)
@@ -785,12 +821,9 @@ def main():
         t = e0.elapsed_time(e1) / 1000.0
         t_job64 += t / m * cnt
         name = j["cls"]["name"]
-        ev64 = int(it64.sum().item())
         fp64[name] = {"sample": m, "seconds": t, "fits_per_s": m / t,
-                      "fp64_tflops": round(ev64 * (flops_per_eval(j["cls"]["R"], j["cls"]["N"]) +
-                                                   8 * (j["cls"]["R"] * window(j["cls"]["R"], j["cls"]["N"]) ** 2 +
-                                                        j["cls"]["R"] ** 2 * window(j["cls"]["R"], j["cls"]["N"])))
-                                           / t / 1e12, 3)}
+                      "fp64_tflops": round(fp64_fit_flops(j["cls"]["R"], j["cls"]["N"], st64.cpu().numpy(),
+                                                          it64.cpu().numpy()) / t / 1e12, 3)}
         b, sb = split_res[name]
         acc64[name] = accuracy_block(out64.cpu().numpy(), st64.cpu().numpy(), b[:m], sb[:m], j["cls"]["zsym"])
     fp64_value = n_total / t_job64
