@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(FL_THREADS, 3) k_cal_eval(CalView V, const dou
     const int D = V.D, W = V.W, R = V.R, RR = R * R, tid = threadIdx.x;
     const Cluster cl;
     const CalSmem m = cal_begin<NFFT>(V, cal_sm);
-    double *part1 = m.red + 128, *part10 = m.red + 136, *part4 = m.red + 152;  // sums of 1, 10 and 4 values
+    double *part1 = m.red + 128, *part9 = m.red + 136, *part4 = m.red + 152;  // sums of 1, 9 and 4 values
     CalWork w = cal_carve(scratch + cl.id() * per_cluster, D, W, R);
     const int i0 = cl.row0(R), i1 = cl.row1(R), nt = (i1 - i0) * R, px0 = i0 * R;
     // T of the CTA's rows: in the transform buffer until the adjoint needs it, else in w.g
@@ -285,9 +285,9 @@ __global__ void __launch_bounds__(FL_THREADS, 3) k_cal_eval(CalView V, const dou
         cluster_sum<1>(cl, sum, m.red, part1);
         const double Ssum = sum[0];
         const double* d = V.stacks + (size_t)bs * RR;
-        double acc[10];  // nll, d/da, d/dc[6], sum g_psi psi, (unused)
+        double acc[9];  // nll, d/da, d/dc[6], sum g_psi psi
 #pragma unroll
-        for (int q = 0; q < 10; ++q) acc[q] = 0.0;
+        for (int q = 0; q < 9; ++q) acc[q] = 0.0;
         auto weight = [&](int k, double psi, double* mu_) {  // 1 - d / mu, 0 where mu is clamped
             const int i = k / R, ii = k - i * R;
             double bg = 0;
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(FL_THREADS, 3) k_cal_eval(CalView V, const dou
             for (int q = 0; q < NPOLY; ++q) acc[2 + q] += wgt * poly_m(q, i, ii);
             acc[8] += At * wgt * psi;
         }
-        cluster_sum<10>(cl, acc, m.red, part10);
+        cluster_sum<9>(cl, acc, m.red, part9);
         double tot4[4] = {0, 0, 0, 0};  // d/dsigma, d/dx, d/dy, d/dz
         if (mode == 1) {
             // g_T = sgn(T) (g_psi - sum g_psi psi) / S, and its product with dT / dsigma

@@ -1044,7 +1044,7 @@ int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap
     const size_t bits_b = (size_t)v.Z * v.SY * ((v.SX + 31) / 32) * 4;
     const size_t per = (4 + (size_t)v.Z) * SS * 8 + (size_t)cap * (7 * 8 + 4 + 17) + bits_b + (size_t)v.Z * 4 + 12 +
                        (gsort ? (size_t)p2 * 12 : 0) +
-                       (fft ? (size_t)d->fft.y.M * (v.SX + d->fft.x.M) * sizeof(double2) : 0);
+                       (fft ? (size_t)d->fft.MY * (v.SX + d->fft.MX) * sizeof(double2) : 0);
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min(nframes, 65535), ((size_t)1 << 31) / per));
     if (ensure_scratch(ctx, per * chunk + (fft ? det_fft_scratch(v, d->fft, 1) + DET_FFT_T_BYTES : 0) + 8192, ctx->err))
         return ZOLA_E_CUDA;
@@ -1083,7 +1083,7 @@ int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap
         k_det_rowsum<<<dim3((v.SX + VR_ROWS - 1) / VR_ROWS, nf), VR_THREADS, VR_SMEM, st>>>(v, fr, rowsum, rowsq, amax);
         k_det_colsum<<<dim3((v.SY + 31) / 32, nf), 32, 0, st>>>(v, rowsum, rowsq, var, isv);
         DetEps E{0, 0, amax, isv};
-        if (fft) det_fft_bound(v.SX, v.SY, v.R, d->fft.x.M, d->fft.y.M, v.inv_m, d->fft.pair, &E.k, &E.base);
+        if (fft) det_fft_bound(v.SX, v.SY, v.R, d->fft.MX, d->fft.MY, v.inv_m, d->fft.pair, &E.k, &E.base);
         k_det_var<<<dim3((unsigned)std::min<size_t>((SS + 255) / 256, 256), nf), 256, 0, st>>>(v, var, isv, E,
                                                                                               fft ? inexact : nullptr);
         ctx->launches += 3;

@@ -210,19 +210,19 @@ __global__ void __launch_bounds__(L::THREADS, L::CTAS) k_fft_rows_inv(const doub
     X(8, 8, 5, 1) X(8, 8, 6, 1) X(8, 8, 8, 1) X(6, 6, 4, 4) X(8, 5, 4, 4) X(6, 6, 5, 4) X(8, 6, 4, 4) X(6, 6, 6, 4)     \
     X(8, 6, 5, 4) X(8, 8, 4, 4) X(8, 8, 5, 4) X(8, 8, 6, 4) X(8, 8, 8, 4)
 
-static bool fft_dim(int n, FftDim* out) {
-    FftDim best;
+static bool fft_length(int n, int* out) {
+    int best = 0;
 #define X(a, b, c, d)                                                     \
     {                                                                     \
         using L = Len<a, b, c, d>;                                        \
-        if (L::M >= n && (best.M == 0 || L::M < best.M)) {                \
-            best.M = L::M;                                                \
+        if (L::M >= n && (best == 0 || L::M < best)) {                    \
+            best = L::M;                                                  \
         }                                                                 \
     }
     FFT_LENGTHS(X)
 #undef X
     *out = best;
-    return best.M > 0 && n >= 50;
+    return best > 0 && n >= 50;
 }
 
 // fn(L()) for the length M.
@@ -264,24 +264,24 @@ void det_fft_build(zola_ctx* ctx, const DetView& v, DetFft& p) {
     p = DetFft();
     if (!det_fft_wanted(v)) return;
     DetFft q;
-    if (!fft_dim(v.SX + v.R / 2, &q.x) || !fft_dim(v.SY + v.R / 2, &q.y)) return;
+    if (!fft_length(v.SX + v.R / 2, &q.MX) || !fft_length(v.SY + v.R / 2, &q.MY)) return;
     q.pairs = (v.Z + 1) / 2;
-    const size_t MM = (size_t)q.x.M * q.y.M, nk = MM * q.pairs;
+    const size_t MM = (size_t)q.MX * q.MY, nk = MM * q.pairs;
     if (nk * sizeof(double2) > DET_FFT_MAX_LIBRARY) return;
     double2* A = nullptr;
-    bool ok = cudaMalloc(&q.d_tab, (q.x.M + q.y.M + nk) * sizeof(double2)) == cudaSuccess &&
-              cudaMalloc(&A, (size_t)q.pairs * v.R * q.y.M * sizeof(double2)) == cudaSuccess;
+    bool ok = cudaMalloc(&q.d_tab, (q.MX + q.MY + nk) * sizeof(double2)) == cudaSuccess &&
+              cudaMalloc(&A, (size_t)q.pairs * v.R * q.MY * sizeof(double2)) == cudaSuccess;
     if (ok) {
-        std::vector<double2> tw(q.x.M + q.y.M);
-        for (int k = 0; k < q.x.M; ++k) tw[k] = make_double2(std::cos(2 * M_PI * k / q.x.M), -std::sin(2 * M_PI * k / q.x.M));
-        for (int k = 0; k < q.y.M; ++k)
-            tw[q.x.M + k] = make_double2(std::cos(2 * M_PI * k / q.y.M), -std::sin(2 * M_PI * k / q.y.M));
+        std::vector<double2> tw(q.MX + q.MY);
+        for (int k = 0; k < q.MX; ++k) tw[k] = make_double2(std::cos(2 * M_PI * k / q.MX), -std::sin(2 * M_PI * k / q.MX));
+        for (int k = 0; k < q.MY; ++k)
+            tw[q.MX + k] = make_double2(std::cos(2 * M_PI * k / q.MY), -std::sin(2 * M_PI * k / q.MY));
         ok = cudaMemcpy(q.d_tab, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice) == cudaSuccess;
     }
     if (ok) {
         cudaStream_t st = ctx->stream;
-        launch_fft_rows_fwd(q.y.M, dim3((unsigned)(v.R), 1, q.pairs), st, q.twy(), v.psf0, v.R, v.R, 1, v.Z, A);
-        launch_fft_cols_fwd(q.x.M, dim3((unsigned)(q.y.M), 1, q.pairs), st, q.twx(), A, v.R, v.R / 2, q.y.M,
+        launch_fft_rows_fwd(q.MY, dim3((unsigned)(v.R), 1, q.pairs), st, q.twy(), v.psf0, v.R, v.R, 1, v.Z, A);
+        launch_fft_cols_fwd(q.MX, dim3((unsigned)(q.MY), 1, q.pairs), st, q.twx(), A, v.R, v.R / 2, q.MY,
                             1.0 / (double)MM, 1, q.K());
         ctx->launches += 2;
         ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
@@ -298,18 +298,18 @@ void det_fft_build(zola_ctx* ctx, const DetView& v, DetFft& p) {
 // Frames whose T fits in about half of the 126 MB L2 go through the two inverse
 // passes together, so that T is read back from L2.
 static int frames_together(const DetView& v, const DetFft& p, int nf) {
-    const size_t t = (size_t)p.pairs * v.SX * p.y.M * sizeof(double2);
+    const size_t t = (size_t)p.pairs * v.SX * p.MY * sizeof(double2);
     return (int)std::max<size_t>(1, std::min<size_t>((size_t)nf, DET_FFT_T_BYTES / t));
 }
 
 size_t det_fft_scratch(const DetView& v, const DetFft& p, int nf) {
-    const size_t t = (size_t)p.pairs * v.SX * p.y.M * frames_together(v, p, nf), a = (size_t)v.SX * p.y.M * nf;
-    return (std::max(t, a) + (size_t)p.x.M * p.y.M * nf) * sizeof(double2);
+    const size_t t = (size_t)p.pairs * v.SX * p.MY * frames_together(v, p, nf), a = (size_t)v.SX * p.MY * nf;
+    return (std::max(t, a) + (size_t)p.MX * p.MY * nf) * sizeof(double2);
 }
 
 void det_fft_scores(zola_ctx* ctx, const DetView& v, const DetFft& p, const double* frames, int nf, const double* isv,
                     char* scratch, double* score, cudaStream_t st) {
-    const int MX = p.x.M, MY = p.y.M, FS = frames_together(v, p, nf);
+    const int MX = p.MX, MY = p.MY, FS = frames_together(v, p, nf);
     const size_t SS = (size_t)v.SX * v.SY;
     double2* F = (double2*)scratch;                 // spectra of the frames
     double2* T = F + (size_t)MX * MY * nf;          // row transforms, then the inverse column transforms

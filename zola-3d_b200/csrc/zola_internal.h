@@ -182,17 +182,14 @@ struct DetView {
 constexpr int DET_FFT_MIN_R = 14;  // see det_fft_wanted
 constexpr size_t DET_FFT_MAX_LIBRARY = (size_t)512 << 20;  // bytes of library spectra a detector may hold
 constexpr size_t DET_FFT_T_BYTES = (size_t)56 << 20;       // column transforms in flight (see frames_together)
-struct FftDim {
-    int M = 0;
-};
 struct DetFft {
-    FftDim x, y;
+    int MX = 0, MY = 0;
     int pairs = 0;
     double pair = 1.0;         // det_pair_ratio of the library
     double2* d_tab = nullptr;  // twiddles of x and y, then the spectra of the slice pairs
     const double2* twx() const { return d_tab; }
-    const double2* twy() const { return d_tab + x.M; }
-    double2* K() const { return d_tab + x.M + y.M; }
+    const double2* twy() const { return d_tab + MX; }
+    double2* K() const { return d_tab + MX + MY; }
 };
 // detect.cu: candidate lists of device frames, and the direct scores and offsets
 // of listed candidates.
