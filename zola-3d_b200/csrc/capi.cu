@@ -479,7 +479,12 @@ int fit_host_impl(zola_ctx* ctx, zola_psf* psf, int R, const float* rois, const 
     // go up, and its results come back, as one copy through pinned memory (with the rounds'
     // reports, 5 fits of 16 px take 279 us instead of 373).  Larger ones gain nothing.
     const size_t in_bytes = off_i + 5 * nn * sizeof(double), res_bytes = off_v - off_o;
-    const bool small = in_bytes <= HOST_STAGE && res_bytes <= HOST_STAGE;
+    // (Device pointers work in these calls too, as the driver's copies take them; the staging's
+    // memcpys do not.)
+    bool small = in_bytes <= HOST_STAGE && res_bytes <= HOST_STAGE;
+    for (const void* p : {(const void*)rois, (const void*)init5, (const void*)out5, (const void*)crlb5, (const void*)nll,
+                          (const void*)status, (const void*)iters})
+        small = small && !zola::device_memory(p);
     if (small) {
         if (!ctx->h_stage) ZOLA_CUDA_CHECK(cudaMallocHost((void**)&ctx->h_stage, HOST_STAGE), ctx);
         std::memcpy(ctx->h_stage, rois, rr * nn * sizeof(float));

@@ -151,6 +151,16 @@ void host_copy_free(zola_ctx* ctx) {
     delete h;
 }
 
+bool device_memory(const void* p) {
+    cudaPointerAttributes a{};
+    if (!p) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice;
+}
+
 // Whether the driver would stage this host memory itself.
 static bool pageable(const void* p) {
     cudaPointerAttributes a{};

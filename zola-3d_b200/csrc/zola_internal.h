@@ -267,6 +267,8 @@ int fit_frames_dev(zola_ctx* ctx, zola_psf* psf, int R, const float* d_rois, con
 cudaError_t copy_in(zola_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
 cudaError_t copy_out(zola_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
 void host_copy_free(zola_ctx* ctx);
+// Whether p, which may be null, is memory that only the GPU reads and writes.
+bool device_memory(const void* p);
 
 // library.cu: normalised R x R images at x = y = 0 and depths zwat[0 .. n), to the host
 int library_psfs(zola_psf* psf, int R, const double* zwat, int n, double* out);
