@@ -1,4 +1,4 @@
-"""GPU test of a host-buffer fit on device pointers, which the driver's copies take as well."""
+"""GPU tests of host-buffer calls on device pointers, which the driver's copies take as well."""
 import os
 import subprocess
 import sys
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
-SCRIPT = """
+FITS = """
 import ctypes, sys
 sys.path[:0] = [{root!r}, {root!r} + "/tests"]
 import numpy as np, torch
@@ -36,7 +36,47 @@ print("FINE")
 """
 
 
+GRADIENT = """
+import ctypes, sys
+sys.path[:0] = [{root!r}, {root!r} + "/tests"]
+import numpy as np, torch
+import __graft_entry__ as ge
+from common import OPTICS
+z = ge.load_package()
+ctx = z.Context(0)
+nz, nb, ns, R = 9, 2, 3, 16
+psf = z.PSF(ctx, z.optics(size_fft=64, n_wat=1.4, **OPTICS), np.zeros(nz))
+rng = np.random.default_rng(0)
+zern = np.r_[0, 0, 0, rng.normal(0, 0.2, nz - 3)]
+bead = np.zeros((nb, 3 + ns + 6))
+bead[:, 3:3 + ns], bead[:, 3 + ns] = 9000, 80
+cal = z.Calibration(psf, rng.poisson(200.0, (nb, ns, R, R)).astype(float), np.linspace(-0.3, 0.3, ns))
+nll, gz, gs, gb = cal.backward(zern, 0.95, bead)
+P = lambda a: ctypes.c_void_p(a.data_ptr() if isinstance(a, torch.Tensor) else a.ctypes.data)
+data = cal._data(nz)
+d_bead, d_gb = torch.tensor(bead, device="cuda"), torch.zeros(nb, 3 + ns + 6, dtype=torch.float64, device="cuda")
+torch.cuda.synchronize()
+f, g, s = np.zeros(1), np.zeros(nz), np.zeros(1)
+L = z.lib()
+assert L.zola_calib_backward(psf.h, ctypes.byref(data), P(zern), ctypes.c_double(0.95), P(d_bead), P(f), P(g), P(s), P(d_gb)) == 0
+torch.cuda.synchronize()
+assert f[0] == nll and np.array_equal(g, gz) and s[0] == gs and np.array_equal(d_gb.cpu().numpy(), gb)
+assert L.zola_calib_forward(psf.h, ctypes.byref(data), P(zern), ctypes.c_double(0.95), P(d_bead), P(f), None) == 0
+assert f[0] == cal.forward(zern, 0.95, bead)
+print("FINE")
+"""
+
+
+def _run(script):
+    r = subprocess.run([sys.executable, "-c", script.format(root=ROOT)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "FINE" in r.stdout, r.stdout + r.stderr
+
+
 def test_fits_on_device_pointers(zpkg):
     """Small and larger calls whose ROIs, starts or results are on the device: the results of host buffers."""
-    r = subprocess.run([sys.executable, "-c", SCRIPT.format(root=ROOT)], capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0 and "FINE" in r.stdout, r.stdout + r.stderr
+    _run(FITS)
+
+
+def test_calibration_gradient_on_device_pointers(zpkg):
+    """Bead parameters and their gradient on the device: those of host buffers."""
+    _run(GRADIENT)

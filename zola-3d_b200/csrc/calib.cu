@@ -984,7 +984,8 @@ int cal_upload(zola_psf* p, CalRun& run, const double* coef, double sigma, const
     const int R = run.V.R, W = run.V.W, DD = run.V.D * run.V.D;
     const size_t head = run.head();
     std::memcpy(run.par.data(), coef, run.nz * 8);
-    std::memcpy(run.par.data() + run.nz, bead, run.n_bead() * 8);
+    const bool on_device = device_memory(bead);  // (as the driver's copies take it)
+    if (!on_device) std::memcpy(run.par.data() + run.nz, bead, run.n_bead() * 8);
     size_t n = head;
     if (sigma != run.sigma) {
         std::vector<double> G, dG;
@@ -999,6 +1000,8 @@ int cal_upload(zola_psf* p, CalRun& run, const double* coef, double sigma, const
         n = run.par.size();
     }
     cudaError_t e = cudaMemcpyAsync(run.d_par, run.par.data(), n * 8, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && on_device)
+        e = cudaMemcpyAsync(run.d_par + run.nz, bead, run.n_bead() * 8, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e == cudaSuccess) {
         k_cal_phase<<<(DD + 127) / 128, 128, 0, ctx->stream>>>(p->d_calZ, run.d_par, run.nz, DD, run.d_phase);
         ctx->launches++;
@@ -1054,14 +1057,17 @@ int cal_eval(zola_psf* p, CalRun& run, const double* coef, double sigma, const d
         e = cudaGetLastError();
     }
     const size_t n = mode ? run.res.size() : 2;
+    const bool on_device = mode && device_memory(gb);
     if (e == cudaSuccess) e = cudaMemcpyAsync(run.res.data(), run.d_res, n * 8, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && on_device)
+        e = cudaMemcpyAsync(gb, run.d_res + 2 + nz, run.n_bead() * 8, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cal_cuda(ctx, e);
     *nll = run.res[0];
     if (!mode) return ZOLA_OK;
     if (gsig) *gsig = run.res[1];
     std::memcpy(gz, run.res.data() + 2, (size_t)nz * 8);
-    std::memcpy(gb, run.res.data() + 2 + nz, run.n_bead() * 8);
+    if (!on_device) std::memcpy(gb, run.res.data() + 2 + nz, run.n_bead() * 8);
     return ZOLA_OK;
 }
 
