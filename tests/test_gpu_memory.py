@@ -43,3 +43,30 @@ def test_large_model_calls_give_their_buffers_back(zpkg, derivs):
     for a, b in zip(few, many) if derivs else [(few, many)]:
         assert np.array_equal(a, b[pick])
     ctx.close()
+
+
+def test_detection_without_room_for_the_spectra(zpkg):
+    """A frame of 1200 x 1200 against 40 slices: 1.1 GB with the FFT correlation, 0.6 without.  With 0.9 GB left the
+    rows are those of a detection with all the memory it wants."""
+    import torch
+    ctx = zpkg.Context(0)
+    psf = zpkg.PSF(ctx, zpkg.optics(size_fft=128, kz_reset=True, **OPTICS), astig_zernike())
+    frames = np.random.default_rng(2).poisson(20.0, (1, 1200, 1200)).astype(float)
+    frames[:, 300:306, 500:506] += 300
+    det = zpkg.Detector(psf, 1200, 1200, 40, -2.0, 2.0, 0.1, 0.1)
+    want, n = det.detect(frames, cap=500)
+    ctx2 = zpkg.Context(0)
+    psf2 = zpkg.PSF(ctx2, zpkg.optics(size_fft=128, kz_reset=True, **OPTICS), astig_zernike())
+    det2 = zpkg.Detector(psf2, 1200, 1200, 40, -2.0, 2.0, 0.1, 0.1)
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info(0)[0] - (900 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got, m = det2.detect(frames, cap=500)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert n[0] == m[0] > 0 and np.array_equal(want[0], got[0])
+    det.close()
+    det2.close()
+    ctx.close()
+    ctx2.close()

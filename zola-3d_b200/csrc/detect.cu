@@ -1036,18 +1036,24 @@ int detect_frames(zola_detector* d, const double* d_frames, int nframes, int cap
     v.cap = cap;
     const size_t SS = (size_t)v.SX * v.SY;
     const int p2 = det_pow2(cap);
-    const bool gsort = p2 > DET_SORT_SMEM, fft = d->fft.d_tab != nullptr;
+    const bool gsort = p2 > DET_SORT_SMEM;
+    bool fft = d->fft.d_tab != nullptr;
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
     // scratch per frame: row sums and their squares, variance, its inverse root, scores
     // (Z x SS), candidates, peak bits and counts, and the sort keys when they do not fit
     // in shared memory; for the FFT correlation also the spectra
     const size_t bits_b = (size_t)v.Z * v.SY * ((v.SX + 31) / 32) * 4;
-    const size_t per = (4 + (size_t)v.Z) * SS * 8 + (size_t)cap * (7 * 8 + 4 + 17) + bits_b + (size_t)v.Z * 4 + 12 +
-                       (gsort ? (size_t)p2 * 12 : 0) +
-                       (fft ? (size_t)d->fft.MY * (v.SX + d->fft.MX) * sizeof(double2) : 0);
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min(nframes, 65535), ((size_t)1 << 31) / per));
-    if (ensure_scratch(ctx, per * chunk + (fft ? det_fft_scratch(v, d->fft, 1) + DET_FFT_T_BYTES : 0) + 8192, ctx->err))
-        return ZOLA_E_CUDA;
+    int chunk = 0;
+    for (;; fft = false) {
+        const size_t per = (4 + (size_t)v.Z) * SS * 8 + (size_t)cap * (7 * 8 + 4 + 17) + bits_b + (size_t)v.Z * 4 + 12 +
+                           (gsort ? (size_t)p2 * 12 : 0) +
+                           (fft ? (size_t)d->fft.MY * (v.SX + d->fft.MX) * sizeof(double2) : 0);
+        chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min(nframes, 65535), ((size_t)1 << 31) / per));
+        if (ensure_scratch(ctx, per * chunk + (fft ? det_fft_scratch(v, d->fft, 1) + DET_FFT_T_BYTES : 0) + 8192, ctx->err) == 0)
+            break;
+        if (!fft) return ZOLA_E_CUDA;
+        cudaGetLastError();  // no room for the spectra: direct sums, which give the same rows
+    }
     const size_t rsmem = refine_smem(v.R), ssort = gsort ? 0 : (size_t)p2 * 12;
     ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_det_rowsum, cudaFuncAttributeMaxDynamicSharedMemorySize, VR_SMEM), ctx);
     ZOLA_CUDA_CHECK(cudaFuncSetAttribute(k_det_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem), ctx);
