@@ -879,6 +879,10 @@ cudaError_t basis(zola_psf* p, int nz) {
         }
     cudaError_t e = cudaMalloc(&p->d_calZ, Z.size() * 8);
     if (e == cudaSuccess) e = cudaMemcpy(p->d_calZ, Z.data(), Z.size() * 8, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {  // (nothing half made is kept)
+        if (p->d_calZ) cudaFree(p->d_calZ);
+        p->d_calZ = nullptr;
+    }
     p->cal_nz = nz;
     return e;
 }
