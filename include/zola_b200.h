@@ -79,7 +79,7 @@ typedef struct {
     int precision;       /* ZOLA_PREC_* */
 } zola_fit_params;
 
-#define ZOLA_PREC_FP64 0     /* plain FP64 GPU form (CUDA cores, one CTA per ROI) */
+#define ZOLA_PREC_FP64 0     /* plain FP64 GPU form (CUDA cores, a cluster of CTAs per ROI) */
 #define ZOLA_PREC_SPLIT 1    /* split-precision tcgen05 partial DFT, FP32 sums, FP64 solve */
 
 /* Per-ROI status codes written by the fits. */
